@@ -1,28 +1,31 @@
 // gfb_kernels.cuh -- sm_100a kernels of the CG-SEM elastic time loop.
 //
-// One time step is NC colour launches of elem_step_kernel followed by one
-// launch of node_update_kernel:
+// One time step is the element phase followed by the node phase:
 //
-//   elem_step_kernel (colour c)  -- for every cell of colour c: gather the
-//       predicted displacement through ibool into shared memory, GLL
-//       derivative contractions, stress, weighted transposed-derivative
-//       divergence (forward/elastic/src/element_cpu.cpp:19-162), C-PML
-//       acceleration term and memory update on C-PML cells
-//       (forward/share/src/pml.cpp:55-216), point-force injection
-//       (forward/share/src/solver.cpp:577-605), then a plain read-modify-
-//       write of the global force.  Cells of one colour share no node, and
-//       colours run in a fixed order, so assembly needs no atomics and is
-//       bit-reproducible run to run.  The first colour touching a node
-//       stores instead of adding, which replaces the memset of the global
-//       residual (cuda_step.cu:289-290).
-//   node_update_kernel -- Newmark corrector with the diagonal mass and the
-//       legacy velocity damping (solver.cpp:52-69, 564-574), followed by the
+//   elem_gather_kernel -- for every cell: gather the predicted displacement
+//       through ibool, GLL derivative contractions, stress, weighted
+//       transposed-derivative divergence (forward/elastic/src/
+//       element_cpu.cpp:19-162), C-PML acceleration term and memory update on
+//       C-PML cells (forward/share/src/pml.cpp:55-216; per-cell form), point-
+//       force injection (forward/share/src/solver.cpp:577-605).  The cell's
+//       force contributions are stored cell by cell.
+//   node_update_kernel, node_pml_kernel -- sum of the contributions of a
+//       node's cells in mesh order (no atomics, bit-reproducible run to run),
+//       node-form C-PML, Newmark corrector with the diagonal mass and the
+//       legacy velocity damping (solver.cpp:52-69, 564-574), then the
 //       predictor of the next step (solver.cpp:40-49), so no separate
 //       predictor launch is needed.
 //
-// Layouts on the device (cells in colour order):
-//   ibool  [cell][NN]            node id | FIRST_TOUCH bit
-//   geom   [cell][12][NN] Real   dxi_dx(9), jac*w_i*w_j*w_k, lambda, mu
+// elem_col_kernel and elem_pipe_kernel assemble in the element phase instead,
+// one launch per colour with a plain read-modify-write of the global force:
+// cells of one colour share no node and colours run in a fixed order, and the
+// first colour touching a node stores instead of adding, which replaces the
+// memset of the global residual (cuda_step.cu:289-290).  elem_step_kernel
+// serves the residual of independent elements.
+//
+// Layouts on the device (cells in mesh order):
+//   ibool  [cell][NN]            node id | FIRST_TOUCH, LAST_TOUCH bits (by colour)
+//   geom   [cell][geo_row] Real  dxi_dx (9), lambda and mu times the weight
 //   state  u, v (double), a (Real): [node][3*n_field];
 //          predicted displacement ut and force (Real): [node][n_field][4]
 //   C-PML  coef [slot][15][NN] Real (alpha 9, abar 5, w*J/rho),
@@ -49,6 +52,16 @@ __device__ __forceinline__ long long padded_index(long long g, int f, int F) {
 // cell, then the index of the model the cell belongs to, padded to whole
 // 16-byte copies.
 __host__ __device__ constexpr int ib_row_words(int nn) { return (nn + 1 + 3) / 4 * 4; }
+
+// Geometry rows of the time loop, [cell][geo_row]: dxi_dx (9 x NN), then
+// lambda and mu times det J w_i w_j w_k (so the stress they give is already
+// the flux's and the weight costs no load or multiply), padded to whole
+// 16-byte copies.  Where mu <= 0 both are 0: the point adds nothing
+// (element_cpu.cpp:42-43).
+template <typename Real>
+__host__ __device__ constexpr int geo_row(int nn) {
+    return (11 * nn * (int)sizeof(Real) + 15) / 16 * 16 / (int)sizeof(Real);
+}
 
 // Time-step constants of one model (several independent models can share
 // one solver): dt, dt^2/2 (beta = 0) and the C-PML field coefficients
@@ -85,6 +98,40 @@ struct Shape {
     static constexpr int THREADS = NNP * EPB;
 };
 
+// Assembly by the node pass.  The element kernel leaves every cell's force
+// contributions in contrib [cell][chunk][NN][fields of the chunk][3], cells in
+// mesh order: a chunk holds up to gather_chunk_fields wavefields, so what a
+// node reads of a cell is contiguous, as its state is.  A touch is an index
+// into it in units of 3 Reals (of the point's first wavefield, chunk 0); a
+// node's touches in mesh order:
+//   touch[g].x .y .z  the first three (kNoTouch: fewer)
+//   touch[g].w        the fourth, kNoTouch, or kMoreTouches | i: the touches
+//                     from the fourth on are more[i] (and more[i+1], ... while
+//                     bit 31 of .x is set), unused entries kNoTouch.
+// All but the corner nodes of a hexahedral mesh (1 in 64 at ngll 5) have at
+// most four touches and need this one 16-byte entry.  The sum runs in mesh
+// order.
+constexpr uint32_t kNoTouch = 0xffffffffu;
+constexpr uint32_t kMoreTouches = 0x80000000u;
+template <typename Real>
+__host__ __device__ constexpr int gather_chunk_fields(int nfld) {
+    return sizeof(Real) == 8 ? 1 : (nfld < 3 ? nfld : 3);
+}
+// Units (3 Reals) of a chunk: whole 16-byte copies.
+template <typename Real>
+__host__ __device__ constexpr int gather_chunk_units(int nn, int nfld) {
+    return (nn * gather_chunk_fields<Real>(nfld) * 3 * (int)sizeof(Real) + 47) / 48 * 48 / (3 * (int)sizeof(Real));
+}
+template <typename Real>
+struct NodeGather {
+    const uint4* touch;
+    const uint4* more;
+    const Real* contrib;
+    int chunk_units;
+    bool keep;              // the assembled force is kept in `force` (increments, records)
+    const int* mdirect;     // [model] 0: this step's contributions add to the kept force (nullptr: in full)
+};
+
 template <typename Real>
 struct NodeArgs {
     long long n_node;
@@ -92,7 +139,8 @@ struct NodeArgs {
     double* v;
     Real* a;
     Real* ut;               // [node][field][4]
-    const Real* force;      // [node][field][4]
+    Real* force;            // [node][field][4]
+    NodeGather<Real> gather;  // cell contributions to assemble (touch == nullptr: `force` is assembled)
     const double* mass;     // [n_node] assembled lumped mass
     const Real* inv_mass;   // [n_node] 1/m (FP32 path) or nullptr
     const double* damping;  // [n_node] or nullptr
@@ -139,7 +187,8 @@ struct NodePml {
 
 template <typename Real>
 struct ElemArgs {
-    int e_begin, e_end;
+    int e_begin, e_end;     // range of `cells` (elem_step_kernel: of the cells themselves)
+    const int* cells;       // the cells colour after colour
     const uint32_t* ibool;
     const Real* geom;
     const Real* ut;
@@ -362,14 +411,6 @@ __device__ __forceinline__ void load4(const double* p, double (&v)[4]) {
     const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
     v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
-__device__ __forceinline__ void load4_nc(const float* p, float (&v)[4]) {
-    const float4 t = __ldg(reinterpret_cast<const float4*>(p));
-    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-}
-__device__ __forceinline__ void load4_nc(const double* p, double (&v)[4]) {
-    const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
 __device__ __forceinline__ void store4(float* p, float a, float b, float c, float d) {
     *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
 }
@@ -378,6 +419,13 @@ __device__ __forceinline__ void store4(double* p, double a, double b, double c, 
     reinterpret_cast<double2*>(p)[1] = make_double2(c, d);
 }
 
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+
 // FP64 operations rounded one by one (no contraction into FMA), so that the
 // node update rounds the same way in every instantiation of the kernels
 // that inline it (a solver of one model and of several must agree bit for
@@ -385,128 +433,154 @@ __device__ __forceinline__ void store4(double* p, double a, double b, double c, 
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 
-// Finalise wavefield d of node g from its complete assembled force fv:
-// node C-PML term (when PML), Newmark corrector with the diagonal mass
+// Real operations rounded the same way wherever the node update is inlined
+// (node passes, fused update).
+__device__ __forceinline__ float rfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double rfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float rmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
+
+// One wavefield of a node on its way through the end of a step: load() issues
+// every load, finish() takes the complete assembled force fv through the node
+// C-PML term (when PML and pml), the Newmark corrector with the diagonal mass
 // (solver.cpp:52-69, legacy damping of 564-574 applied to v first) and the
-// next step's predictor (40-49), written as one 16-byte vector.  Every load
-// is issued before the first store, so a thread's memory round trips
-// overlap.  On the FP32 path 1/m == 0 marks a node with m <= 0 (the host
-// stores 0 there), so the f64 mass is not read.
+// next step's predictor (40-49).  On the FP32 path 1/m == 0 marks a node with
+// m <= 0 (the host stores 0 there), so the f64 mass is not read.
+// HALF_V: Newmark with beta = 0, gamma = 1/2 (solver.cpp:40-69) written on
+// the half-step velocity w = v + dt/2 a: u_{n+1} = u_n + dt w_n, a_{n+1} = f/m,
+// w_{n+1} = w_n + dt a_{n+1}, and the next predicted displacement
+// u_{n+1} + dt w_{n+1} (its increment dt w_{n+1}).  The same values as the
+// (u, v, a) form in exact arithmetic, without the acceleration's read and
+// write; v and a are recovered from w and the assembled force when they are
+// needed (records, state).  w is held in float (its rounding adds a random
+// walk of ~1e-7 relative per step, far below the float rounding of the
+// predicted displacement that bounds this path), u in double.
+template <typename Real, int NFLD, bool PML, bool HALF_V>
+struct NodeField {
+    static constexpr int F = 3 * NFLD;
+    double u[3], v[3], m, dmp;
+    Real a[3], im;
+    float w[3];
+    Real mm[3][3], pr[3];
+
+    // cf: the node's C-PML coefficients (when pml)
+    __device__ __forceinline__ void load(const NodeArgs<Real>& A, const NodePml<Real>& P, long long g, int d, bool pml,
+                                         const Real* cf) {
+        const size_t i = (size_t)g * F + d * 3;
+        im = A.inv_mass ? __ldg(A.inv_mass + g) : Real(0);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) u[c] = A.u[i + c];
+        if constexpr (HALF_V) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) w[c] = A.w32[i + c];
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                v[c] = A.v[i + c];
+                a[c] = A.a[i + c];
+            }
+            m = A.inv_mass ? 1.0 : __ldg(A.mass + g);
+            dmp = A.damping ? __ldg(A.damping + g) : 0.0;
+            if (PML && pml) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) pr[c] = P.prev[i + c];
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    const Real* mem = P.mem + (size_t)q * P.n_slot * F + i;
+                    const bool live = cf[2 + q] != Real(0);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) mm[q][c] = live ? mem[c] : Real(0);
+                }
+            }
+        }
+    }
+
+    __device__ __forceinline__ void finish(const NodeArgs<Real>& A, const NodePml<Real>& P, long long g, int d, bool pml,
+                                           const Real* cf, const Real (&fv)[3], const ModelConst& K, bool full) {
+        const size_t i = (size_t)g * F + d * 3;
+        Real out[3];
+        if constexpr (HALF_V) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                double ww = (double)w[c];
+                if (im != Real(0)) {  // m <= 0: the node stays as it is (a = 0, solver.cpp:58-61)
+                    const double a_new = (double)rmul(fv[c], im);
+                    u[c] = dadd(u[c], dmul(K.dt, ww));
+                    ww = (double)(float)dadd(ww, dmul(K.dt, a_new));
+                    A.u[i + c] = u[c];
+                    A.w32[i + c] = (float)ww;
+                }
+                out[c] = full ? (Real)dadd(u[c], dmul(K.dt, ww)) : (Real)dmul(K.dt, ww);
+            }
+        } else {
+            const bool massless = A.inv_mass ? (im == Real(0)) : (m <= 0.0);
+            Real force[3] = {fv[0], fv[1], fv[2]};
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                if (dmp > 0.0) v[c] = __dsub_rn(v[c], dmul(dmp, v[c]));
+            if (PML && pml) {
+                Real nv[3], ov[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    nv[c] = (Real)dadd(u[c], dmul(K.c1, v[c]));
+                    ov[c] = rfma((Real)K.c2, a[c], pr[c]);
+                    Real t = rmul(cf[0], (Real)v[c]);
+                    t = rfma(cf[1], (Real)u[c], t);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) t = rfma(cf[2 + q], mm[q][c], t);
+                    force[c] += t;
+                    P.prev[i + c] = nv[c];
+                }
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                    if (cf[2 + q] != Real(0)) {
+                        Real* mem = P.mem + (size_t)q * P.n_slot * F + i;
+                        const Real k0 = cf[5 + 3 * q], k1 = cf[6 + 3 * q], k2 = cf[7 + 3 * q];
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) mem[c] = rfma(k2, ov[c], rfma(k1, nv[c], rmul(k0, mm[q][c])));
+                    }
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                double a_new = 0.0;
+                if (!massless) {
+                    a_new = A.inv_mass ? (double)rmul(force[c], im) : __ddiv_rn((double)force[c], m);
+                    a_new = (double)(Real)a_new;
+                    const double a_old = (double)a[c];
+                    // solver.cpp:62-66
+                    const double ta = dadd(dmul(0.5 - A.beta, a_old), dmul(A.beta, a_new));
+                    u[c] = dadd(u[c], dadd(dmul(K.dt, v[c]), dmul(dmul(K.dt, K.dt), ta)));
+                    v[c] = dadd(v[c], dmul(K.dt, dadd(dmul(1.0 - A.gamma, a_old), dmul(A.gamma, a_new))));
+                }
+                A.u[i + c] = u[c];
+                A.v[i + c] = v[c];
+                A.a[i + c] = (Real)a_new;
+                // the next step's predicted displacement (solver.cpp:40-49), or its
+                // increment over this step's (u_{n+1} is this step's prediction)
+                const double inc = dadd(dmul(K.dt, v[c]), dmul(K.half_dt2, a_new));
+                out[c] = full ? (Real)dadd(u[c], inc) : (Real)inc;
+            }
+        }
+        store4(A.ut + ((size_t)g * NFLD + d) * 4, out[0], out[1], out[2], Real(0));
+    }
+};
+
+// Wavefield d of node g finalised from its complete assembled force (the
+// node update fused into the element kernel).
 template <typename Real, int NFLD, bool PML>
 __device__ __forceinline__ void update_node_field(const NodeArgs<Real>& A, const NodePml<Real>& P, long long g,
                                                   int d, const Real (&fv)[3], int sl, const ModelConst& K,
                                                   bool full = true) {
-    constexpr int F = 3 * NFLD;
-    const long long i0 = g * F + d * 3;
-    double* __restrict__ pu = A.u + i0;
-    double* __restrict__ pv = A.v + i0;
-    Real* __restrict__ pa = A.a + i0;
-    if (!PML && A.half_v) {
-        // Newmark with beta = 0, gamma = 1/2 (solver.cpp:40-69) written on
-        // the half-step velocity w = v + dt/2 a: u_{n+1} = u_n + dt w_n,
-        // a_{n+1} = f/m, w_{n+1} = w_n + dt a_{n+1}, and the next predicted
-        // displacement u_{n+1} + dt w_{n+1} (its increment dt w_{n+1}).  The
-        // same values as the (u, v, a) form in exact arithmetic, without the
-        // acceleration's read and write; v and a are recovered from w and
-        // the assembled force when they are needed (records, state).  w is
-        // held in float (its rounding adds a random walk of ~1e-7 relative
-        // per step, far below the float rounding of the predicted
-        // displacement that bounds this path), u in double.
-        float* __restrict__ pw = A.w32 + i0;
-        double uu[3], ww[3];
+    NodeField<Real, NFLD, PML, false> x;
+    Real cf[14];
+    if (PML && sl >= 0) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            uu[c] = pu[c];
-            ww[c] = (double)pw[c];
-        }
-        const Real im = __ldg(A.inv_mass + g);
-        Real out[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            if (im != Real(0)) {  // m <= 0: the node stays as it is (a = 0, solver.cpp:58-61)
-                const double a_new = (double)(Real)(fv[c] * im);
-                uu[c] = dadd(uu[c], dmul(K.dt, ww[c]));
-                ww[c] = (double)(float)dadd(ww[c], dmul(K.dt, a_new));
-                pu[c] = uu[c];
-                pw[c] = (float)ww[c];
-            }
-            out[c] = full ? (Real)dadd(uu[c], dmul(K.dt, ww[c])) : (Real)dmul(K.dt, ww[c]);
-        }
-        store4(A.ut + ((size_t)g * NFLD + d) * 4, out[0], out[1], out[2], Real(0));
-        return;
+        for (int q = 0; q < 14; ++q) cf[q] = __ldg(P.coef + (size_t)sl * 14 + q);
     }
-    double vv[3], uu[3];
-    Real ao[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        vv[c] = pv[c];
-        uu[c] = pu[c];
-        ao[c] = pa[c];
-    }
-    const Real im = A.inv_mass ? __ldg(A.inv_mass + g) : Real(0);
-    const bool massless = A.inv_mass ? (im == Real(0)) : (__ldg(A.mass + g) <= 0.0);
-    const double m = A.inv_mass ? 1.0 : __ldg(A.mass + g);
-    const double dmp = A.damping ? __ldg(A.damping + g) : 0.0;
-    Real cf[14], mm[3][3], pr[3];
-    if (PML) {
-        if (sl >= 0) {
-#pragma unroll
-            for (int q = 0; q < 14; ++q) cf[q] = __ldg(P.coef + (size_t)sl * 14 + q);
-#pragma unroll
-            for (int q = 0; q < 3; ++q)
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-                    mm[q][c] = cf[2 + q] != Real(0) ? P.mem[((size_t)q * P.n_slot + sl) * F + d * 3 + c] : Real(0);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) pr[c] = P.prev[(size_t)sl * F + d * 3 + c];
-        }
-    }
-    Real out[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        if (dmp > 0.0) vv[c] = __dsub_rn(vv[c], dmul(dmp, vv[c]));
-        Real force = fv[c];
-        if (PML && sl >= 0) {
-            const Real nv = (Real)dadd(uu[c], dmul(K.c1, vv[c]));
-            const Real ov = pr[c] + (Real)K.c2 * ao[c];
-            force += cf[0] * (Real)vv[c] + cf[1] * (Real)uu[c] + cf[2] * mm[0][c] + cf[3] * mm[1][c] + cf[4] * mm[2][c];
-#pragma unroll
-            for (int q = 0; q < 3; ++q)
-                if (cf[2 + q] != Real(0))
-                    P.mem[((size_t)q * P.n_slot + sl) * F + d * 3 + c] =
-                        cf[5 + 3 * q] * mm[q][c] + cf[6 + 3 * q] * nv + cf[7 + 3 * q] * ov;
-            P.prev[(size_t)sl * F + d * 3 + c] = nv;
-        }
-        double a_new;
-        if (massless) {
-            a_new = 0.0;
-        } else {
-            a_new = A.inv_mass ? (double)(force * im) : __ddiv_rn((double)force, m);
-            a_new = (double)(Real)a_new;
-            const double a_old = (double)ao[c];
-            // solver.cpp:62-66
-            const double ta = dadd(dmul(0.5 - A.beta, a_old), dmul(A.beta, a_new));
-            uu[c] = dadd(uu[c], dadd(dmul(K.dt, vv[c]), dmul(dmul(K.dt, K.dt), ta)));
-            vv[c] = dadd(vv[c], dmul(K.dt, dadd(dmul(1.0 - A.gamma, a_old), dmul(A.gamma, a_new))));
-        }
-        pu[c] = uu[c];
-        pv[c] = vv[c];
-        pa[c] = (Real)a_new;
-        // the next step's predicted displacement (solver.cpp:40-49), or its
-        // increment over this step's (u_{n+1} is this step's prediction)
-        const double inc = dadd(dmul(K.dt, vv[c]), dmul(K.half_dt2, a_new));
-        out[c] = full ? (Real)dadd(uu[c], inc) : (Real)inc;
-    }
-    store4(A.ut + ((size_t)g * NFLD + d) * 4, out[0], out[1], out[2], Real(0));
+    x.load(A, P, g, d, sl >= 0, cf);
+    x.finish(A, P, g, d, sl >= 0, cf, fv, K, full);
 }
 
-// Separate node pass (used when the element kernel does not finalise nodes):
-// one thread per (node, wavefield), the wavefields of a node in adjacent
-// threads, so a warp streams contiguous u, v, a and force/prediction
-// vectors and reads each node's mass once.  With node-form C-PML the pass
-// is two launches over contiguous node ranges: node_update_kernel over the
-// plain nodes [g0, n_node) without the C-PML registers, node_pml_kernel
-// over the C-PML nodes [0, g0).
 // Constants of the model node g belongs to; false when that model has
 // taken all its steps (its state stays as it is).
 template <typename Real, bool MULTI>
@@ -524,29 +598,170 @@ __device__ __forceinline__ bool node_constants(const NodeArgs<Real>& A, const No
     return true;
 }
 
-template <typename Real, int NFLD, bool MULTI>
-__global__ void __launch_bounds__(256, 3) node_update_kernel(NodeArgs<Real> A, NodePml<Real> P, long long g0) {
-    const long long g1 = (MULTI && A.live_node_end) ? min(A.n_node, A.live_node_end[1]) : A.n_node;
-    const long long total = max(0LL, g1 - g0) * NFLD;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
-        const long long gl = t / NFLD;
-        const int d = (int)(t - gl * NFLD);
-        const long long g = g0 + gl;
-        ModelConst K;
-        bool full;
-        if (!node_constants<Real, MULTI>(A, P, g, K, full)) continue;
-        Real fv4[4];
-        load4_nc(A.force + ((size_t)g * NFLD + d) * 4, fv4);
-        const Real fv[3] = {fv4[0], fv4[1], fv4[2]};
-        update_node_field<Real, NFLD, false>(A, P, g, d, fv, -1, K, full);
+// The parts of the assembled force of a node's wavefield, loaded: the kept
+// force (add: the contributions add to it) and the first four touches.
+template <typename Real, int NFLD>
+struct ForceParts {
+    Real old[4], c[4][3];
+    static __device__ __forceinline__ const Real* touches(const NodeArgs<Real>& A, int d) {
+        constexpr int FC = gather_chunk_fields<Real>(NFLD);
+        return A.gather.contrib + ((size_t)(d / FC) * A.gather.chunk_units + d % FC) * 3;
     }
+    static __device__ __forceinline__ void touch(const Real* base, uint32_t q, bool on, Real (&x)[3]) {
+        const Real* p = base + (size_t)q * 3;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) x[k] = on ? __ldg(p + k) : Real(0);
+    }
+    __device__ __forceinline__ void load(const NodeArgs<Real>& A, long long g, int d, const uint4& t, bool add) {
+        const Real* base = touches(A, d);
+        touch(base, t.x, t.x != kNoTouch, c[0]);
+        touch(base, t.y, t.y != kNoTouch, c[1]);
+        touch(base, t.z, t.z != kNoTouch, c[2]);
+        touch(base, t.w, !(t.w & kMoreTouches), c[3]);
+        old[0] = old[1] = old[2] = Real(0);
+        if (add) load4(A.force + ((size_t)g * NFLD + d) * 4, old);
+    }
+    __device__ __forceinline__ void sum(const NodeArgs<Real>& A, int d, const uint4& t, Real (&fv)[3]) const {
+        Real s[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            s[k] = c[0][k] + c[1][k];
+            s[k] += c[2][k];
+            s[k] += c[3][k];
+        }
+        if ((t.w & kMoreTouches) && t.w != kNoTouch) {
+            const Real* base = touches(A, d);
+            const uint4* m = A.gather.more + (t.w & ~kMoreTouches);
+            bool on = true;
+            while (on) {
+                const uint4 q = __ldg(m++);
+                on = (q.x & kMoreTouches) != 0;
+                Real x[4][3];
+                touch(base, q.x & ~kMoreTouches, true, x[0]);
+                touch(base, q.y, q.y != kNoTouch, x[1]);
+                touch(base, q.z, q.z != kNoTouch, x[2]);
+                touch(base, q.w, q.w != kNoTouch, x[3]);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    s[k] += x[0][k];
+                    s[k] += x[1][k];
+                    s[k] += x[2][k];
+                    s[k] += x[3][k];
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) fv[k] = old[k] + s[k];
+    }
+};
+
+// Node pass: one thread per (node, wavefield), the wavefields of a node in
+// adjacent threads, so a warp reads and writes whole rows of u, v, a and of a
+// cell's contributions.  A warp takes 32 nodes at a time, every load of a
+// thread issued before its first store; their touches and C-PML coefficients, which the other addresses wait
+// for, come through the warp's own shared memory two tiles ahead (cp.async),
+// so the warps run without block barriers.  With node-form C-PML the pass is
+// two launches over contiguous node ranges: node_update_kernel over the plain
+// nodes [g0, n_node), node_pml_kernel over the C-PML nodes [0, g0).
+constexpr int kNodeThreads = 128, kNodeTile = 32;
+
+template <typename Real, int NFLD, bool MULTI, bool PML, bool HALF_V>
+__device__ __forceinline__ void node_pass(const NodeArgs<Real>& A, const NodePml<Real>& P, long long g0, long long g1) {
+    constexpr int TN = kNodeTile, WARPS = kNodeThreads / 32;
+    constexpr int COEF_W = 16 / (int)sizeof(Real), COEF_N = PML ? TN * 14 : COEF_W;
+    __shared__ __align__(16) uint4 s_touch[WARPS][3][TN];
+    __shared__ __align__(16) Real s_cf[PML ? WARPS : 1][3][COEF_N];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const bool gather = A.gather.touch != nullptr;
+    const long long n_tile = (g1 - g0 + TN - 1) / TN;
+    const long long step = (long long)gridDim.x * WARPS;
+    auto fetch = [&](long long tile, int st) {
+        if (tile < n_tile) {
+            const long long b = g0 + tile * TN;
+            const int n = (int)min((long long)TN, g1 - b);
+            if (gather && lane < n) cp_async16(&s_touch[wp][st][lane], A.gather.touch + b + lane);
+            if (PML)  // the coefficient array is padded to whole copies
+                for (int i = lane; i * COEF_W < n * 14; i += 32)
+                    cp_async16(&s_cf[PML ? wp : 0][st][i * COEF_W], P.coef + b * 14 + i * COEF_W);
+        }
+        cp_async_commit();
+    };
+    ModelConst K;
+    bool full, add = false;
+    if (!MULTI) {
+        node_constants<Real, MULTI>(A, P, 0, K, full);
+        add = A.gather.keep && A.gather.mdirect && __ldg(A.gather.mdirect) == 0;
+    }
+    const long long first = (long long)blockIdx.x * WARPS + wp;
+    fetch(first, 0);
+    fetch(first + step, 1);
+    int st = 0;
+    for (long long tile = first; tile < n_tile; tile += step) {
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        __syncwarp();  // this tile's tables; and every lane is done with the tile before
+        fetch(tile + 2 * step, st >= 1 ? st - 1 : 2);
+        const long long b = g0 + tile * TN;
+        const int n = (int)min((long long)TN, g1 - b) * NFLD;
+#pragma unroll 1
+        for (int r = 0; r < NFLD; ++r) {
+            const int s = r * 32 + lane;
+            if (s >= n) continue;
+            const int gl = s / NFLD, d = s - gl * NFLD;
+            const long long g = b + gl;
+            if (MULTI && !node_constants<Real, MULTI>(A, P, g, K, full)) continue;
+            const uint4 t = s_touch[wp][st][gl];
+            const Real* cf = &s_cf[PML ? wp : 0][st][PML ? gl * 14 : 0];
+            NodeField<Real, NFLD, PML, HALF_V> x;
+            ForceParts<Real, NFLD> p;
+            if (gather) {
+                if (MULTI)
+                    add = A.gather.keep && A.gather.mdirect && __ldg(A.gather.mdirect + __ldg(A.node_model + g)) == 0;
+                p.load(A, g, d, t, add);
+            } else {
+                load4(A.force + ((size_t)g * NFLD + d) * 4, p.old);
+            }
+            x.load(A, P, g, d, true, cf);
+            Real fv[3] = {p.old[0], p.old[1], p.old[2]};
+            if (gather) p.sum(A, d, t, fv);
+            x.finish(A, P, g, d, true, cf, fv, K, full);
+            if (A.gather.keep) store4(A.force + ((size_t)g * NFLD + d) * 4, fv[0], fv[1], fv[2], Real(0));
+        }
+        st = st == 2 ? 0 : st + 1;
+    }
+    cp_async_wait_all();
 }
 
+// Resident blocks per SM.  The passes are bound by DRAM and by the loads in
+// flight: on 40 x 40 x 20 cells (1.06 M plain and 1.03 M C-PML nodes, three
+// wavefields) the plain pass takes 102 / 89 / 120 us with 6 / 8 / 10 blocks
+// (72 / 64 / 48 registers, the last with spills), the C-PML pass 157 / 146 /
+// 200 us with 5 / 6 / 8 (96 / 80 / 64), 5.3 and 5.5 TB/s of DRAM traffic at
+// the best.  Three wavefields per thread at once (128 registers) or whole
+// tiles by bulk copies (fewer warps, by shared memory) were slower.
+template <typename Real>
+constexpr int node_blocks_per_sm(bool pml) {
+    return pml ? 6 : (sizeof(Real) == 4 ? 8 : 5);
+}
+
+template <typename Real, int NFLD, bool MULTI, bool HALF_V>
+__global__ void __launch_bounds__(kNodeThreads, node_blocks_per_sm<Real>(false))
+    node_update_kernel(const __grid_constant__ NodeArgs<Real> A, const __grid_constant__ NodePml<Real> P, long long g0) {
+    node_pass<Real, NFLD, MULTI, false, HALF_V>(A, P, g0,
+                                                (MULTI && A.live_node_end) ? min(A.n_node, A.live_node_end[1]) : A.n_node);
+}
+
+template <int NFLD, bool MULTI>
+__global__ void __launch_bounds__(kNodeThreads, node_blocks_per_sm<float>(true))
+    node_pml_kernel(const __grid_constant__ NodeArgs<float> A, const __grid_constant__ NodePml<float> P) {
+    node_pass<float, NFLD, MULTI, true, false>(A, P, 0,
+                                               (MULTI && A.live_node_end) ? min(P.n_slot, A.live_node_end[0]) : P.n_slot);
+}
+
+// The assembled force alone (a learned layer adds to it between the element
+// and the node phase; the autotuner times it).
 template <typename Real, int NFLD, bool MULTI>
-__global__ void __launch_bounds__(256, 2) node_pml_kernel(NodeArgs<Real> A, NodePml<Real> P) {
-    const long long n1 = (MULTI && A.live_node_end) ? min(P.n_slot, A.live_node_end[0]) : P.n_slot;
-    const long long total = n1 * NFLD;
+__global__ void __launch_bounds__(256) assemble_kernel(NodeArgs<Real> A, NodePml<Real> P) {
+    const long long total = A.n_node * NFLD;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
         const long long g = t / NFLD;
@@ -554,10 +769,12 @@ __global__ void __launch_bounds__(256, 2) node_pml_kernel(NodeArgs<Real> A, Node
         ModelConst K;
         bool full;
         if (!node_constants<Real, MULTI>(A, P, g, K, full)) continue;
-        Real fv4[4];
-        load4_nc(A.force + ((size_t)g * NFLD + d) * 4, fv4);
-        const Real fv[3] = {fv4[0], fv4[1], fv4[2]};
-        update_node_field<Real, NFLD, true>(A, P, g, d, fv, (int)g, K, full);
+        const uint4 q = __ldg(A.gather.touch + g);
+        ForceParts<Real, NFLD> p;
+        p.load(A, g, d, q, A.gather.keep && A.gather.mdirect && __ldg(A.gather.mdirect + (MULTI ? __ldg(A.node_model + g) : 0)) == 0);
+        Real fv[3];
+        p.sum(A, d, q, fv);
+        store4(A.force + ((size_t)g * NFLD + d) * 4, fv[0], fv[1], fv[2], Real(0));
     }
 }
 
@@ -641,13 +858,6 @@ static __global__ void live_bounds_kernel(int n_model, int n_colour, const int* 
 // words and are padded so every copy is a 16-byte cp.async.
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
 // Bulk copies (TMA, no tensor map, no multicast) completing on an mbarrier
 // of this block: one thread announces the bytes of a stage and issues its
 // copies; every thread waits for the phase with a bounded poll.
@@ -690,13 +900,25 @@ __device__ __forceinline__ void bulk_copy_g2s(void* smem, const void* gmem, unsi
                  : "memory");
 }
 
+// A chunk of shared memory to global memory, in the issuing thread's current
+// bulk group; bulk_wait_read: the groups committed so far have read their
+// shared memory, bulk_wait_all: and written their global memory.
+__device__ __forceinline__ void bulk_copy_s2g(void* gmem, const void* smem, unsigned bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(gmem), "r"(smem_u32(smem)),
+                 "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
+
 template <typename Real, int NG, int NFLD>
 struct PipeShape {
     static constexpr int NN = NG * NG * NG;
     static constexpr int NNP = (NN + 31) / 32 * 32;
     static constexpr int EPB = NNP <= 32 ? 8 : (NNP <= 64 ? 4 : (NNP <= 128 ? 2 : 1));
     static constexpr int THREADS = NNP * EPB;
-    static constexpr int GEO_B = 12 * NN * (int)sizeof(Real);         // geometry bytes per cell
+    static constexpr int GEO_B = geo_row<Real>(NN) * (int)sizeof(Real); // geometry bytes per cell
     static constexpr int IB_B = ib_row_words(NN) * 4;                  // node-table bytes per cell
     static constexpr int BUF_B = NN * NFLD * 4 * (int)sizeof(Real);    // field vectors per cell
     // a geometry stage also receives the cell's old force vectors once the
@@ -740,26 +962,25 @@ __global__ void __launch_bounds__(PipeShape<Real, NG, NFLD>::THREADS, (sizeof(Re
         constexpr int CI = S::IB_B / 16;
         for (int q = tid; q < EPB * CI; q += THREADS) {
             const int c = q / CI, r = q - c * CI;
-            const int e = A.e_begin + grp * EPB + c;
-            if (e < A.e_end)
+            const int x = A.e_begin + grp * EPB + c;
+            if (x < A.e_end)
                 cp_async16(reinterpret_cast<unsigned char*>(ib_of(st, c)) + r * 16,
-                           reinterpret_cast<const unsigned char*>(ibool_padded) + (size_t)e * S::IB_B + r * 16);
+                           reinterpret_cast<const unsigned char*>(ibool_padded) + (size_t)__ldg(A.cells + x) * S::IB_B + r * 16);
         }
     };
     auto issue_geo = [&](int grp, int st) {
         constexpr int CG = S::GEO_B / 16;
         for (int q = tid; q < EPB * CG; q += THREADS) {
             const int c = q / CG, r = q - c * CG;
-            const int e = A.e_begin + grp * EPB + c;
-            if (e < A.e_end)
+            const int x = A.e_begin + grp * EPB + c;
+            if (x < A.e_end)
                 cp_async16(reinterpret_cast<unsigned char*>(geo_of(st, c)) + r * 16,
-                           reinterpret_cast<const unsigned char*>(A.geom) + (size_t)e * S::GEO_B + r * 16);
+                           reinterpret_cast<const unsigned char*>(A.geom) + (size_t)__ldg(A.cells + x) * S::GEO_B + r * 16);
         }
     };
     // this point's predicted-displacement vectors (node table in stage ist)
     auto issue_gather = [&](int grp, int ist, int bs) {
-        const int e = A.e_begin + grp * EPB + el;
-        if (e >= A.e_end || p >= NN) return;
+        if (A.e_begin + grp * EPB + el >= A.e_end || p >= NN) return;
         const uint32_t g = ib_of(ist, el)[p] & kNodeMask;
 #pragma unroll
         for (int d = 0; d < NFLD; ++d)
@@ -788,21 +1009,21 @@ __global__ void __launch_bounds__(PipeShape<Real, NG, NFLD>::THREADS, (sizeof(Re
         const int cur = it & 1, ist = it % 3;
         cp_async_wait_all();
         __syncthreads();  // vectors + geometry of this group, node table of the next
-        const int e = A.e_begin + grp * EPB + el;
-        const int mdl = (e < A.e_end) ? (int)ib_of(ist, el)[NN] : 0;
-        const bool active = (e < A.e_end) && (p < NN) && (!A.mlive || __ldg(A.mlive + mdl));
+        const bool in = A.e_begin + grp * EPB + el < A.e_end;
+        const int e = in ? __ldg(A.cells + A.e_begin + grp * EPB + el) : 0;
+        const int mdl = in ? (int)ib_of(ist, el)[NN] : 0;
+        const bool active = in && (p < NN) && (!A.mlive || __ldg(A.mlive + mdl));
         const uint32_t first_bit = (!A.mdirect || __ldg(A.mdirect + mdl)) ? kFirstTouch : 0u;
         Real* geo = geo_of(cur, el);
         Real* buf = buf_of(cur, el);
         uint32_t gword = 0;
-        Real dd[9], jw = Real(0), lam = Real(0), mu = Real(0);
+        Real dd[9], lam = Real(0), mu = Real(0);
         if (active) {
             gword = ib_of(ist, el)[p];
 #pragma unroll
             for (int q = 0; q < 9; ++q) dd[q] = geo[q * NN + p];
-            jw = geo[9 * NN + p];
-            lam = geo[10 * NN + p];
-            mu = geo[11 * NN + p];
+            lam = geo[9 * NN + p];
+            mu = geo[10 * NN + p];
         }
         __syncthreads();  // geometry stage now takes this group's old force vectors
         if (active && !(gword & first_bit)) {
@@ -827,7 +1048,7 @@ __global__ void __launch_bounds__(PipeShape<Real, NG, NFLD>::THREADS, (sizeof(Re
         for (int d = 0; d < NFLD; ++d)
 #pragma unroll
             for (int q = 0; q < 6; ++q) st[d][q] = Real(0);
-        if (active && mu > Real(0)) {  // element_cpu.cpp:42-43: mu <= 0 adds nothing
+        if (active) {
 #pragma unroll
             for (int d = 0; d < NFLD; ++d) {
                 Real gx[3] = {0, 0, 0}, gy[3] = {0, 0, 0}, gz[3] = {0, 0, 0};
@@ -872,9 +1093,9 @@ __global__ void __launch_bounds__(PipeShape<Real, NG, NFLD>::THREADS, (sizeof(Re
                 const Real ea = dd[a], eb = dd[3 + a], ec = dd[6 + a];
 #pragma unroll
                 for (int d = 0; d < NFLD; ++d)
-                    store4(buf + (p * NFLD + d) * 4, jw * (st[d][0] * ea + st[d][3] * eb + st[d][4] * ec),
-                           jw * (st[d][3] * ea + st[d][1] * eb + st[d][5] * ec),
-                           jw * (st[d][4] * ea + st[d][5] * eb + st[d][2] * ec), Real(0));
+                    store4(buf + (p * NFLD + d) * 4, st[d][0] * ea + st[d][3] * eb + st[d][4] * ec,
+                           st[d][3] * ea + st[d][1] * eb + st[d][5] * ec,
+                           st[d][4] * ea + st[d][5] * eb + st[d][2] * ec, Real(0));
             }
             __syncthreads();
             if (active) {
@@ -997,22 +1218,6 @@ __global__ void __launch_bounds__(PipeShape<Real, NG, NFLD>::THREADS, (sizeof(Re
 // the kernel parameters (constant bank); those indexed by the thread's own j
 // and k are kept in registers.
 //
-// XCH (line owners): instead of every thread reading the five eta and five
-// zeta neighbours of each of its points (30 shared loads per point for the
-// gradient, 30 for the divergence), the thread with column (j, k) also owns
-// the eta line (i = j, k) and the zeta line (i = k, j) of its (cell,
-// wavefield): it reads the line, contracts it with D in registers and
-// writes the derivative back in place, so a point costs one shared load per
-// direction and component afterwards.  Phases per group: own points'
-// displacement into both arrays | line contractions | gradient, stress and
-// fluxes (the eta and zeta fluxes replace the derivatives in place) | line
-// contractions of the fluxes | divergence and assembly; four barriers instead
-// of two, and 40 % fewer shared-memory wavefronts.  The arrays' point layout
-// (PIE, PIZ) and slot stride SP put a warp's own-point accesses and its
-// line accesses in distinct banks.  The eta and zeta sums of the divergence
-// are added in another order than in the default layout, so the two agree
-// to rounding, not bit for bit.
-//
 // Pipelining: the geometry of the next group and the node table of the one
 // after are bulk copies (TMA engine, one per cell, issued by one thread and
 // completing on a per-stage mbarrier) into rotating shared stages; the
@@ -1029,10 +1234,7 @@ __host__ __device__ constexpr int col_default_epb(int ng, int nfld) {
     return (150 / (nfld * ng * ng)) > 0 ? 150 / (nfld * ng * ng) : 1;
 }
 
-// XCH: the eta and zeta contractions done by line owners (see
-// elem_col_kernel) in two [3][GR][SP] arrays laid out point (i, j, k) ->
-// PI*i + NG*j + k with PI = PIE (eta array) or PIZ (zeta array).
-template <int NG, int NFLD, int EPB_ = col_default_epb(NG, NFLD), bool XCH = false>
+template <int NG, int NFLD, int EPB_ = col_default_epb(NG, NFLD)>
 struct ColShape {
     static constexpr int NN = NG * NG * NG;
     static constexpr int NG2 = NG * NG;
@@ -1040,16 +1242,13 @@ struct ColShape {
     static constexpr int GR = EPB * NFLD;                 // (cell, wavefield) lines per group
     static constexpr int ACTIVE = GR * NG2;               // threads with work
     static constexpr int THREADS = (ACTIVE + 31) / 32 * 32;
-    // at NG = 5 (PIE, PIZ, SP) = (37, 33, 185): the own-point accesses and
-    // the eta- (zeta-) line accesses of a warp fall in distinct banks
-    static constexpr int PIE = NG2 + 12, PIZ = NG2 + 8;
-    static constexpr int SP = XCH ? NG * PIE : NN + ((NG2 - NN) % 32 + 32) % 32;  // >= NN, == NG2 (mod 32)
-    static constexpr int GEO_B = 12 * NN * 4;
+    static constexpr int SP = NN + ((NG2 - NN) % 32 + 32) % 32;  // >= NN, == NG2 (mod 32)
+    static constexpr int GEO_B = geo_row<float>(NN) * 4;
     static constexpr int GEO_W = GEO_B / 4;
     static constexpr int GEO_SLOT = GEO_B + 4 * (((24 - GEO_W) % 32 + 32) % 32 / 4 * 4);
     static constexpr int IB_B = ib_row_words(NN) * 4;
     static constexpr int ARR = 3 * GR * SP;               // floats of one [3][GR][SP] array
-    static constexpr int N_ARR = XCH ? 2 : 3;
+    static constexpr int N_ARR = 3;
     // dynamic shared memory without the per-model values (col_model_smem)
     static constexpr int SMEM = 2 * EPB * GEO_SLOT + 3 * EPB * IB_B + (N_ARR * ARR + 64) * 4;
     static constexpr int MIN_BLOCKS = THREADS <= 160 ? 3 : 2;
@@ -1057,7 +1256,8 @@ struct ColShape {
 };
 
 struct ColArgs {
-    int e_begin, e_end, n_groups;
+    int e_begin, e_end, n_groups;  // range of `cells`
+    const int* cells;              // the cells colour after colour
     const int* live_end;           // [colour] end of the stepping cells (several models), or null
     int colour;
     const uint32_t* ibool_padded;  // [cell][ib_row_words(NN)]: node words, model index
@@ -1084,10 +1284,10 @@ struct ColArgs {
 // function values [n_model][n_set], live and full-force flags [n_model].
 __host__ __device__ constexpr int col_model_smem(int n_model, int n_set) { return (n_model * n_set + 2 * n_model) * 4; }
 
-template <int NG, int NFLD, int EPB_, bool XCH = false>
-__global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_, XCH>::THREADS, ColShape<NG, NFLD, EPB_, XCH>::MIN_BLOCKS)
+template <int NG, int NFLD, int EPB_>
+__global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_>::THREADS, ColShape<NG, NFLD, EPB_>::MIN_BLOCKS)
     elem_col_kernel(ColArgs A) {
-    using S = ColShape<NG, NFLD, EPB_, XCH>;
+    using S = ColShape<NG, NFLD, EPB_>;
     constexpr int NN = S::NN, NG2 = S::NG2, EPB = S::EPB, GR = S::GR, SP = S::SP;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char* gbase = smem_raw;
@@ -1096,10 +1296,6 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_, XCH>::THREADS, ColSha
     float* fe = us + S::ARR;                                          // [3][GR][SP] eta flux
     float* fz = fe + S::ARR;                                          // [3][GR][SP] zeta flux
     float* sD = us + S::N_ARR * S::ARR;
-    // XCH: [3][GR][SP] eta and zeta arrays (u, then its derivative, the
-    // flux, then the flux's contraction, each in place)
-    float* xe = us;
-    float* xz = us + S::ARR;
 
     // cells of this colour that still step (several models: the cells past
     // the last one of a live model belong to finished models)
@@ -1163,7 +1359,7 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_, XCH>::THREADS, ColSha
         mbar_expect_tx(&s_bar[st], (unsigned)(nc * S::GEO_B));
         for (int c = 0; c < nc; ++c)
             bulk_copy_g2s(gbase + (st * EPB + c) * S::GEO_SLOT,
-                          reinterpret_cast<const unsigned char*>(A.geom) + (size_t)(e0 + c) * S::GEO_B, S::GEO_B,
+                          reinterpret_cast<const unsigned char*>(A.geom) + (size_t)__ldg(A.cells + e0 + c) * S::GEO_B, S::GEO_B,
                           &s_bar[st]);
     };
     auto tma_ib = [&](int grp, int st) {
@@ -1173,7 +1369,7 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_, XCH>::THREADS, ColSha
         mbar_expect_tx(&s_bar[2 + st], (unsigned)(nc * S::IB_B));
         for (int c = 0; c < nc; ++c)
             bulk_copy_g2s(ibase + (st * EPB + c) * S::IB_B,
-                          reinterpret_cast<const unsigned char*>(A.ibool_padded) + (size_t)(e0 + c) * S::IB_B,
+                          reinterpret_cast<const unsigned char*>(A.ibool_padded) + (size_t)__ldg(A.cells + e0 + c) * S::IB_B,
                           S::IB_B, &s_bar[2 + st]);
     };
     // a wait that gave up: flag it, give the copies in flight a second
@@ -1208,16 +1404,9 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_, XCH>::THREADS, ColSha
     const int ubase = line * SP + col;        // + c*GR*SP + i*NG2
     const int ebase = line * SP + col - j * NG;  // + s*NG  (eta line: i*NG2 + s*NG + k)
     const int zbase = line * SP + j * NG;        // + s     (zeta line: i*NG2 + j*NG + s)
-    // XCH: own points (i, j, k) at xown + i*PI; the eta line this thread owns
-    // is (i = j, k = k) of its (cell, wavefield): points xline_e + s*NG; the
-    // zeta line is (i = k, j = j): points xline_z + s
-    const int xown_e = line * SP + j * NG + k, xown_z = xown_e;
-    const int xline_e = line * SP + j * S::PIE + k;
-    const int xline_z = line * SP + k * S::PIZ + j * NG;
-
     int it = 0;
     for (int grp = grp0; grp < n_groups; grp += G, ++it) {
-        const int e = A.e_begin + grp * EPB + cl;
+        const int x = A.e_begin + grp * EPB + cl;  // of A.cells
         const int mdl = pre_ok ? (int)ib_of(it % 3, cl)[NN] : 0;
         const bool act = pre_ok && s_live[mdl];
         // first touch stores only on a full-force step; by increments
@@ -1232,18 +1421,9 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_, XCH>::THREADS, ColSha
             u1[i] = pre[i].y;
             u2[i] = pre[i].z;
             if (act) {
-                if constexpr (XCH) {
-                    xe[0 * GR * SP + xown_e + i * S::PIE] = u0[i];
-                    xe[1 * GR * SP + xown_e + i * S::PIE] = u1[i];
-                    xe[2 * GR * SP + xown_e + i * S::PIE] = u2[i];
-                    xz[0 * GR * SP + xown_z + i * S::PIZ] = u0[i];
-                    xz[1 * GR * SP + xown_z + i * S::PIZ] = u1[i];
-                    xz[2 * GR * SP + xown_z + i * S::PIZ] = u2[i];
-                } else {
-                    us[0 * GR * SP + ubase + i * NG2] = u0[i];
-                    us[1 * GR * SP + ubase + i * NG2] = u1[i];
-                    us[2 * GR * SP + ubase + i * NG2] = u2[i];
-                }
+                us[0 * GR * SP + ubase + i * NG2] = u0[i];
+                us[1 * GR * SP + ubase + i * NG2] = u1[i];
+                us[2 * GR * SP + ubase + i * NG2] = u2[i];
             }
         }
         const int nx = grp + G;
@@ -1273,7 +1453,7 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_, XCH>::THREADS, ColSha
                 }
         }
         const float stf = act ? s_stf[mdl * A.n_set + fs] : 0.f;
-        const int src = (act && stf != 0.f && A.src_head) ? __ldg(A.src_head + e) : -1;
+        const int src = (act && stf != 0.f && A.src_head) ? __ldg(A.src_head + __ldg(A.cells + x)) : -1;
         pre_ok = line_nodes(nx, (it + 1) % 3, nw);
         load_vectors(nw, pre_ok, pre);
 
@@ -1286,36 +1466,6 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_, XCH>::THREADS, ColSha
                             ? *(reinterpret_cast<const float4*>(A.force) + (size_t)(cw[i] & kNodeMask) * NFLD + fld)
                             : make_float4(0.f, 0.f, 0.f, 0.f);
         };
-        if constexpr (XCH) {
-            // line owners: d/d-eta along this thread's eta line and d/d-zeta
-            // along its zeta line, in place (the lines of a (cell, wavefield)
-            // are disjoint; the two arrays hold the same displacement)
-            if (act) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    float* le = xe + c * GR * SP + xline_e;
-                    float* lz = xz + c * GR * SP + xline_z;
-                    float ve[NG], vz[NG];
-#pragma unroll
-                    for (int t = 0; t < NG; ++t) {
-                        ve[t] = le[t * NG];
-                        vz[t] = lz[t];
-                    }
-#pragma unroll
-                    for (int s2 = 0; s2 < NG; ++s2) {
-                        float de = 0.f, dz = 0.f;
-#pragma unroll
-                        for (int t = 0; t < NG; ++t) {
-                            de += A.D[s2 * NG + t] * ve[t];
-                            dz += A.D[s2 * NG + t] * vz[t];
-                        }
-                        le[s2 * NG] = de;
-                        lz[s2] = dz;
-                    }
-                }
-            }
-            __syncthreads();  // the eta and zeta derivatives of the whole group
-        }
         // gradient, stress and the three fluxes at each point of the line
         float fx0[NG], fx1[NG], fx2[NG];
         const float* geo = geo_of(it & 1, cl);
@@ -1327,7 +1477,7 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_, XCH>::THREADS, ColSha
             float dd[9];
 #pragma unroll
             for (int q = 0; q < 9; ++q) dd[q] = geo[q * NN + p];
-            const float jw = geo[9 * NN + p], lam = geo[10 * NN + p], mu = geo[11 * NN + p];
+            const float lam = geo[9 * NN + p], mu = geo[10 * NN + p];
             float gx[3] = {0.f, 0.f, 0.f}, gy[3] = {0.f, 0.f, 0.f}, gz[3] = {0.f, 0.f, 0.f};
 #pragma unroll
             for (int s = 0; s < NG; ++s) {
@@ -1336,98 +1486,49 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_, XCH>::THREADS, ColSha
                 gx[1] += Di * u1[s];
                 gx[2] += Di * u2[s];
             }
-            if constexpr (XCH) {
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    gy[c] = xe[c * GR * SP + xown_e + i * S::PIE];
-                    gz[c] = xz[c * GR * SP + xown_z + i * S::PIZ];
-                }
-            } else {
+            for (int c = 0; c < 3; ++c) {
+                const float* uc = us + c * GR * SP + i * NG2;
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const float* uc = us + c * GR * SP + i * NG2;
-#pragma unroll
-                    for (int s = 0; s < NG; ++s) {
-                        gy[c] += Dj[s] * uc[ebase + s * NG];
-                        gz[c] += Dk[s] * uc[zbase + s];
-                    }
+                for (int s = 0; s < NG; ++s) {
+                    gy[c] += Dj[s] * uc[ebase + s * NG];
+                    gz[c] += Dk[s] * uc[zbase + s];
                 }
             }
-            float st0 = 0.f, st1 = 0.f, st2 = 0.f, st3 = 0.f, st4 = 0.f, st5 = 0.f;
-            if (mu > 0.f) {  // element_cpu.cpp:42-43: mu <= 0 adds nothing
-                float gr[3][3];
+            float gr[3][3];
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    gr[c][0] = gx[c] * dd[0] + gy[c] * dd[1] + gz[c] * dd[2];
-                    gr[c][1] = gx[c] * dd[3] + gy[c] * dd[4] + gz[c] * dd[5];
-                    gr[c][2] = gx[c] * dd[6] + gy[c] * dd[7] + gz[c] * dd[8];
-                }
-                const float tr = gr[0][0] + gr[1][1] + gr[2][2];
-                const float m2 = 2.f * mu;
-                st0 = m2 * gr[0][0] + lam * tr;
-                st1 = m2 * gr[1][1] + lam * tr;
-                st2 = m2 * gr[2][2] + lam * tr;
-                st3 = m2 * (0.5f * (gr[0][1] + gr[1][0]));
-                st4 = m2 * (0.5f * (gr[0][2] + gr[2][0]));
-                st5 = m2 * (0.5f * (gr[1][2] + gr[2][1]));
+            for (int c = 0; c < 3; ++c) {
+                gr[c][0] = gx[c] * dd[0] + gy[c] * dd[1] + gz[c] * dd[2];
+                gr[c][1] = gx[c] * dd[3] + gy[c] * dd[4] + gz[c] * dd[5];
+                gr[c][2] = gx[c] * dd[6] + gy[c] * dd[7] + gz[c] * dd[8];
             }
-            // flux along axis a: jw * sigma . (dd[a], dd[3+a], dd[6+a])
-            fx0[i] = jw * (st0 * dd[0] + st3 * dd[3] + st4 * dd[6]);
-            fx1[i] = jw * (st3 * dd[0] + st1 * dd[3] + st5 * dd[6]);
-            fx2[i] = jw * (st4 * dd[0] + st5 * dd[3] + st2 * dd[6]);
-            const float e0 = jw * (st0 * dd[1] + st3 * dd[4] + st4 * dd[7]);
-            const float e1 = jw * (st3 * dd[1] + st1 * dd[4] + st5 * dd[7]);
-            const float e2 = jw * (st4 * dd[1] + st5 * dd[4] + st2 * dd[7]);
-            const float z0 = jw * (st0 * dd[2] + st3 * dd[5] + st4 * dd[8]);
-            const float z1 = jw * (st3 * dd[2] + st1 * dd[5] + st5 * dd[8]);
-            const float z2 = jw * (st4 * dd[2] + st5 * dd[5] + st2 * dd[8]);
-            if constexpr (XCH) {  // own points: the derivatives read above are replaced
-                xe[0 * GR * SP + xown_e + i * S::PIE] = e0;
-                xe[1 * GR * SP + xown_e + i * S::PIE] = e1;
-                xe[2 * GR * SP + xown_e + i * S::PIE] = e2;
-                xz[0 * GR * SP + xown_z + i * S::PIZ] = z0;
-                xz[1 * GR * SP + xown_z + i * S::PIZ] = z1;
-                xz[2 * GR * SP + xown_z + i * S::PIZ] = z2;
-            } else {
-                fe[0 * GR * SP + ubase + i * NG2] = e0;
-                fe[1 * GR * SP + ubase + i * NG2] = e1;
-                fe[2 * GR * SP + ubase + i * NG2] = e2;
-                fz[0 * GR * SP + ubase + i * NG2] = z0;
-                fz[1 * GR * SP + ubase + i * NG2] = z1;
-                fz[2 * GR * SP + ubase + i * NG2] = z2;
-            }
+            const float tr = gr[0][0] + gr[1][1] + gr[2][2];
+            const float m2 = 2.f * mu;
+            const float st0 = m2 * gr[0][0] + lam * tr;
+            const float st1 = m2 * gr[1][1] + lam * tr;
+            const float st2 = m2 * gr[2][2] + lam * tr;
+            const float st3 = mu * (gr[0][1] + gr[1][0]);
+            const float st4 = mu * (gr[0][2] + gr[2][0]);
+            const float st5 = mu * (gr[1][2] + gr[2][1]);
+            // flux along axis a: sigma . (dd[a], dd[3+a], dd[6+a])
+            fx0[i] = (st0 * dd[0] + st3 * dd[3] + st4 * dd[6]);
+            fx1[i] = (st3 * dd[0] + st1 * dd[3] + st5 * dd[6]);
+            fx2[i] = (st4 * dd[0] + st5 * dd[3] + st2 * dd[6]);
+            const float e0 = (st0 * dd[1] + st3 * dd[4] + st4 * dd[7]);
+            const float e1 = (st3 * dd[1] + st1 * dd[4] + st5 * dd[7]);
+            const float e2 = (st4 * dd[1] + st5 * dd[4] + st2 * dd[7]);
+            const float z0 = (st0 * dd[2] + st3 * dd[5] + st4 * dd[8]);
+            const float z1 = (st3 * dd[2] + st1 * dd[5] + st5 * dd[8]);
+            const float z2 = (st4 * dd[2] + st5 * dd[5] + st2 * dd[8]);
+            fe[0 * GR * SP + ubase + i * NG2] = e0;
+            fe[1 * GR * SP + ubase + i * NG2] = e1;
+            fe[2 * GR * SP + ubase + i * NG2] = e2;
+            fz[0 * GR * SP + ubase + i * NG2] = z0;
+            fz[1 * GR * SP + ubase + i * NG2] = z1;
+            fz[2 * GR * SP + ubase + i * NG2] = z2;
         }
         load_old_force();
         __syncthreads();  // fluxes of the whole group
-        if constexpr (XCH) {
-            // line owners: the eta (zeta) contraction of the divergence along
-            // this thread's eta (zeta) line, in place
-            if (act) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    float* le = xe + c * GR * SP + xline_e;
-                    float* lz = xz + c * GR * SP + xline_z;
-                    float ve[NG], vz[NG];
-#pragma unroll
-                    for (int t = 0; t < NG; ++t) {
-                        ve[t] = le[t * NG];
-                        vz[t] = lz[t];
-                    }
-#pragma unroll
-                    for (int s2 = 0; s2 < NG; ++s2) {
-                        float de = 0.f, dz = 0.f;
-#pragma unroll
-                        for (int t = 0; t < NG; ++t) {
-                            de += A.D[t * NG + s2] * ve[t];
-                            dz += A.D[t * NG + s2] * vz[t];
-                        }
-                        le[s2 * NG] = de;
-                        lz[s2] = dz;
-                    }
-                }
-            }
-            __syncthreads();  // contractions of the whole group
-        }
         if (act) {
 #pragma unroll
             for (int i = 0; i < NG; ++i) {
@@ -1440,22 +1541,14 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_, XCH>::THREADS, ColSha
                     r[1] += Ti * fx1[s];
                     r[2] += Ti * fx2[s];
                 }
-                if constexpr (XCH) {
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        r[c] += xe[c * GR * SP + xown_e + i * S::PIE];
-                        r[c] += xz[c * GR * SP + xown_z + i * S::PIZ];
-                    }
-                } else {
+                for (int c = 0; c < 3; ++c) {
+                    const float* ec = fe + c * GR * SP + i * NG2;
+                    const float* zc = fz + c * GR * SP + i * NG2;
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const float* ec = fe + c * GR * SP + i * NG2;
-                        const float* zc = fz + c * GR * SP + i * NG2;
-#pragma unroll
-                        for (int s = 0; s < NG; ++s) {
-                            r[c] += Tj[s] * ec[ebase + s * NG];
-                            r[c] += Tk[s] * zc[zbase + s];
-                        }
+                    for (int s = 0; s < NG; ++s) {
+                        r[c] += Tj[s] * ec[ebase + s * NG];
+                        r[c] += Tk[s] * zc[zbase + s];
                     }
                 }
                 r[0] = -r[0];
@@ -1477,6 +1570,420 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_, XCH>::THREADS, ColSha
             }
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// elem_gather_kernel: the element kernel of the time loop (both precisions).
+//
+// A group of WARPS warps takes CELLS cells at a time and leaves their force
+// contributions in contrib; the node pass adds them up (NodeGather).  Against a read-modify-write of the assembled force colour
+// after colour this stores 4 (8) bytes per value in whole rows instead of
+// reading and writing 16-byte vectors node by node, needs one launch instead
+// of one per colour, and takes the cells in mesh order, so the predicted
+// displacement of the nodes that neighbours share comes from L2.
+//
+// One thread per xi-line: the NG points (i = 0..NG-1, j, k) of a cell, for one
+// wavefield after the other, so the geometry is fetched once for all of them
+// and the wavefield count is a run-time value.  The xi contractions run on
+// registers.  For the eta and zeta contractions the thread with column (j, k)
+// also owns the eta line (i = j, k) and the zeta line (i = k, j): it reads the
+// line from shared memory, contracts it with D (constant bank) and writes the
+// result back in place.  Phases per wavefield: own displacements into both
+// arrays | line contractions | gradient, stress, fluxes in place | line
+// contractions | divergence and store.  With one warp per group (NG <= 5; 25
+// of 32 lanes at NG = 5) the phases are separated by warp-level barriers only
+// and the warps of a block run independently, which hides the exchange's
+// latency better than full lanes behind block barriers.
+//
+// A group's geometry is a bulk copy (TMA engine) on an mbarrier, issued as
+// soon as the last wavefield of the previous group has read the stage; the
+// node words two groups and the displacement vectors one wavefield ahead are
+// register loads.  The contributions of a chunk of wavefields are collected in
+// shared memory and leave as one bulk store per cell.
+// ---------------------------------------------------------------------------
+
+// Point (i, j, k) of an exchange array at P*i + NG*j + k, a cell's component
+// S words apart (eta: PE, SE; zeta: PZ, SZ), chosen by enumeration so that a
+// warp's own-point and line accesses fall in distinct banks (4-byte words) or
+// nearly so (8-byte words).
+template <int NG, bool WIDE>
+struct GatherPad;
+template <> struct GatherPad<3, false> { static constexpr int PE = 14, SE = 43, PZ = 27, SZ = 73; };
+template <> struct GatherPad<3, true> { static constexpr int PE = 19, SE = 57, PZ = 17, SZ = 57; };
+template <> struct GatherPad<4, false> { static constexpr int PE = 20, SE = 80, PZ = 17, SZ = 80; };
+template <> struct GatherPad<4, true> { static constexpr int PE = 20, SE = 76, PZ = 17, SZ = 67; };
+template <> struct GatherPad<5, false> { static constexpr int PE = 26, SE = 130, PZ = 25, SZ = 125; };
+template <> struct GatherPad<5, true> { static constexpr int PE = 26, SE = 130, PZ = 26, SZ = 130; };
+template <> struct GatherPad<6, false> { static constexpr int PE = 38, SE = 228, PZ = 49, SZ = 292; };
+template <> struct GatherPad<6, true> { static constexpr int PE = 38, SE = 228, PZ = 41, SZ = 244; };
+
+template <typename Real, int NG>
+struct GatherShape : GatherPad<NG, sizeof(Real) == 8> {
+    using Pad = GatherPad<NG, sizeof(Real) == 8>;
+    static constexpr int NN = NG * NG * NG, NG2 = NG * NG;
+    static constexpr int WARPS = NG2 <= 32 ? 1 : 4;        // warps of a group
+    static constexpr int CELLS = WARPS * 32 / NG2;         // cells of a group
+    static constexpr int GROUPS = WARPS == 1 ? 4 : 1;      // groups of a block
+    static constexpr int THREADS = 32 * WARPS * GROUPS;
+    static constexpr int GEO_B = geo_row<Real>(NN) * (int)sizeof(Real);
+    // several cells per warp: their rows NG2 words apart modulo the banks
+    static constexpr int SKEW = CELLS == 1 ? 0 : ((NG2 * (int)sizeof(Real) - GEO_B) % 128 + 128) % 128 / 16 * 16;
+    static constexpr int GEO_SLOT = GEO_B + SKEW;
+    static constexpr int XCH_B = (3 * CELLS * (Pad::SE + Pad::SZ) * (int)sizeof(Real) + 15) / 16 * 16;
+    // contributions on their way out (FP64: in the eta array, which is free by then)
+    static constexpr int CHUNK_MAX_B = gather_chunk_units<Real>(NN, 3) * 3 * (int)sizeof(Real);
+    static constexpr bool OUT_IN_XCH = sizeof(Real) == 8;
+    static_assert(!OUT_IN_XCH || CHUNK_MAX_B <= 3 * Pad::SE * (int)sizeof(Real), "a chunk fits in the eta array");
+    static constexpr int GROUP_B = CELLS * GEO_SLOT + XCH_B + (OUT_IN_XCH ? 0 : CELLS * CHUNK_MAX_B);
+    static constexpr int SMEM = GROUPS * GROUP_B;
+    // registers: 104 a thread in FP32, 168 in FP64
+    static constexpr int MIN_BLOCKS = (sizeof(Real) == 4 ? 608 : 384) / THREADS;
+};
+
+template <typename Real>
+struct GatherArgs {
+    int n_cell;
+    const int* live_end;           // [1] end of the stepping cells (several models), or null
+    const uint32_t* ibool_padded;  // [cell][ib_row_words(NN)]: node words, model index
+    const Real* geom;              // [cell][geo_row]
+    const Real* ut;                // [node][nfld][4]
+    Real* contrib;                 // [cell][chunk][NN][chunk's fields][3]
+    int nfld;                      // wavefields
+    int nfld_item;                 // wavefields of one work item: nfld, or 1 where the cells alone are too few
+    const int* mlive;              // [model]
+    bool multi;                    // several models
+    // source
+    const int* src_head;
+    const int* src_next;
+    const Real* src_w;
+    const Real* mstf;              // [model][set] source time function value of this step
+    const int* src_set;
+    int n_set;
+    int dir[kMaxFields];
+    int fset[kMaxFields];
+    // C-PML per cell
+    const int* pml_slot;           // [cell] -1 if not a C-PML cell
+    const Real* pml_coef;          // [slot][15][NN]
+    Real* pml_mem;                 // [slot][9*nfld][NN]
+    Real* pml_prev;                // [slot][3*nfld][NN]
+    const double* u;               // [node][3*nfld]
+    const double* v;
+    const Real* a;
+    const ModelConst* mc;          // [model]
+    unsigned* err;                 // set to 1 when a bulk copy's wait gave up (the launch did not finish)
+    Real D[36];                    // D[i*NG+s], read with compile-time indices only
+};
+
+// C-PML of one wavefield at the points of this thread's line (pml.cpp:55-216):
+// the term with last step's memory added to r, then the memory update, which
+// only uses values fixed at the start of the step.
+template <typename Real, int NG>
+__device__ __forceinline__ void line_cell_pml(const GatherArgs<Real>& A, int slot, int mdl, int d, int col,
+                                              const uint32_t (&w)[NG], Real (&r)[3][NG]) {
+    constexpr int NN = NG * NG * NG, NG2 = NG * NG;
+    const double k1 = A.mc[mdl].c1;
+    const Real k2 = (Real)A.mc[mdl].c2;
+    const int F = 3 * A.nfld;
+#pragma unroll
+    for (int i = 0; i < NG; ++i) {
+        const int p = i * NG2 + col;
+        const Real* cf = A.pml_coef + (size_t)slot * 15 * NN + p;
+        Real* mem = A.pml_mem + ((size_t)slot * 3 * F + 9 * d) * NN + p;
+        Real* prev = A.pml_prev + ((size_t)slot * F + 3 * d) * NN + p;
+        const size_t at = (size_t)(w[i] & kNodeMask) * F + 3 * d;
+        Real al[9], ab[5], m[9], pr[3], an[3];
+        double un[3], vn[3];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) al[q] = __ldg(cf + q * NN);
+#pragma unroll
+        for (int q = 0; q < 5; ++q) ab[q] = __ldg(cf + (9 + q) * NN);
+        const Real scale = __ldg(cf + 14 * NN);
+#pragma unroll
+        for (int q = 0; q < 9; ++q) m[q] = mem[q * NN];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            pr[c] = prev[c * NN];
+            un[c] = A.u[at + c];
+            vn[c] = A.v[at + c];
+            an[c] = A.a[at + c];
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const Real nv = Real(un[c] + k1 * vn[c]);
+            const Real ov = pr[c] + k2 * an[c];
+            r[c][i] += scale * (ab[0] * Real(vn[c]) + ab[1] * Real(un[c]) + ab[2] * m[3 * c] + ab[3] * m[3 * c + 1] +
+                                ab[4] * m[3 * c + 2]);
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+                mem[(3 * c + q) * NN] = al[3 * q] * m[3 * c + q] + al[3 * q + 1] * nv + al[3 * q + 2] * ov;
+            prev[c * NN] = nv;
+        }
+    }
+}
+
+template <typename Real, int NG, bool PML>
+__global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Real, NG>::MIN_BLOCKS)
+    elem_gather_kernel(const __grid_constant__ GatherArgs<Real> A) {
+    using S = GatherShape<Real, NG>;
+    constexpr int NN = S::NN, NG2 = S::NG2, CELLS = S::CELLS, PE = S::PE, SE = S::SE, PZ = S::PZ, SZ = S::SZ;
+    constexpr int IB_W = ib_row_words(NN);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t s_bar[S::GROUPS];
+    const int gid = threadIdx.x / (32 * S::WARPS), gt = threadIdx.x - gid * 32 * S::WARPS;
+    unsigned char* geo_b = smem_raw + gid * S::GROUP_B;
+    Real* xe = reinterpret_cast<Real*>(geo_b + CELLS * S::GEO_SLOT);  // [3][CELLS][SE]
+    Real* xz = xe + 3 * CELLS * SE;                                   // [3][CELLS][SZ]
+    Real* stage = S::OUT_IN_XCH ? xe : reinterpret_cast<Real*>(geo_b + CELLS * S::GEO_SLOT + S::XCH_B);
+    uint64_t* bar = s_bar + gid;
+    auto sync = [&]() {
+        if constexpr (S::WARPS == 1) __syncwarp();
+        else __syncthreads();
+    };
+    auto any = [&](bool x) -> bool {
+        if constexpr (S::WARPS == 1) return __any_sync(0xffffffffu, x);
+        else return __syncthreads_or(x);
+    };
+    if (gt == 0) {
+        mbar_init(bar, 1);
+        mbar_init_fence();
+    }
+    __syncthreads();
+
+    const bool lane_ok = gt < CELLS * NG2;
+    const int cl = lane_ok ? gt / NG2 : 0;
+    const int col = lane_ok ? gt - cl * NG2 : 0;
+    const int j = col / NG, k = col - j * NG;
+    const int n_cell = A.live_end ? min(A.n_cell, __ldg(A.live_end)) : A.n_cell;
+    const int split = A.nfld / A.nfld_item;
+    const int fc = gather_chunk_fields<Real>(A.nfld), chunk_u = gather_chunk_units<Real>(NN, A.nfld);
+    const bool staged = A.nfld_item % fc == 0;  // an item fills whole chunks
+    const size_t row_u = (size_t)(A.nfld / fc) * chunk_u;
+    const int n_item = (n_cell + CELLS - 1) / CELLS * split;
+    const int step = gridDim.x * S::GROUPS;
+    const int first = blockIdx.x * S::GROUPS + gid;
+    const Real* geo = reinterpret_cast<const Real*>(geo_b + cl * S::GEO_SLOT);
+    const int own_e = cl * SE + col, own_z = cl * SZ + col;            // + i*PE, i*PZ
+    const int line_e = cl * SE + j * PE + k, line_z = cl * SZ + k * PZ + j * NG;  // + s*NG, + s
+
+    auto copy_geo = [&](int item) {
+        if (gt != 0) return;
+        const int e0 = item / split * CELLS, nc = min(CELLS, n_cell - e0);
+        fence_proxy_async_smem();
+        mbar_expect_tx(bar, (unsigned)(nc * S::GEO_B));
+        for (int c = 0; c < nc; ++c)
+            bulk_copy_g2s(geo_b + c * S::GEO_SLOT, A.geom + (size_t)(e0 + c) * geo_row<Real>(NN), S::GEO_B, bar);
+    };
+    auto cell_of = [&](int item) -> int {  // this thread's cell, -1 without one
+        const int e = item / split * CELLS + cl;
+        return lane_ok && item < n_item && e < n_cell ? e : -1;
+    };
+    auto load_words = [&](int item, uint32_t (&w)[NG]) {
+        const int e = cell_of(item);
+#pragma unroll
+        for (int i = 0; i < NG; ++i) w[i] = e >= 0 ? __ldg(A.ibool_padded + (size_t)e * IB_W + i * NG2 + col) : 0u;
+    };
+    auto load_vectors = [&](const uint32_t (&w)[NG], bool ok, int d, Real (&x)[3][NG]) {
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+            const Real* src = A.ut + ((size_t)(w[i] & kNodeMask) * A.nfld + d) * 4;
+            if constexpr (sizeof(Real) == 4) {
+                const float4 t = ok ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[0][i] = t.x, x[1][i] = t.y, x[2][i] = t.z;
+            } else {
+                const double2 t = ok ? __ldg(reinterpret_cast<const double2*>(src)) : make_double2(0.0, 0.0);
+                x[0][i] = t.x, x[1][i] = t.y, x[2][i] = ok ? __ldg(src + 2) : 0.0;
+            }
+        }
+    };
+
+    uint32_t cw[NG], nw[NG], nw2[NG];  // node words: this item's (C-PML), the next one's, the one's after
+    Real pre[3][NG];                   // displacement of the wavefield to come
+    load_words(first, nw);
+    load_words(first + step, nw2);
+    if (first < n_item) copy_geo(first);
+    load_vectors(nw, cell_of(first) >= 0, first % split * A.nfld_item, pre);
+    unsigned phase = 0;
+    for (int item = first; item < n_item; item += step) {
+        const int e = cell_of(item), next = item + step;
+        const int mdl = A.multi && e >= 0 ? (int)__ldg(A.ibool_padded + (size_t)e * IB_W + NN) : 0;
+        const bool act = e >= 0 && __ldg(A.mlive + mdl) != 0;
+        const int src0 = act && A.src_head ? __ldg(A.src_head + e) : -1;
+        const int slot = PML && act ? __ldg(A.pml_slot + e) : -1;
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+            if (PML) cw[i] = nw[i];
+            nw[i] = nw2[i];
+        }
+        load_words(next + step, nw2);
+        if (any(!mbar_wait(bar, phase))) {
+            // the copy never came: flag it, give it a second bounded wait, leave
+            if (gt == 0) {
+                atomicOr(A.err, 1u);
+                mbar_wait(bar, phase);
+            }
+            return;
+        }
+        phase ^= 1u;
+        const int d0 = item % split * A.nfld_item, d1 = d0 + A.nfld_item;
+        for (int d = d0; d < d1; ++d) {
+            Real u[3][NG];
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int i = 0; i < NG; ++i) {
+                    u[c][i] = pre[c][i];
+                    if (lane_ok) {
+                        xe[c * CELLS * SE + own_e + i * PE] = u[c][i];
+                        xz[c * CELLS * SZ + own_z + i * PZ] = u[c][i];
+                    }
+                }
+            sync();
+            if (d + 1 < d1) {
+                // the same cells' next wavefield: the words are PML's cw or read again
+                if constexpr (PML) {
+                    load_vectors(cw, e >= 0, d + 1, pre);
+                } else {
+                    uint32_t w[NG];
+                    load_words(item, w);
+                    load_vectors(w, e >= 0, d + 1, pre);
+                }
+            } else {
+                load_vectors(nw, cell_of(next) >= 0, next % split * A.nfld_item, pre);
+            }
+            // the eta and zeta derivatives along this thread's lines, in place
+            auto contract = [&](auto coef) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    Real* le = xe + c * CELLS * SE + line_e;
+                    Real* lz = xz + c * CELLS * SZ + line_z;
+                    Real ve[NG], vz[NG];
+#pragma unroll
+                    for (int t = 0; t < NG; ++t) {
+                        ve[t] = le[t * NG];
+                        vz[t] = lz[t];
+                    }
+#pragma unroll
+                    for (int s2 = 0; s2 < NG; ++s2) {
+                        Real de = Real(0), dz = Real(0);
+#pragma unroll
+                        for (int t = 0; t < NG; ++t) {
+                            de += coef(s2, t) * ve[t];
+                            dz += coef(s2, t) * vz[t];
+                        }
+                        le[s2 * NG] = de;
+                        lz[s2] = dz;
+                    }
+                }
+            };
+            if (lane_ok) contract([&](int s2, int t) { return A.D[s2 * NG + t]; });
+            sync();
+            // gradient, stress and the three fluxes at each point of the line
+            Real fx[3][NG];
+            if (lane_ok) {
+#pragma unroll
+                for (int i = 0; i < NG; ++i) {
+                    const int p = i * NG2 + col;
+                    Real dd[9];
+#pragma unroll
+                    for (int q = 0; q < 9; ++q) dd[q] = geo[q * NN + p];
+                    const Real lam = geo[9 * NN + p], mu = geo[10 * NN + p];
+                    Real gr[3][3];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        Real gx = Real(0);
+#pragma unroll
+                        for (int s = 0; s < NG; ++s) gx += A.D[i * NG + s] * u[c][s];
+                        const Real gy = xe[c * CELLS * SE + own_e + i * PE], gz = xz[c * CELLS * SZ + own_z + i * PZ];
+                        gr[c][0] = gx * dd[0] + gy * dd[1] + gz * dd[2];
+                        gr[c][1] = gx * dd[3] + gy * dd[4] + gz * dd[5];
+                        gr[c][2] = gx * dd[6] + gy * dd[7] + gz * dd[8];
+                    }
+                    const Real tr = lam * (gr[0][0] + gr[1][1] + gr[2][2]);
+                    const Real m2 = Real(2) * mu;
+                    const Real s0 = m2 * gr[0][0] + tr, s1 = m2 * gr[1][1] + tr, s2 = m2 * gr[2][2] + tr;
+                    const Real s3 = mu * (gr[0][1] + gr[1][0]), s4 = mu * (gr[0][2] + gr[2][0]),
+                               s5 = mu * (gr[1][2] + gr[2][1]);
+                    // flux along axis a: sigma . (dd[a], dd[3+a], dd[6+a])
+                    fx[0][i] = s0 * dd[0] + s3 * dd[3] + s4 * dd[6];
+                    fx[1][i] = s3 * dd[0] + s1 * dd[3] + s5 * dd[6];
+                    fx[2][i] = s4 * dd[0] + s5 * dd[3] + s2 * dd[6];
+                    xe[0 * CELLS * SE + own_e + i * PE] = s0 * dd[1] + s3 * dd[4] + s4 * dd[7];
+                    xe[1 * CELLS * SE + own_e + i * PE] = s3 * dd[1] + s1 * dd[4] + s5 * dd[7];
+                    xe[2 * CELLS * SE + own_e + i * PE] = s4 * dd[1] + s5 * dd[4] + s2 * dd[7];
+                    xz[0 * CELLS * SZ + own_z + i * PZ] = s0 * dd[2] + s3 * dd[5] + s4 * dd[8];
+                    xz[1 * CELLS * SZ + own_z + i * PZ] = s3 * dd[2] + s1 * dd[5] + s5 * dd[8];
+                    xz[2 * CELLS * SZ + own_z + i * PZ] = s4 * dd[2] + s5 * dd[5] + s2 * dd[8];
+                }
+            }
+            sync();  // and the geometry has been read
+            if (d + 1 == d1 && next < n_item) copy_geo(next);
+            if (lane_ok) contract([&](int s2, int t) { return A.D[t * NG + s2]; });
+            if (gt == 0) bulk_wait_read();  // the chunk before has left the stage
+            sync();
+            Real r[3][NG];
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int i = 0; i < NG; ++i) {
+                    Real x = Real(0);
+#pragma unroll
+                    for (int s = 0; s < NG; ++s) x += A.D[s * NG + i] * fx[c][s];
+                    x += xe[c * CELLS * SE + own_e + i * PE];
+                    x += xz[c * CELLS * SZ + own_z + i * PZ];
+                    r[c][i] = -x;
+                }
+            if constexpr (PML)
+                if (slot >= 0) line_cell_pml<Real, NG>(A, slot, mdl, d, col, cw, r);
+            // point force (solver.cpp:577-605)
+            if (src0 >= 0 && A.mstf) {
+                const int fs = A.fset[d], dir = A.dir[d];
+                const Real stf = __ldg(A.mstf + mdl * A.n_set + fs);
+                for (int sl = stf != Real(0) ? src0 : -1; sl >= 0; sl = __ldg(A.src_next + sl)) {
+                    if (A.src_set && __ldg(A.src_set + sl) != fs) continue;
+#pragma unroll
+                    for (int i = 0; i < NG; ++i) {
+                        const Real sw = stf * __ldg(A.src_w + (size_t)sl * NN + i * NG2 + col);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c)
+                            if (c == dir) r[c][i] += sw;
+                    }
+                }
+            }
+            const int dc = d % fc;
+            if (!staged) {
+                if (act) {
+                    Real* out = A.contrib + ((size_t)e * row_u + (size_t)(d / fc) * chunk_u + col * fc + dc) * 3;
+#pragma unroll
+                    for (int i = 0; i < NG; ++i)
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) out[i * NG2 * fc * 3 + c] = r[c][i];
+                }
+                continue;
+            }
+            if constexpr (S::OUT_IN_XCH) sync();  // every thread has read the eta array
+            if (lane_ok) {
+                Real* out = stage + (cl * chunk_u + col * fc + dc) * 3;
+#pragma unroll
+                for (int i = 0; i < NG; ++i)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) out[i * NG2 * fc * 3 + c] = r[c][i];
+            }
+            if (dc + 1 == fc) {
+                fence_proxy_async_smem();
+                sync();
+                if (gt == 0) {
+                    const int e0 = item / split * CELLS, nc = min(CELLS, n_cell - e0);
+                    for (int c = 0; c < nc; ++c)
+                        bulk_copy_s2g(A.contrib + ((size_t)(e0 + c) * row_u + (size_t)(d / fc) * chunk_u) * 3,
+                                      stage + c * chunk_u * 3, (unsigned)(chunk_u * 3 * sizeof(Real)));
+                    bulk_commit();
+                    if constexpr (S::OUT_IN_XCH) bulk_wait_read();
+                }
+                if constexpr (S::OUT_IN_XCH) sync();
+            }
+        }
+    }
+    if (gt == 0) bulk_wait_all();
 }
 
 // Predictor only (start of a run or after a state overwrite).
@@ -1547,7 +2054,7 @@ __global__ void record_kernel(RecArgs<Real, Out> A) {
     if (p >= NN) return;
     const int i = p / (NG * NG), j = (p / NG) % NG, k = p % NG;
     double dd[9];
-    const Real* gp = A.geom + (size_t)e * 12 * NN + p;
+    const Real* gp = A.geom + (size_t)e * geo_row<Real>(NN) + p;
     for (int q = 0; q < 9; ++q) dd[q] = (double)gp[q * NN];
     for (int d = 0; d < NFLD; ++d) {
         double gx[3] = {0, 0, 0}, gy[3] = {0, 0, 0}, gz[3] = {0, 0, 0};

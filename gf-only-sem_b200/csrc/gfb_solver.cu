@@ -254,7 +254,16 @@ struct gfb_solver {
     int flags = 0;
     bool fuse = false;  // node update in the element kernel's last colour
     int step = 0;
-    std::vector<int> colour_begin;  // [n_colour+1] device cell ranges
+    std::vector<int> colour_begin;  // [n_colour+1] ranges of clist
+    int* clist = nullptr;           // the cells colour after colour (kernels that assemble by colour)
+    // the default element kernel leaves the cells' contributions for the node
+    // pass to assemble (gather_ok: the mesh is small enough for its indices
+    // and its buffer fits on the device)
+    bool gather_ok = false;
+    void* contrib = nullptr;        // Real [cell][chunk][nn][fields of the chunk][3] (gfb::NodeGather)
+    uint4* touch = nullptr;         // [node] (gfb::NodeGather)
+    uint4* touch_more = nullptr;
+    int gather_blocks = 0;          // persistent grid of the gather kernel
     bool has_cpml = false, has_damping = false, has_src = false;
     int n_pml = 0, n_src = 0, n_rec = 0, slots = 0;
     double c1 = 0.0, c2 = 0.0;
@@ -264,13 +273,13 @@ struct gfb_solver {
     uint32_t* ibool_padded = nullptr;  // [cell][NNP] for the pipelined kernel
     int pipe_blocks = 0;               // persistent grid of the element kernel
     int col_blocks = 0;                // persistent grid of the line kernel (FP32)
-    int col_variant = 0;               // line kernel: 0 default (line owners where built), 1 fewer cells, 2 more, 3 default cells, exchange by every thread
+    int col_variant = 0;               // FP32: 0 the gather kernel, 1..3 the line kernel by colour with fewer, more, default cells per group
     int n_col_variants = 1;
     int col_epb = 0;                   // cells per group of the variant in use
-    bool point_kernel = false;         // thread-per-point element kernel on the FP32 path
+    bool point_kernel = false;         // thread-per-point element kernel
     void* geom = nullptr;
     void* dmat = nullptr;
-    float dmat_host[36] = {};          // D of the line kernel's parameters
+    double dmat_host[36] = {};         // D of the line kernels' parameters
     double *u = nullptr, *v = nullptr;
     void *a = nullptr, *ut = nullptr, *force = nullptr;
     double* mass = nullptr;
@@ -504,6 +513,16 @@ struct StageClock {
 // kernel dispatch
 // ---------------------------------------------------------------------------
 
+// The gather kernel runs unless the fused node update,
+// GFB_FLAG_POINT_KERNEL or another FP32 variant asks for assembly by colour.
+bool use_gather(const gfb_solver* s) {
+    return s->gather_ok && !s->fuse && !s->point_kernel && (s->prec == GFB_FP64 || s->col_variant == 0);
+}
+
+// Whether the assembled force outlives the step: the stored force of the
+// increments, the acceleration of the half-step velocity nodes.
+bool keep_force(const gfb_solver* s) { return s->refresh > 1 || s->half_v; }
+
 template <typename Real>
 void node_args(const gfb_solver* s, gfb::NodeArgs<Real>& A, gfb::NodePml<Real>& P) {
     A.n_node = s->n_node;
@@ -511,7 +530,16 @@ void node_args(const gfb_solver* s, gfb::NodeArgs<Real>& A, gfb::NodePml<Real>& 
     A.v = s->v;
     A.a = static_cast<Real*>(s->a);
     A.ut = static_cast<Real*>(s->ut);
-    A.force = static_cast<const Real*>(s->force);
+    A.force = static_cast<Real*>(s->force);
+    A.gather = gfb::NodeGather<Real>{};
+    if (use_gather(s) && !s->layer) {  // a layer: assembled before it (step_body)
+        A.gather.touch = s->touch;
+        A.gather.more = s->touch_more;
+        A.gather.contrib = static_cast<const Real*>(s->contrib);
+        A.gather.chunk_units = gfb::gather_chunk_units<Real>(s->nn, s->nfld);
+        A.gather.keep = keep_force(s);
+        A.gather.mdirect = s->refresh > 1 ? s->d_mdirect : nullptr;
+    }
     A.mass = s->mass;
     A.inv_mass = static_cast<const Real*>(s->inv_mass);
     A.damping = s->has_damping ? s->damping : nullptr;
@@ -544,6 +572,7 @@ gfb_status launch_elem_t(gfb_solver* s, int c) {
     A.e_begin = s->colour_begin[c];
     A.e_end = s->colour_begin[c + 1];
     if (A.e_end <= A.e_begin) return GFB_OK;
+    A.cells = s->clist;
     A.ibool = s->ibool;
     A.geom = static_cast<const Real*>(s->geom);
     A.ut = static_cast<const Real*>(s->ut);
@@ -583,20 +612,34 @@ gfb_status launch_elem_t(gfb_solver* s, int c) {
     return GFB_OK;
 }
 
-// The FP32 path runs the line kernel unless per-cell C-PML, the fused node
-// update or GFB_FLAG_POINT_KERNEL asks for the thread-per-point kernel.
+// FP32 kernels that can be chosen between (gfb_select_element_kernel): not
+// with per-cell C-PML or the fused node update.
 bool col_kernel_eligible(const gfb_solver* s) {
     return s->prec == GFB_FP32 && !(s->has_cpml && !s->node_pml) && !s->fuse;
 }
-bool use_col_kernel(const gfb_solver* s) { return col_kernel_eligible(s) && !s->point_kernel; }
 
-template <int NG, int NFLD, int EPB, bool XCH = false>
+// Candidates at ngll 5 with up to three wavefields: 0 the gather kernel, and
+// the line kernel by colour with 1 one fewer cell per group, 2 one more, 3
+// the default count.  Elsewhere the gather kernel only.
+constexpr int col_epb_lo(int nfld) { return nfld == 3 ? 1 : (nfld == 2 ? 2 : 4); }
+constexpr int col_epb_hi(int nfld) { return nfld == 3 ? 3 : (nfld == 2 ? 4 : 8); }
+template <int NG, int NFLD>
+constexpr bool kHasCol = NG == 5 && NFLD <= 3;
+
+// Line kernel by colour: a variant of it is selected, or the mesh is too
+// large for the gather kernel.
+bool use_col_kernel(const gfb_solver* s) {
+    return col_kernel_eligible(s) && !s->point_kernel && !use_gather(s) && s->ng == 5 && s->nfld <= 3;
+}
+
+template <int NG, int NFLD, int EPB>
 gfb_status launch_col_e(gfb_solver* s, int c) {
-    using S = gfb::ColShape<NG, NFLD, EPB, XCH>;
+    using S = gfb::ColShape<NG, NFLD, EPB>;
     gfb::ColArgs A;
     A.e_begin = s->colour_begin[c];
     A.e_end = s->colour_begin[c + 1];
     if (A.e_end <= A.e_begin) return GFB_OK;
+    A.cells = s->clist;
     const int n = A.e_end - A.e_begin;
     A.n_groups = (n + S::EPB - 1) / S::EPB;
     A.live_end = s->d_live_cell_end;  // null with one model
@@ -619,80 +662,138 @@ gfb_status launch_col_e(gfb_solver* s, int c) {
         A.dir[d] = s->dirs[d];
         A.fset[d] = s->fset[d];
     }
-    for (int q = 0; q < 36; ++q) A.D[q] = q < NG * NG ? s->dmat_host[q] : 0.f;
+    for (int q = 0; q < 36; ++q) A.D[q] = q < NG * NG ? s->dmat_host[q] : 0.0;
     const int blocks = std::max(1, std::min(A.n_groups, s->col_blocks));
     A.err = reinterpret_cast<unsigned*>(s->d_kernel_err);
     const int smem = S::SMEM + gfb::col_model_smem(s->n_model, s->n_set);
-    gfb::elem_col_kernel<NG, NFLD, EPB, XCH><<<blocks, S::THREADS, smem, s->stream>>>(A);
+    gfb::elem_col_kernel<NG, NFLD, EPB><<<blocks, S::THREADS, smem, s->stream>>>(A);
     CU(cudaGetLastError());
     s->launches++;
     return GFB_OK;
 }
 
-// Candidates of the line kernel.  At ngll 5 with up to three wavefields:
-// 0 the default cells per group with the eta/zeta contractions done by line
-// owners (ColShape's XCH; the fastest measured), and with the exchange done
-// by every thread 1 one fewer cell per group ("LO"), 2 one more ("HI"),
-// 3 the default count.  Elsewhere: 0 the default count, exchange by every
-// thread.
-constexpr int col_epb_lo(int nfld) { return nfld == 3 ? 1 : (nfld == 2 ? 2 : 4); }
-constexpr int col_epb_hi(int nfld) { return nfld == 3 ? 3 : (nfld == 2 ? 4 : 8); }
-template <int NG, int NFLD>
-struct ColEpb {
-    static constexpr int D = gfb::col_default_epb(NG, NFLD);
-    // the other variants exist for ngll 5 with up to three wavefields (more
-    // would exceed a block's threads)
-    static constexpr int N = (NG == 5 && NFLD <= 3) ? 4 : 1;
-};
-
 template <int NG, int NFLD>
 gfb_status launch_col_t(gfb_solver* s, int c) {
-    using E = ColEpb<NG, NFLD>;
-    if constexpr (E::N > 1) {
-        if (s->col_variant == 0) return launch_col_e<NG, NFLD, E::D, true>(s, c);
-        if (s->col_variant == 1) return launch_col_e<NG, NFLD, col_epb_lo(NFLD)>(s, c);
-        if (s->col_variant == 2) return launch_col_e<NG, NFLD, col_epb_hi(NFLD)>(s, c);
-    }
-    return launch_col_e<NG, NFLD, E::D>(s, c);
+    if (s->col_variant == 1) return launch_col_e<NG, NFLD, col_epb_lo(NFLD)>(s, c);
+    if (s->col_variant == 2) return launch_col_e<NG, NFLD, col_epb_hi(NFLD)>(s, c);
+    return launch_col_e<NG, NFLD, gfb::col_default_epb(NG, NFLD)>(s, c);
 }
 
 // Persistent grid of the line kernel variant EPB: occupancy x SMs.
-template <int NG, int NFLD, int EPB, bool XCH = false>
-gfb_status col_grid(gfb_solver* s, int* blocks) {
-    using C = gfb::ColShape<NG, NFLD, EPB, XCH>;
-    auto* fn = gfb::elem_col_kernel<NG, NFLD, EPB, XCH>;
+template <int NG, int NFLD, int EPB>
+gfb_status col_grid(gfb_solver* s) {
+    using C = gfb::ColShape<NG, NFLD, EPB>;
+    auto* fn = gfb::elem_col_kernel<NG, NFLD, EPB>;
     const int smem = C::SMEM + gfb::col_model_smem(s->n_model, s->n_set);
     CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     int per_sm = 0, n_sm = 0;
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, C::THREADS, smem));
     CU(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, s->device));
     if (per_sm < 1) return fail(GFB_ERR_UNSUPPORTED, "line element kernel does not fit on an SM");
-    *blocks = per_sm * n_sm;
+    s->col_blocks = per_sm * n_sm;
+    s->col_epb = EPB;
     return GFB_OK;
 }
 
 template <int NG, int NFLD>
 gfb_status col_grid_t(gfb_solver* s) {
-    using E = ColEpb<NG, NFLD>;
-    gfb_status st;
-    s->n_col_variants = E::N;
-    if constexpr (E::N > 1) {
-        if (s->col_variant == 1) {
-            s->col_epb = col_epb_lo(NFLD);
-            return col_grid<NG, NFLD, col_epb_lo(NFLD)>(s, &s->col_blocks);
-        }
-        if (s->col_variant == 2) {
-            s->col_epb = col_epb_hi(NFLD);
-            return col_grid<NG, NFLD, col_epb_hi(NFLD)>(s, &s->col_blocks);
-        }
-        if (s->col_variant == 0) {
-            s->col_epb = E::D;
-            return col_grid<NG, NFLD, E::D, true>(s, &s->col_blocks);
-        }
+    s->n_col_variants = 1;
+    if constexpr (kHasCol<NG, NFLD>) {
+        s->n_col_variants = 4;
+        if (s->col_variant == 1) return col_grid<NG, NFLD, col_epb_lo(NFLD)>(s);
+        if (s->col_variant == 2) return col_grid<NG, NFLD, col_epb_hi(NFLD)>(s);
+        return col_grid<NG, NFLD, gfb::col_default_epb(NG, NFLD)>(s);
     }
-    if ((st = col_grid<NG, NFLD, E::D>(s, &s->col_blocks))) return st;
-    s->col_epb = E::D;
     return GFB_OK;
+}
+
+template <typename Real, int NG>
+gfb_status launch_gather_t(gfb_solver* s) {
+    using S = gfb::GatherShape<Real, NG>;
+    gfb::GatherArgs<Real> A;
+    A.n_cell = s->n_cell;
+    A.live_end = s->d_live_cell_end ? s->d_live_cell_end + (s->colour_begin.size() - 1) : nullptr;
+    A.ibool_padded = s->ibool_padded;
+    A.geom = static_cast<const Real*>(s->geom);
+    A.ut = static_cast<const Real*>(s->ut);
+    A.contrib = static_cast<Real*>(s->contrib);
+    A.nfld = s->nfld;
+    A.mlive = s->d_mlive;
+    A.multi = s->n_model > 1;
+    A.src_head = s->has_src ? s->src_head : nullptr;
+    A.src_next = s->src_next;
+    A.src_w = static_cast<const Real*>(s->src_w);
+    A.mstf = static_cast<const Real*>(s->d_mstf);
+    A.src_set = s->src_set;
+    A.n_set = s->n_set;
+    for (int d = 0; d < gfb::kMaxFields; ++d) {
+        A.dir[d] = s->dirs[d];
+        A.fset[d] = s->fset[d];
+    }
+    const bool pml = s->has_cpml && !s->node_pml;
+    A.pml_slot = s->pml_slot;
+    A.pml_coef = static_cast<const Real*>(s->pml_coef);
+    A.pml_mem = static_cast<Real*>(s->pml_mem);
+    A.pml_prev = static_cast<Real*>(s->pml_prev);
+    A.u = s->u;
+    A.v = s->v;
+    A.a = static_cast<const Real*>(s->a);
+    A.mc = s->d_mc;
+    A.err = reinterpret_cast<unsigned*>(s->d_kernel_err);
+    for (int q = 0; q < 36; ++q) A.D[q] = q < NG * NG ? (Real)s->dmat_host[q] : Real(0);
+    // a work item is a group's cells with all their wavefields (the geometry
+    // read once), or one wavefield of them where that would leave more than
+    // half of the resident groups without work
+    const int groups = (s->n_cell + S::CELLS - 1) / S::CELLS;
+    A.nfld_item = 2 * groups <= s->gather_blocks * S::GROUPS ? 1 : s->nfld;
+    const int items = groups * (s->nfld / A.nfld_item);
+    const int blocks = std::max(1, std::min((items + S::GROUPS - 1) / S::GROUPS, s->gather_blocks));
+    if (pml) gfb::elem_gather_kernel<Real, NG, true><<<blocks, S::THREADS, S::SMEM, s->stream>>>(A);
+    else gfb::elem_gather_kernel<Real, NG, false><<<blocks, S::THREADS, S::SMEM, s->stream>>>(A);
+    CU(cudaGetLastError());
+    s->launches++;
+    return GFB_OK;
+}
+
+// Persistent grid of the gather kernel: occupancy x SMs.
+template <typename Real, int NG>
+gfb_status gather_grid_t(gfb_solver* s) {
+    using S = gfb::GatherShape<Real, NG>;
+    auto* fn = s->has_cpml && !s->node_pml ? gfb::elem_gather_kernel<Real, NG, true>
+                                           : gfb::elem_gather_kernel<Real, NG, false>;
+    CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
+    int per_sm = 0, n_sm = 0;
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, S::THREADS, S::SMEM));
+    CU(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, s->device));
+    if (per_sm < 1) return fail(GFB_ERR_UNSUPPORTED, "gather element kernel does not fit on an SM");
+    s->gather_blocks = per_sm * n_sm;
+    return GFB_OK;
+}
+
+int gather_cells(int ng) {
+    return ng == 3 ? gfb::GatherShape<float, 3>::CELLS
+                   : (ng == 4 ? gfb::GatherShape<float, 4>::CELLS
+                              : (ng == 5 ? gfb::GatherShape<float, 5>::CELLS : gfb::GatherShape<float, 6>::CELLS));
+}
+
+template <typename Real>
+gfb_status launch_gather(gfb_solver* s) {
+    switch (s->ng) {
+        case 3: return launch_gather_t<Real, 3>(s);
+        case 4: return launch_gather_t<Real, 4>(s);
+        case 5: return launch_gather_t<Real, 5>(s);
+        default: return launch_gather_t<Real, 6>(s);
+    }
+}
+
+template <typename Real>
+gfb_status gather_grid(gfb_solver* s) {
+    switch (s->ng) {
+        case 3: return gather_grid_t<Real, 3>(s);
+        case 4: return gather_grid_t<Real, 4>(s);
+        case 5: return gather_grid_t<Real, 5>(s);
+        default: return gather_grid_t<Real, 6>(s);
+    }
 }
 
 template <typename Real, int NG, int NFLD>
@@ -766,7 +867,7 @@ gfb_status dispatch(int ng, int nfld, Args... args) {
 template <typename Real, int NG, int NFLD>
 struct ElemOp {
     static gfb_status run(gfb_solver* s, int c) {
-        if constexpr (std::is_same<Real, float>::value)
+        if constexpr (std::is_same<Real, float>::value && kHasCol<NG, NFLD>)
             if (use_col_kernel(s)) return launch_col_t<NG, NFLD>(s, c);
         return launch_elem_t<Real, NG, NFLD>(s, c);
     }
@@ -780,20 +881,31 @@ struct RecOp {
     static gfb_status run(gfb_solver* s, void* out) { return launch_record_t<Real, NG, NFLD>(s, out); }
 };
 
-gfb_status launch_elem(gfb_solver* s, int c) {
+gfb_status launch_colour(gfb_solver* s, int c) {
     if (s->prec == GFB_FP64) return dispatch<double, ElemOp>(s->ng, s->nfld, s, c);
     return dispatch<float, ElemOp>(s->ng, s->nfld, s, c);
 }
 
-// Autotuner of the FP32 element phase: times full colour sweeps of every
-// element-kernel candidate on this mesh (the line kernel with each cells-per-
-// group count it is built with, and the thread-per-point kernel) and keeps
-// the fastest.  A full sweep only rewrites the assembled force from the
-// current predicted displacement (the first colour touching a node stores),
-// so tuning leaves the solver's state as it was.
+// The element phase of a step: one launch, or one per colour.
+gfb_status launch_elem(gfb_solver* s) {
+    if (use_gather(s)) return s->prec == GFB_FP64 ? launch_gather<double>(s) : launch_gather<float>(s);
+    gfb_status st;
+    for (int c = 0; c + 1 < (int)s->colour_begin.size(); ++c)
+        if ((st = launch_colour(s, c))) return st;
+    return GFB_OK;
+}
+
+gfb_status launch_assemble(gfb_solver* s);
+
+// Autotuner of the FP32 element phase: times full sweeps of every
+// element-kernel candidate on this mesh (the gather kernel with an assembly
+// pass, the line kernel with each cells-per-group count it is built with, and
+// the thread-per-point kernel) and keeps the fastest.  A full sweep only
+// rewrites the assembled force from the current predicted displacement (the
+// first colour touching a node stores), so tuning leaves the solver's state
+// as it was.
 gfb_status autotune(gfb_solver* s) {
     if (!col_kernel_eligible(s)) return GFB_OK;
-    const int n_colour = (int)s->colour_begin.size() - 1;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     CU(cudaEventCreate(&e0));
     CU(cudaEventCreate(&e1));
@@ -812,10 +924,8 @@ gfb_status autotune(gfb_solver* s) {
         s->col_variant = c.variant;
         if (!c.point && (st = dispatch<float, ColGridOp>(s->ng, s->nfld, s))) break;
         auto sweep = [&]() -> gfb_status {
-            gfb_status r;
-            for (int k = 0; k < n_colour; ++k)
-                if ((r = launch_elem(s, k))) return r;
-            return GFB_OK;
+            gfb_status r = launch_elem(s);
+            return r || !use_gather(s) ? r : launch_assemble(s);
         };
         if ((st = sweep())) break;  // warm-up
         if (cudaEventRecord(e0, s->stream) != cudaSuccess) { st = fail(GFB_ERR_CUDA, "autotune event"); break; }
@@ -849,6 +959,12 @@ int grid_for(long long n, int threads) {
     return (int)std::max(1LL, std::min(b, 148LL * 32));
 }
 
+// Blocks of a node pass over n nodes: resident ones, looping over tiles.
+int node_grid(long long n, int per_sm) {
+    const long long per_block = gfb::kNodeTile * (gfb::kNodeThreads / 32);
+    return (int)std::max(1LL, std::min((n + per_block - 1) / per_block, 148LL * per_sm));
+}
+
 template <typename Real, int NFLD, bool MULTI>
 gfb_status launch_node_m(gfb_solver* s) {
     gfb::NodeArgs<Real> A;
@@ -857,18 +973,52 @@ gfb_status launch_node_m(gfb_solver* s) {
     // node-form C-PML nodes are device nodes [0, n_pml_node)
     const long long g0 = s->node_pml ? s->n_pml_node : 0;
     if (g0 < s->n_node) {
-        const int grid = grid_for((long long)(s->n_node - g0) * NFLD, 256);
-        gfb::node_update_kernel<Real, NFLD, MULTI><<<grid, 256, 0, s->stream>>>(A, P, g0);
+        const int grid = node_grid(s->n_node - g0, gfb::node_blocks_per_sm<Real>(false));
+        bool done = false;
+        if constexpr (std::is_same<Real, float>::value)
+            if ((done = A.half_v))
+                gfb::node_update_kernel<Real, NFLD, MULTI, true><<<grid, gfb::kNodeThreads, 0, s->stream>>>(A, P, g0);
+        if (!done) gfb::node_update_kernel<Real, NFLD, MULTI, false><<<grid, gfb::kNodeThreads, 0, s->stream>>>(A, P, g0);
         CU(cudaGetLastError());
         s->launches++;
     }
-    if (g0 > 0) {
-        const int gp = grid_for(g0 * NFLD, 256);
-        gfb::node_pml_kernel<Real, NFLD, MULTI><<<gp, 256, 0, s->stream>>>(A, P);
-        CU(cudaGetLastError());
-        s->launches++;
+    if constexpr (std::is_same<Real, float>::value) {
+        if (g0 > 0) {
+            const int gp = node_grid(g0, gfb::node_blocks_per_sm<float>(true));
+            gfb::node_pml_kernel<NFLD, MULTI><<<gp, gfb::kNodeThreads, 0, s->stream>>>(A, P);
+            CU(cudaGetLastError());
+            s->launches++;
+        }
     }
     return GFB_OK;
+}
+
+// The assembled force of the gather kernel's contributions, in `force`.
+template <typename Real, int NFLD>
+gfb_status launch_assemble_f(gfb_solver* s) {
+    gfb::NodeArgs<Real> A;
+    gfb::NodePml<Real> P;
+    gfb::Layer* const layer = s->layer;
+    s->layer = nullptr;  // node_args: the contributions, not the assembled force
+    node_args(s, A, P);
+    s->layer = layer;
+    const int grid = grid_for((long long)s->n_node * NFLD, 256);
+    if (s->n_model > 1) gfb::assemble_kernel<Real, NFLD, true><<<grid, 256, 0, s->stream>>>(A, P);
+    else gfb::assemble_kernel<Real, NFLD, false><<<grid, 256, 0, s->stream>>>(A, P);
+    CU(cudaGetLastError());
+    s->launches++;
+    return GFB_OK;
+}
+
+gfb_status launch_assemble(gfb_solver* s) {  // FP32
+    switch (s->nfld) {
+        case 1: return launch_assemble_f<float, 1>(s);
+        case 2: return launch_assemble_f<float, 2>(s);
+        case 3: return launch_assemble_f<float, 3>(s);
+        case 6: return launch_assemble_f<float, 6>(s);
+        case 9: return launch_assemble_f<float, 9>(s);
+        default: return launch_assemble_f<float, 12>(s);
+    }
 }
 
 template <typename Real, int NFLD>
@@ -1077,7 +1227,7 @@ gfb_status upload_node_pml(gfb_solver* s, const std::vector<double>& coef) {
     gfb_status st;
     const int n = (int)(coef.size() / 14);
     Real* dc = nullptr;
-    if ((st = s->alloc(&dc, (size_t)std::max(n, 1) * 14))) return st;
+    if ((st = s->alloc(&dc, (size_t)std::max(n, 1) * 14 + 4))) return st;  // read in 16-byte copies
     st = staged_upload(s, dc, 14 * sizeof(Real), n, [&](long long i0, long long i1, unsigned char* out) {
         Real* o = reinterpret_cast<Real*>(out);
         parallel_for((i1 - i0) * 14, [&](long long a0, long long a1) {
@@ -1098,11 +1248,99 @@ gfb_status upload_node_pml(gfb_solver* s, const std::vector<double>& coef) {
     return GFB_OK;
 }
 
+// What the gather kernel and the node pass assemble through: the cells'
+// contribution buffer and every node's touches (gfb::NodeGather).  Without
+// them (a mesh past 2^31 touches, or a buffer that no longer fits on the
+// device) the element phase assembles by colour.  Called last.
+template <typename Real>
+gfb_status build_gather(gfb_solver* s, const gfb_mesh* m, const NodeBuckets& nb, const std::vector<long long>& first_q) {
+    const int nn = s->nn, fc = gfb::gather_chunk_fields<Real>(s->nfld);
+    const size_t row_u = (size_t)(s->nfld / fc) * gfb::gather_chunk_units<Real>(nn, s->nfld);
+    const size_t units = (size_t)s->n_cell * row_u;
+    auto unit_of = [&](long long q) -> uint32_t { return (uint32_t)((size_t)(q / nn) * row_u + (size_t)(q % nn) * fc); };
+    // the fused node update keeps to assembly by colour; so does the
+    // thread-per-point kernel where no other can be selected later
+    if (units >= (size_t)0x7fffffff || s->fuse || (s->point_kernel && s->prec == GFB_FP64)) return GFB_OK;
+    const size_t contrib = units * 3 * sizeof(Real);
+    // beside the buffer: the touches and the half-step velocity (create_impl),
+    // and some room for what a user attaches later
+    size_t free_b = 0, total_b = 0;
+    CU(cudaMemGetInfo(&free_b, &total_b));
+    if (free_b < contrib + (size_t)s->n_node * (24 + 4 * s->F) + (size_t(1) << 30)) return GFB_OK;
+    // the second to fourth touch of each node, or where the touches from the
+    // fourth on are
+    struct Rest {
+        uint32_t q[3];
+    };
+    std::vector<Rest> rest((size_t)s->n_node, Rest{{gfb::kNoTouch, gfb::kNoTouch, gfb::kNoTouch}});
+    std::vector<std::vector<uint4>> more(nb.n_owner);
+    nb.for_each_owner([&](int t, long long g0, long long g1, const long long* qs, size_t nq) {
+        std::vector<uint16_t> cnt((size_t)(g1 - g0), 0);
+        for (size_t k = 0; k < nq; ++k) {
+            const int g = m->ibool[qs[k]];
+            const uint16_t c = cnt[g - g0];
+            if (c >= 1 && c <= 3) rest[g].q[c - 1] = unit_of(qs[k]);
+            if (c < 0xffff) cnt[g - g0] = (uint16_t)(c + 1);
+        }
+        // nodes of more than four: touches 3, 4, ... in groups of four
+        std::vector<long long> many;
+        size_t n4 = 0;
+        for (long long g = g0; g < g1; ++g)
+            if (cnt[g - g0] > 4) {
+                rest[g].q[2] = gfb::kMoreTouches | (uint32_t)n4;  // the owner's offset is added below
+                n4 += cnt[g - g0] / 4;                              // (cnt - 3) entries
+                many.push_back(g);
+            }
+        if (many.empty()) return;
+        more[t].assign(n4, uint4{gfb::kNoTouch, gfb::kNoTouch, gfb::kNoTouch, gfb::kNoTouch});
+        std::vector<uint16_t> seen((size_t)(g1 - g0), 0);
+        for (size_t k = 0; k < nq; ++k) {
+            const int g = m->ibool[qs[k]];
+            const int c = cnt[g - g0];
+            if (c <= 4) continue;
+            const int slot = (int)seen[g - g0]++ - 3;
+            if (slot < 0) continue;
+            uint32_t* w = &more[t][(rest[g].q[2] & ~gfb::kMoreTouches) + slot / 4].x;
+            w[slot % 4] = unit_of(qs[k]) | (slot % 4 == 0 && slot + 4 < c - 3 ? gfb::kMoreTouches : 0u);
+        }
+    });
+    std::vector<size_t> base(nb.n_owner + 1, 0);
+    for (int t = 0; t < nb.n_owner; ++t) base[t + 1] = base[t] + more[t].size();
+    if (base.back() >= (size_t)0x7fffffff) return GFB_OK;
+    gfb_status st;
+    uint4* dt = nullptr;
+    if ((st = s->alloc(&dt, (size_t)s->n_node))) return st;
+    st = staged_upload(s, dt, sizeof(uint4), s->n_node, [&](long long d0, long long d1, unsigned char* out) {
+        uint4* o = reinterpret_cast<uint4*>(out);
+        parallel_for(d1 - d0, [&](long long a0, long long a1) {
+            for (long long i = a0; i < a1; ++i) {
+                const long long g = s->node_perm.empty() ? d0 + i : s->node_perm[d0 + i];
+                uint32_t w = rest[g].q[2];
+                if ((w & gfb::kMoreTouches) && w != gfb::kNoTouch) w += (uint32_t)base[nb.owner(g)];
+                o[i] = uint4{first_q[g] < 0 ? gfb::kNoTouch : unit_of(first_q[g]), rest[g].q[0], rest[g].q[1], w};
+            }
+        });
+    });
+    if (st) return st;
+    uint4* dm = nullptr;
+    if ((st = s->alloc(&dm, base.back()))) return st;
+    for (int t = 0; t < nb.n_owner; ++t)
+        if (!more[t].empty() && (st = h2d(s, dm + base[t], more[t].data(), more[t].size() * sizeof(uint4)))) return st;
+    Real* dc = nullptr;
+    if ((st = s->alloc(&dc, units * 3))) return st;
+    s->touch = dt;
+    s->touch_more = dm;
+    s->contrib = dc;
+    s->gather_ok = true;
+    return GFB_OK;
+}
+
 template <typename Real>
 gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src, int n_model,
-                        const gfb_model* models, const std::vector<int>& perm, const std::vector<int>& inv_perm,
+                        const gfb_model* models, const std::vector<int>& clist,
                         const std::vector<uint32_t>& ibool_dev, const std::vector<double>& node_mass,
-                        const std::vector<double>& node_damp, const std::vector<long long>& first_q,
+                        const std::vector<double>& node_damp, const NodeBuckets& nb,
+                        const std::vector<long long>& first_q,
                         std::vector<uint8_t>& first_flag, const std::vector<uint8_t>& node_live,
                         const std::vector<std::vector<long long>>& live_pts, const std::vector<double>& w,
                         const std::vector<double>& D, StageClock& clk) {
@@ -1231,7 +1469,7 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
                     uint32_t* row = o + i * nnp;
                     for (int p = 0; p < nn; ++p) row[p] = dev_word(ibool_dev[e * nn + p]);
                     int mi = 0;
-                    while (perm[e] >= models[mi].cell_end) ++mi;
+                    while (e >= models[mi].cell_end) ++mi;
                     row[nn] = (uint32_t)mi;
                     for (int p = nn + 1; p < nnp; ++p) row[p] = 0u;
                 }
@@ -1241,25 +1479,28 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
         s->ibool_padded = dp;
     }
     clk.mark("ibool upload");
-    // geometry [cell][12][NN] in colour order
+    // geometry [cell][geo_row], cells in mesh order
     {
+        const int row = gfb::geo_row<Real>(nn);
         Real* dg = nullptr;
-        if ((st = s->alloc(&dg, (size_t)n_cell * 12 * nn))) return st;
-        st = staged_upload(s, dg, (size_t)12 * nn * sizeof(Real), n_cell,
+        if ((st = s->alloc(&dg, (size_t)n_cell * row))) return st;
+        st = staged_upload(s, dg, (size_t)row * sizeof(Real), n_cell,
                            [&](long long e0, long long e1, unsigned char* out) {
             parallel_for(e1 - e0, [&](long long a0, long long a1) {
                 for (long long i = a0; i < a1; ++i) {
-                    const long long e = perm[e0 + i];
-                    Real* o = reinterpret_cast<Real*>(out) + i * 12 * nn;
+                    const long long e = e0 + i;
+                    Real* o = reinterpret_cast<Real*>(out) + i * row;
                     for (int p = 0; p < nn; ++p) {
                         const long long q = e * nn + p;
                         for (int f = 0; f < 9; ++f) o[f * nn + p] = (Real)m->dxi_dx[q * 9 + f];
                         const int i0 = p / (ng * ng), j = (p / ng) % ng, k = p % ng;
-                        // factor = detJ * w_i * w_j * w_k (element_cpu.cpp:108)
-                        o[9 * nn + p] = (Real)(m->jacobian[q] * w[i0] * w[j] * w[k]);
-                        o[10 * nn + p] = (Real)m->lambda_[q];
-                        o[11 * nn + p] = (Real)m->mu[q];
+                        // factor = detJ * w_i * w_j * w_k (element_cpu.cpp:108); mu <= 0
+                        // adds nothing (element_cpu.cpp:42-43)
+                        const double f = m->mu[q] > 0.0 ? m->jacobian[q] * w[i0] * w[j] * w[k] : 0.0;
+                        o[9 * nn + p] = f != 0.0 ? (Real)(m->lambda_[q] * f) : Real(0);
+                        o[10 * nn + p] = f != 0.0 ? (Real)(m->mu[q] * f) : Real(0);
                     }
+                    for (int x = 11 * nn; x < row; ++x) o[x] = Real(0);
                 }
             }, 256);
         });
@@ -1268,9 +1509,14 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
     }
     clk.mark("geometry upload");
     {
+        int* d = nullptr;
+        if ((st = s->alloc(&d, clist.size())) || (st = h2d(s, d, clist.data(), clist.size() * 4))) return st;
+        s->clist = d;
+    }
+    {
         std::vector<Real> d(D.size());
         for (size_t i = 0; i < D.size(); ++i) d[i] = (Real)D[i];
-        for (size_t i = 0; i < D.size() && i < 36; ++i) s->dmat_host[i] = (float)D[i];
+        for (size_t i = 0; i < D.size() && i < 36; ++i) s->dmat_host[i] = D[i];
         if ((st = upload(s, &s->dmat, d))) return st;
     }
     const long long nF = (long long)s->n_node * s->F;
@@ -1333,9 +1579,9 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
         std::vector<int> slot(n_cell, -1);
         std::vector<long long> slot_cell;
         for (long long ed = 0; ed < n_cell; ++ed)
-            if (m->pml_region[perm[ed]] != 0) {
+            if (m->pml_region[ed] != 0) {
                 slot[ed] = (int)slot_cell.size();
-                slot_cell.push_back(perm[ed]);
+                slot_cell.push_back(ed);
             }
         s->n_pml = (int)slot_cell.size();
         {
@@ -1396,7 +1642,7 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
                     set_of[si] = k;
                     auto it = cell_of.find(ss.cell_ids[q]);  // the first cell with the id
                     if (it == cell_of.end()) continue;       // not in this mesh (reference: -1, skipped)
-                    const int ed = inv_perm[it->second];
+                    const int ed = (int)it->second;
                     for (int p = 0; p < nn; ++p) wts[(size_t)si * nn + p] = (Real)ss.weights[(size_t)q * nn + p];
                     if (head[ed] < 0) head[ed] = (int)si;
                     else next[tail[ed]] = (int)si;
@@ -1473,16 +1719,21 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
             // ends of each model's cells per colour and nodes per range
             const int nc = (int)s->colour_begin.size() - 1;
             const long long g0 = s->node_pml ? s->n_pml_node : 0;
-            std::vector<int> cell_end((size_t)n_model * nc), first(nc), live_cell(nc);
-            for (int k = 0; k < n_model; ++k)
-                for (int c = 0; c < nc; ++c) cell_end[(size_t)k * nc + c] = s->colour_begin[c];
+            const int w = nc + 1;  // the colours' ranges of clist, then all cells in mesh order
+            std::vector<int> cell_end((size_t)n_model * w), first(w), live_cell(w);
+            for (int k = 0; k < n_model; ++k) {
+                for (int c = 0; c < nc; ++c) cell_end[(size_t)k * w + c] = s->colour_begin[c];
+                cell_end[(size_t)k * w + nc] = models[k].cell_end;
+            }
+            first[nc] = 0;
+            live_cell[nc] = s->n_cell;
             for (int c = 0; c < nc; ++c) {
                 first[c] = s->colour_begin[c];
                 live_cell[c] = s->colour_begin[c + 1];
-                for (int ed = s->colour_begin[c]; ed < s->colour_begin[c + 1]; ++ed) {
+                for (int x = s->colour_begin[c]; x < s->colour_begin[c + 1]; ++x) {
                     int mi = 0;
-                    while (perm[ed] >= models[mi].cell_end) ++mi;
-                    cell_end[(size_t)mi * nc + c] = ed + 1;
+                    while (clist[x] >= models[mi].cell_end) ++mi;
+                    cell_end[(size_t)mi * w + c] = x + 1;
                 }
             }
             std::vector<long long> node_end((size_t)n_model * 2), live_node{g0, (long long)s->n_node};
@@ -1513,7 +1764,7 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
     // recording cells and snapshot ring
     if (s->n_rec > 0) {
         std::vector<int> rc(s->n_rec);
-        for (int ci = 0; ci < s->n_rec; ++ci) rc[ci] = inv_perm[m->rec_cell_local[ci]];
+        for (int ci = 0; ci < s->n_rec; ++ci) rc[ci] = m->rec_cell_local[ci];
         int* d = nullptr;
         if ((st = s->alloc(&d, rc.size()))) return st;
         if ((st = h2d(s, d, rc.data(), rc.size() * 4))) return st;
@@ -1533,6 +1784,8 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
         host_ring.taken = true;
     }
     clk.mark("snapshot ring");
+    if ((st = build_gather<Real>(s, m, nb, first_q))) return st;
+    clk.mark("assembly lists");
     return GFB_OK;
 }
 
@@ -1574,7 +1827,7 @@ gfb_status launch_step_begin_t(gfb_solver* s) {
     CU(cudaGetLastError());
     s->launches++;
     if (s->d_live_cell_end) {
-        const int nc = (int)s->colour_begin.size() - 1;
+        const int nc = (int)s->colour_begin.size();  // the colours, then all cells in mesh order
         gfb::live_bounds_kernel<<<1, 128, 0, s->stream>>>(s->n_model, nc, s->d_mlive, s->d_cell_end,
                                                           s->d_colour_first, s->d_node_end,
                                                           s->node_pml ? (long long)s->n_pml_node : 0LL,
@@ -1585,16 +1838,15 @@ gfb_status launch_step_begin_t(gfb_solver* s) {
     return GFB_OK;
 }
 
-// The device work of one step: step start, NC colour launches, node pass.
+// The device work of one step: step start, element phase, node pass.
 // With ev != nullptr, events 0..2 bracket the element and node phases.
 gfb_status step_body(gfb_solver* s, cudaEvent_t* ev) {
     gfb_status st;
-    const int n_colour = (int)s->colour_begin.size() - 1;
     if (ev) CU(cudaEventRecord(ev[0], s->stream));
     st = s->prec == GFB_FP64 ? launch_step_begin_t<double>(s) : launch_step_begin_t<float>(s);
     if (st) return st;
-    for (int c = 0; c < n_colour; ++c)
-        if ((st = launch_elem(s, c))) return st;
+    if ((st = launch_elem(s))) return st;
+    if (s->layer && use_gather(s) && (st = launch_assemble(s))) return st;
     if (s->layer && (st = gfb::layer_step(s, s->layer))) return st;
     if (ev) CU(cudaEventRecord(ev[1], s->stream));
     if (!s->fuse)
@@ -1919,31 +2171,26 @@ gfb_status create_impl(const gfb_mesh* m, const gfb_config* c, const gfb_source*
     }
     auto used_mask = [&](uint32_t g) -> uint64_t { return narrow ? (uint64_t)used8[g] : used64[g]; };
     clk.mark("colouring");
-    std::vector<int> perm(m->n_cell), inv_perm(m->n_cell);
+    std::vector<int> clist(m->n_cell);
     s->colour_begin.assign(n_colour + 1, 0);
     for (long long e = 0; e < m->n_cell; ++e) s->colour_begin[colour[e] + 1]++;
     for (int k = 0; k < n_colour; ++k) s->colour_begin[k + 1] += s->colour_begin[k];
     {
         std::vector<int> fill(s->colour_begin.begin(), s->colour_begin.end() - 1);
-        for (long long e = 0; e < m->n_cell; ++e) {
-            const int ed = fill[colour[e]]++;
-            perm[ed] = (int)e;
-            inv_perm[e] = ed;
-        }
+        for (long long e = 0; e < m->n_cell; ++e) clist[fill[colour[e]]++] = (int)e;
     }
-    // device ibool with the first/last-touch bits: the lowest colour
-    // touching a node stores its force, later colours add, the highest
+    // ibool with the first/last-touch bits of assembly by colour: the lowest
+    // colour touching a node stores its force, later colours add, the highest
     // colour finalises the node
     std::vector<uint32_t> ibool_dev((size_t)P);
     parallel_for(m->n_cell, [&](long long e0, long long e1) {
-        for (long long ed = e0; ed < e1; ++ed) {
-            const long long e = perm[ed];
+        for (long long e = e0; e < e1; ++e) {
             for (int p = 0; p < nn; ++p) {
                 const uint32_t g = (uint32_t)m->ibool[e * nn + p];
                 const uint64_t um = used_mask(g);
                 const bool first = __builtin_ctzll(um) == colour[e];
                 const bool last = 63 - __builtin_clzll(um) == colour[e];
-                ibool_dev[ed * nn + p] = g | (first ? gfb::kFirstTouch : 0u) | (last ? gfb::kLastTouch : 0u);
+                ibool_dev[e * nn + p] = g | (first ? gfb::kFirstTouch : 0u) | (last ? gfb::kLastTouch : 0u);
             }
         }
     });
@@ -1954,14 +2201,17 @@ gfb_status create_impl(const gfb_mesh* m, const gfb_config* c, const gfb_source*
     if (D_tab) D.assign(D_tab, D_tab + (size_t)m->ngll * m->ngll);
     if (s->prec == GFB_FP64) {
         if ((st = dispatch<double, SmemOp>(s->ng, s->nfld, s.get()))) return st;
-        st = build_device<double>(s.get(), m, src, n_model, models, perm, inv_perm, ibool_dev, node_mass, node_damp,
-                                  first_q, first_flag, node_live, live_pts, w, D, clk);
+        st = build_device<double>(s.get(), m, src, n_model, models, clist, ibool_dev, node_mass, node_damp,
+                                  nb, first_q, first_flag, node_live, live_pts, w, D, clk);
     } else {
         if ((st = dispatch<float, SmemOp>(s->ng, s->nfld, s.get()))) return st;
-        st = build_device<float>(s.get(), m, src, n_model, models, perm, inv_perm, ibool_dev, node_mass, node_damp,
-                                 first_q, first_flag, node_live, live_pts, w, D, clk);
+        st = build_device<float>(s.get(), m, src, n_model, models, clist, ibool_dev, node_mass, node_damp,
+                                 nb, first_q, first_flag, node_live, live_pts, w, D, clk);
     }
     if (st) return st;
+    if (s->gather_ok) {
+        if ((st = s->prec == GFB_FP64 ? gather_grid<double>(s.get()) : gather_grid<float>(s.get()))) return st;
+    }
     CU(cudaStreamSynchronize(s->stream));
     clk.mark("device set-up");
     // FP32 path: the element force of most steps from the predicted
@@ -2190,12 +2440,13 @@ gfb_status gfb_get_info(const gfb_solver* s, gfb_info* info) {
     info->upload_bytes = s->upload_bytes;
     info->kernel_launches = s->launches;
     info->n_pml_node = s->node_pml ? s->n_pml_node : 0;
-    info->elem_blocks = use_col_kernel(s) ? s->col_blocks : s->pipe_blocks;
-    info->elem_kernel = use_col_kernel(s) ? 1 : 0;
-    info->cells_per_group = use_col_kernel(s) ? s->col_epb : 0;
+    const bool gather = use_gather(s), col = use_col_kernel(s);
+    info->elem_blocks = gather ? s->gather_blocks : (col ? s->col_blocks : s->pipe_blocks);
+    info->elem_kernel = gather || col ? 1 : 0;
+    info->cells_per_group = gather ? gather_cells(s->ng) : (col ? s->col_epb : 0);
     info->force_refresh = s->refresh;
     info->half_v = s->half_v ? 1 : 0;
-    info->elem_variant = use_col_kernel(s) ? s->col_variant : -1;
+    info->elem_variant = col_kernel_eligible(s) && !s->point_kernel ? s->col_variant : -1;
     info->n_elem_variants = col_kernel_eligible(s) ? s->n_col_variants : 0;
     return GFB_OK;
 }
@@ -2654,8 +2905,20 @@ gfb_status gfb_element_residual(int32_t n_elem, const double* dxi_dx, const doub
             for (int c = 0; c < 3; ++c) h[q * 4 + c] = (float)u[q * 3 + c];
         if ((st = h2d(s, s->ut, h.data(), nP * 4))) return st;
     }
-    if ((st = launch_elem(s, 0))) return st;
+    if ((st = launch_elem(s))) return st;
     CU(cudaStreamSynchronize(s->stream));
+    if (use_gather(s)) {  // one touch per node: the contributions are the residual
+        auto read = [&](auto zero) -> gfb_status {
+            const size_t row = (size_t)gfb::gather_chunk_units<decltype(zero)>(nn, 1) * 3;
+            std::vector<decltype(zero)> h((size_t)n_elem * row);
+            gfb_status rs = d2h(s, h.data(), s->contrib, h.size() * sizeof(zero));
+            if (rs) return rs;
+            for (long long e = 0; e < n_elem; ++e)
+                for (int x = 0; x < nn * 3; ++x) r[e * nn * 3 + x] = h[(size_t)e * row + x];
+            return GFB_OK;
+        };
+        return precision == GFB_FP64 ? read(0.0) : read(0.0f);
+    }
     if (precision == GFB_FP64) {
         std::vector<double> h(nP);
         if ((st = d2h(s, h.data(), s->force, nP * 8))) return st;

@@ -98,17 +98,17 @@ typedef struct gfb_config {
  * Slower on B200 as laid out today: the epilogue's scattered per-node
  * accesses cost far more L1 transactions than the contiguous node pass. */
 #define GFB_FLAG_FUSED_NODE 4
-/* Run the FP32 path with the thread-per-GLL-point element kernel instead of
- * the thread-per-xi-line kernel (same arithmetic, different summation order;
- * for comparisons). */
+/* Run the thread-per-GLL-point element kernel with assembly by colour instead
+ * of the default thread-per-xi-line kernel (same arithmetic, different
+ * summation order; for comparisons). */
 #define GFB_FLAG_POINT_KERNEL 8
 /* Launch each step's kernels one by one instead of replaying the step as a
  * captured CUDA graph. */
 #define GFB_FLAG_NO_GRAPH 16
-/* At the end of gfb_create(_batch), time full colour sweeps of each FP32
- * element-kernel candidate (the line kernel with each cells-per-group count
- * it is built with, and the thread-per-point kernel) on this mesh and keep
- * the fastest; gfb_get_info reports the choice.  Tuning leaves the state
+/* At the end of gfb_create(_batch), time full sweeps of each FP32
+ * element-kernel candidate (the default, the line kernel by colour with each
+ * cells-per-group count it is built with, and the thread-per-point kernel) on
+ * this mesh and keep the fastest; gfb_get_info reports the choice.  Tuning leaves the state
  * unchanged. */
 #define GFB_FLAG_AUTOTUNE 32
 /* FP32 path: evaluate the element force from the full predicted
@@ -240,7 +240,7 @@ gfb_status gfb_advance_profiled(gfb_solver* solver, int32_t n_steps, double* ms_
 
 /* Static description of a solver and its cumulative kernel-launch count. */
 typedef struct gfb_info {
-    int32_t n_colour;        /* assembly colours (launches of the element kernel per step) */
+    int32_t n_colour;        /* colours of an assembly by colour (element_kernel variants -1, 1..3) */
     int32_t n_pml_cell;      /* cells with C-PML state                                      */
     int32_t n_rec_cell;
     int32_t n_field;
@@ -254,16 +254,15 @@ typedef struct gfb_info {
     int32_t n_pml_node;      /* global nodes carrying C-PML state (0: per-cell form)        */
     int32_t elem_blocks;     /* blocks in the persistent grid of the element kernel in use  */
     int32_t elem_kernel;     /* 1: thread-per-xi-line kernel, 0: thread-per-point kernel    */
-    int32_t cells_per_group; /* cells per block iteration of the line kernel (0 otherwise)  */
+    int32_t cells_per_group; /* cells a thread-per-xi-line kernel takes at a time (0 otherwise) */
     int32_t force_refresh;   /* steps between full element-force evaluations (1: every step) */
     int32_t half_v;          /* 1: plain nodes keep the half-step velocity, no acceleration */
-    int32_t elem_variant;    /* FP32 element kernel in use: -1 thread-per-point; line kernel
-                                0 the default (at ngll 5 with <= 3 wavefields: eta/zeta
-                                contractions by line owners); there also 1 one fewer cell
-                                per group, 2 one more, 3 the default count, the exchange
-                                done by every thread                                         */
-    int32_t n_elem_variants; /* line-kernel variants built for this ngll / field count
-                                (0: the solver has one element kernel)                        */
+    int32_t elem_variant;    /* FP32 element kernel in use: -1 thread-per-point by colour; 0 the
+                                default (cell contributions assembled by the node pass); at
+                                ngll 5 with <= 3 wavefields also the line kernel by colour with 1
+                                one fewer cell per group, 2 one more, 3 its default count        */
+    int32_t n_elem_variants; /* variants built for this ngll / field count (0: the solver has
+                                one element kernel)                                            */
 } gfb_info;
 
 gfb_status gfb_get_info(const gfb_solver* solver, gfb_info* info);
