@@ -1578,10 +1578,11 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
     if (s->has_cpml && !s->node_pml) {
         std::vector<int> slot(n_cell, -1);
         std::vector<long long> slot_cell;
-        for (long long ed = 0; ed < n_cell; ++ed)
-            if (m->pml_region[ed] != 0) {
-                slot[ed] = (int)slot_cell.size();
-                slot_cell.push_back(ed);
+        // in the order of clist, which is that of the memory in a checkpoint
+        for (long long x = 0; x < n_cell; ++x)
+            if (m->pml_region[clist[x]] != 0) {
+                slot[clist[x]] = (int)slot_cell.size();
+                slot_cell.push_back(clist[x]);
             }
         s->n_pml = (int)slot_cell.size();
         {
