@@ -1600,6 +1600,11 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_>::THREADS, ColShape<NG
 // node words two groups and the displacement vectors one wavefield ahead are
 // register loads.  The contributions of a chunk of wavefields are collected in
 // shared memory and leave as one bulk store per cell.
+//
+// Measured on 40 x 40 x 20 cells of ngll 5: FP32 with three wavefields 205 us
+// (3,780 instructions and 1,020 shared wavefronts per cell, the L1 pipe 69 %
+// busy, issue 57 %, DRAM 24 %); by colour the same took about 310 us.  FP64
+// with one wavefield and per-cell C-PML in half of the cells 378 us.
 // ---------------------------------------------------------------------------
 
 // Point (i, j, k) of an exchange array at P*i + NG*j + k, a cell's component
@@ -1672,6 +1677,7 @@ struct GatherArgs {
     const ModelConst* mc;          // [model]
     unsigned* err;                 // set to 1 when a bulk copy's wait gave up (the launch did not finish)
     Real D[36];                    // D[i*NG+s], read with compile-time indices only
+    float2 D2[36];                 // the same twice, for packed operations (FP32)
 };
 
 // C-PML of one wavefield at the points of this thread's line (pml.cpp:55-216):
@@ -1719,6 +1725,57 @@ __device__ __forceinline__ void line_cell_pml(const GatherArgs<Real>& A, int slo
             prev[c * NN] = nv;
         }
     }
+}
+
+// Packed pairs of FP32 operations (one instruction for two, sm_100) beside the
+// plain ones, so that one expression serves two points or one.
+__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double vfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ double vmul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double vadd(double a, double b) { return __dadd_rn(a, b); }
+// One value, or two that lie `step` apart.
+template <typename Real>
+__device__ __forceinline__ void vload(const Real* p, int, Real& x) { x = p[0]; }
+__device__ __forceinline__ void vload(const float* p, int step, float2& x) { x = make_float2(p[0], p[step]); }
+template <typename Real>
+__device__ __forceinline__ void vstore(Real* p, int, Real x) { p[0] = x; }
+__device__ __forceinline__ void vstore(float* p, int step, float2 x) { p[0] = x.x, p[step] = x.y; }
+__device__ __forceinline__ float2 vpair(float a, float b) { return make_float2(a, b); }
+
+// Gradient to fluxes at one point (V = Real) or, in FP32, two (float2) whose
+// geometry lies `step` apart: g[c][b] the derivatives of component c along
+// reference axis b; fl[b][c] the flux along axis b.
+template <typename Real, typename V>
+__device__ __forceinline__ void point_fluxes(const Real* geo, int nn, int step, const V (&g)[3][3], V (&fl)[3][3]) {
+    V dd[9], lam, mu, gr[3][3];
+#pragma unroll
+    for (int x = 0; x < 9; ++x) vload(geo + x * nn, step, dd[x]);
+    vload(geo + 9 * nn, step, lam);
+    vload(geo + 10 * nn, step, mu);
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+            gr[c][a] = vfma(g[c][2], dd[3 * a + 2], vfma(g[c][1], dd[3 * a + 1], vmul(g[c][0], dd[3 * a])));
+    const V tr = vmul(lam, vadd(vadd(gr[0][0], gr[1][1]), gr[2][2]));
+    const V m2 = vadd(mu, mu);
+    V st[3][3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) st[c][c] = vfma(m2, gr[c][c], tr);
+    st[0][1] = st[1][0] = vmul(mu, vadd(gr[0][1], gr[1][0]));
+    st[0][2] = st[2][0] = vmul(mu, vadd(gr[0][2], gr[2][0]));
+    st[1][2] = st[2][1] = vmul(mu, vadd(gr[1][2], gr[2][1]));
+    // flux along axis b: sigma . (dd[b], dd[3+b], dd[6+b])
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            fl[b][c] = vfma(st[c][2], dd[6 + b], vfma(st[c][1], dd[3 + b], vmul(st[c][0], dd[b])));
 }
 
 template <typename Real, int NG, bool PML>
@@ -1851,73 +1908,91 @@ __global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Re
                 load_vectors(nw, cell_of(next) >= 0, next % split * A.nfld_item, pre);
             }
             // the eta and zeta derivatives along this thread's lines, in place
-            auto contract = [&](auto coef) {
+            // (FP32: the two lines as one packed pair)
+            auto contract = [&](auto index) {
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     Real* le = xe + c * CELLS * SE + line_e;
                     Real* lz = xz + c * CELLS * SZ + line_z;
-                    Real ve[NG], vz[NG];
+                    if constexpr (sizeof(Real) == 4) {
+                        float2 v[NG];
 #pragma unroll
-                    for (int t = 0; t < NG; ++t) {
-                        ve[t] = le[t * NG];
-                        vz[t] = lz[t];
-                    }
+                        for (int t = 0; t < NG; ++t) v[t] = vpair(le[t * NG], lz[t]);
 #pragma unroll
-                    for (int s2 = 0; s2 < NG; ++s2) {
-                        Real de = Real(0), dz = Real(0);
+                        for (int s2 = 0; s2 < NG; ++s2) {
+                            float2 x = vmul(A.D2[index(s2, 0)], v[0]);
+#pragma unroll
+                            for (int t = 1; t < NG; ++t) x = vfma(A.D2[index(s2, t)], v[t], x);
+                            le[s2 * NG] = x.x;
+                            lz[s2] = x.y;
+                        }
+                    } else {
+                        Real ve[NG], vz[NG];
 #pragma unroll
                         for (int t = 0; t < NG; ++t) {
-                            de += coef(s2, t) * ve[t];
-                            dz += coef(s2, t) * vz[t];
+                            ve[t] = le[t * NG];
+                            vz[t] = lz[t];
                         }
-                        le[s2 * NG] = de;
-                        lz[s2] = dz;
+#pragma unroll
+                        for (int s2 = 0; s2 < NG; ++s2) {
+                            Real de = Real(0), dz = Real(0);
+#pragma unroll
+                            for (int t = 0; t < NG; ++t) {
+                                de += A.D[index(s2, t)] * ve[t];
+                                dz += A.D[index(s2, t)] * vz[t];
+                            }
+                            le[s2 * NG] = de;
+                            lz[s2] = dz;
+                        }
                     }
                 }
             };
-            if (lane_ok) contract([&](int s2, int t) { return A.D[s2 * NG + t]; });
+            if (lane_ok) contract([&](int s2, int t) { return s2 * NG + t; });
             sync();
             // gradient, stress and the three fluxes at each point of the line
             Real fx[3][NG];
             if (lane_ok) {
+                auto xi = [&](int c, int i) -> Real {
+                    Real x = A.D[i * NG] * u[c][0];
 #pragma unroll
-                for (int i = 0; i < NG; ++i) {
-                    const int p = i * NG2 + col;
-                    Real dd[9];
-#pragma unroll
-                    for (int q = 0; q < 9; ++q) dd[q] = geo[q * NN + p];
-                    const Real lam = geo[9 * NN + p], mu = geo[10 * NN + p];
-                    Real gr[3][3];
+                    for (int s = 1; s < NG; ++s) x = vfma(A.D[i * NG + s], u[c][s], x);
+                    return x;
+                };
+                // at points i and, in pairs, i + 1 (FP32: two at a time)
+                auto fluxes = [&](auto zero, int i) {
+                    using V = decltype(zero);
+                    V g[3][3], fl[3][3];
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        Real gx = Real(0);
-#pragma unroll
-                        for (int s = 0; s < NG; ++s) gx += A.D[i * NG + s] * u[c][s];
-                        const Real gy = xe[c * CELLS * SE + own_e + i * PE], gz = xz[c * CELLS * SZ + own_z + i * PZ];
-                        gr[c][0] = gx * dd[0] + gy * dd[1] + gz * dd[2];
-                        gr[c][1] = gx * dd[3] + gy * dd[4] + gz * dd[5];
-                        gr[c][2] = gx * dd[6] + gy * dd[7] + gz * dd[8];
+                        if constexpr (sizeof(V) > sizeof(Real)) g[c][0] = vpair(xi(c, i), xi(c, i + 1));
+                        else g[c][0] = xi(c, i);
+                        vload(xe + c * CELLS * SE + own_e + i * PE, PE, g[c][1]);
+                        vload(xz + c * CELLS * SZ + own_z + i * PZ, PZ, g[c][2]);
                     }
-                    const Real tr = lam * (gr[0][0] + gr[1][1] + gr[2][2]);
-                    const Real m2 = Real(2) * mu;
-                    const Real s0 = m2 * gr[0][0] + tr, s1 = m2 * gr[1][1] + tr, s2 = m2 * gr[2][2] + tr;
-                    const Real s3 = mu * (gr[0][1] + gr[1][0]), s4 = mu * (gr[0][2] + gr[2][0]),
-                               s5 = mu * (gr[1][2] + gr[2][1]);
-                    // flux along axis a: sigma . (dd[a], dd[3+a], dd[6+a])
-                    fx[0][i] = s0 * dd[0] + s3 * dd[3] + s4 * dd[6];
-                    fx[1][i] = s3 * dd[0] + s1 * dd[3] + s5 * dd[6];
-                    fx[2][i] = s4 * dd[0] + s5 * dd[3] + s2 * dd[6];
-                    xe[0 * CELLS * SE + own_e + i * PE] = s0 * dd[1] + s3 * dd[4] + s4 * dd[7];
-                    xe[1 * CELLS * SE + own_e + i * PE] = s3 * dd[1] + s1 * dd[4] + s5 * dd[7];
-                    xe[2 * CELLS * SE + own_e + i * PE] = s4 * dd[1] + s5 * dd[4] + s2 * dd[7];
-                    xz[0 * CELLS * SZ + own_z + i * PZ] = s0 * dd[2] + s3 * dd[5] + s4 * dd[8];
-                    xz[1 * CELLS * SZ + own_z + i * PZ] = s3 * dd[2] + s1 * dd[5] + s5 * dd[8];
-                    xz[2 * CELLS * SZ + own_z + i * PZ] = s4 * dd[2] + s5 * dd[5] + s2 * dd[8];
+                    point_fluxes(geo + i * NG2 + col, NN, NG2, g, fl);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        if constexpr (sizeof(V) > sizeof(Real)) {
+                            fx[c][i] = fl[0][c].x;
+                            fx[c][i + 1] = fl[0][c].y;
+                        } else {
+                            fx[c][i] = fl[0][c];
+                        }
+                        vstore(xe + c * CELLS * SE + own_e + i * PE, PE, fl[1][c]);
+                        vstore(xz + c * CELLS * SZ + own_z + i * PZ, PZ, fl[2][c]);
+                    }
+                };
+                constexpr int PAIRS = sizeof(Real) == 4 ? NG / 2 : 0;
+                if constexpr (PAIRS > 0) {
+#pragma unroll
+                    for (int h = 0; h < PAIRS; ++h) fluxes(float2{}, 2 * h);
                 }
+#pragma unroll
+                for (int i = 2 * PAIRS; i < NG; ++i) fluxes(Real(0), i);
             }
             sync();  // and the geometry has been read
             if (d + 1 == d1 && next < n_item) copy_geo(next);
-            if (lane_ok) contract([&](int s2, int t) { return A.D[t * NG + s2]; });
+            if (lane_ok) contract([&](int s2, int t) { return t * NG + s2; });
             if (gt == 0) bulk_wait_read();  // the chunk before has left the stage
             sync();
             Real r[3][NG];
@@ -1984,6 +2059,309 @@ __global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Re
         }
     }
     if (gt == 0) bulk_wait_all();
+}
+
+// ---------------------------------------------------------------------------
+// elem_plane_kernel: the gather kernel's work for wavefields in threes at
+// ngll 5 in FP32, one thread per xi-plane.
+//
+// A warp takes two cells and three wavefields: lane (cell, wavefield, i) owns
+// the 25 points (i, j, k) of one plane, with their displacement and the
+// residual it accumulates in registers, so the eta and zeta contractions, of
+// the gradient and of the divergence, touch no shared memory.  Only the xi
+// contractions exchange: lane (., i) also owns the five xi-lines of row j = i,
+// in place in one array.  Against one thread per xi-line (two directions
+// exchanged, 25 of 32 lanes) that halves the shared-memory accesses and takes
+// 30 of 32 lanes: 2,400 instructions and 580 shared wavefronts per cell
+// against 3,780 and 1,020.  It runs 8 warps per SM (255 registers), which the
+// independent work of 25 points per thread does not quite make up for (issue
+// slots 43 % busy; waits for the gathers, FMA latency and instruction fetch
+// on top): 32,000 cells x 3 wavefields take 173 us against 205, DRAM 25 %
+// busy in both.  Pairs of points use packed FP32 operations (2,900
+// instructions and 190 us without).  Point (i, j, k) of (cell, wavefield) q sits
+// at 135 q + 27 i + 5 j + k: a warp's own-point and line accesses fall in
+// distinct banks.  Node words come by bulk copy one item ahead, the geometry
+// as soon as the last one has been read; the contributions leave as one bulk
+// copy per cell, collected in the exchange array.
+// ---------------------------------------------------------------------------
+struct PlaneShape {
+    static constexpr int NG = 5, NN = 125, NG2 = 25, CELLS = 2, WARPS = 4, THREADS = 32 * WARPS;
+    static constexpr int PI = 27, SQ = 135, SC = 6 * SQ;  // words between planes, (cell, wavefield)s, components
+    static constexpr int GEO_B = geo_row<float>(NN) * 4;
+    static constexpr int GEO_SLOT = GEO_B + 48;            // 12 banks apart
+    static constexpr int IB_B = ib_row_words(NN) * 4;
+    static constexpr int CHUNK_W = gather_chunk_units<float>(NN, 3) * 3;
+    static constexpr int XCH_B = (3 * SC * 4 + 15) / 16 * 16;
+    static constexpr int WARP_B = CELLS * GEO_SLOT + 2 * CELLS * IB_B + XCH_B;
+    static constexpr int SMEM = WARPS * WARP_B;
+    static_assert(CELLS * CHUNK_W * 4 <= XCH_B, "the contributions fit in the exchange array");
+};
+
+static __global__ void __launch_bounds__(PlaneShape::THREADS, 2)
+    elem_plane_kernel(const __grid_constant__ GatherArgs<float> A) {
+    using S = PlaneShape;
+    constexpr int NG = S::NG, NN = S::NN, IB_W = ib_row_words(NN);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t s_bar[S::WARPS][3];  // geometry, node words (two stages)
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    unsigned char* geo_b = smem_raw + wp * S::WARP_B;
+    uint32_t* ibs = reinterpret_cast<uint32_t*>(geo_b + S::CELLS * S::GEO_SLOT);  // [2][CELLS][IB_W]
+    float* xch = reinterpret_cast<float*>(geo_b + S::CELLS * S::GEO_SLOT + 2 * S::CELLS * S::IB_B);
+    uint64_t* bar = s_bar[wp];
+    if (lane == 0) {
+        for (int b = 0; b < 3; ++b) mbar_init(bar + b, 1);
+        mbar_init_fence();
+    }
+    __syncwarp();
+    const bool lane_ok = lane < 30;
+    const int q = lane_ok ? lane / 5 : 0, i = lane_ok ? lane - 5 * q : 0;
+    const int cl = q / 3, f = q - 3 * cl;
+    const int n_cell = A.live_end ? min(A.n_cell, __ldg(A.live_end)) : A.n_cell;
+    const int split = A.nfld / A.nfld_item;
+    const int n_item = (n_cell + S::CELLS - 1) / S::CELLS * split;
+    const int step = gridDim.x * S::WARPS;
+    const int first = blockIdx.x * S::WARPS + wp;
+    const size_t row_u = (size_t)(A.nfld / 3) * (S::CHUNK_W / 3);
+    const float* geo = reinterpret_cast<const float*>(geo_b + cl * S::GEO_SLOT) + i * 25;
+    float* own = xch + q * S::SQ + i * S::PI;   // + c*SC + p
+    float* line = xch + q * S::SQ + 5 * i;      // + c*SC + s*PI + k
+
+    auto copy_geo = [&](int item) {
+        if (lane != 0) return;
+        const int e0 = item / split * S::CELLS, nc = min(S::CELLS, n_cell - e0);
+        fence_proxy_async_smem();
+        mbar_expect_tx(bar, (unsigned)(nc * S::GEO_B));
+        for (int c = 0; c < nc; ++c)
+            bulk_copy_g2s(geo_b + c * S::GEO_SLOT, A.geom + (size_t)(e0 + c) * geo_row<float>(NN), S::GEO_B, bar);
+    };
+    auto copy_words = [&](int item, int st) {
+        if (lane != 0) return;
+        const int e0 = item / split * S::CELLS, nc = min(S::CELLS, n_cell - e0);
+        fence_proxy_async_smem();
+        mbar_expect_tx(bar + 1 + st, (unsigned)(nc * S::IB_B));
+        bulk_copy_g2s(ibs + st * S::CELLS * IB_W, A.ibool_padded + (size_t)e0 * IB_W, (unsigned)(nc * S::IB_B), bar + 1 + st);
+    };
+    // a wait that gave up: flag it, give the copies in flight a second
+    // bounded wait, leave (the whole warp)
+    auto give_up = [&](unsigned pg, int b1, unsigned p1, int b2, unsigned p2) {
+        if (lane == 0) {
+            atomicOr(A.err, 1u);
+            mbar_wait(bar, pg);
+            if (b1 >= 0) mbar_wait(bar + b1, p1);
+            if (b2 >= 0) mbar_wait(bar + b2, p2);
+            bulk_wait_all();
+        }
+    };
+
+    if (first < n_item) {
+        copy_words(first, 0);
+        copy_geo(first);
+    }
+    int it = 0;
+    for (int item = first; item < n_item; item += step, ++it) {
+        const int st = it & 1, next = item + step;
+        const unsigned pw = (unsigned)(it >> 1) & 1u, pg = (unsigned)it & 1u;
+        if (next < n_item) copy_words(next, st ^ 1);
+        if (__any_sync(0xffffffffu, !mbar_wait(bar + 1 + st, pw))) {
+            give_up(pg, 1 + st, pw, next < n_item ? 2 - st : -1, (unsigned)((it + 1) >> 1) & 1u);
+            return;
+        }
+        const int e0 = item / split * S::CELLS, e = e0 + cl;
+        const bool in = lane_ok && e < n_cell;
+        const uint32_t* words = ibs + (st * S::CELLS + cl) * IB_W;
+        const int mdl = A.multi && in ? (int)words[NN] : 0;
+        const int src0 = in && A.src_head ? __ldg(A.src_head + e) : -1;
+        const int d0 = item % split * A.nfld_item, d1 = d0 + A.nfld_item;
+        for (int g0 = d0; g0 < d1; g0 += 3) {
+            // row j of component c: points k = 0, 1 | 2, 3 | 4
+            float2 u2[3][NG][2];
+            float u1[3][NG];
+#pragma unroll
+            for (int j = 0; j < NG; ++j) {
+                float4 t[NG];
+#pragma unroll
+                for (int k = 0; k < NG; ++k) {
+                    const uint32_t w = in ? words[i * 25 + j * NG + k] & kNodeMask : 0u;
+                    t[k] = __ldg(reinterpret_cast<const float4*>(A.ut) + (size_t)w * A.nfld + g0 + f);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    u2[0][j][h] = make_float2(t[2 * h].x, t[2 * h + 1].x);
+                    u2[1][j][h] = make_float2(t[2 * h].y, t[2 * h + 1].y);
+                    u2[2][j][h] = make_float2(t[2 * h].z, t[2 * h + 1].z);
+                }
+                u1[0][j] = t[4].x, u1[1][j] = t[4].y, u1[2][j] = t[4].z;
+            }
+            auto u_at = [&](int c, int j, int k) -> float {
+                return k == 4 ? u1[c][j] : (k & 1 ? u2[c][j][k / 2].y : u2[c][j][k / 2].x);
+            };
+            if (lane == 0) bulk_wait_read();  // the contributions before have left the exchange array
+            __syncwarp();
+            if (lane_ok) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+#pragma unroll
+                    for (int p = 0; p < 25; ++p) own[c * S::SC + p] = u_at(c, p / NG, p % NG);
+            }
+            __syncwarp();
+            // the xi contractions along this lane's five lines, in place
+            auto contract = [&](auto coef) {
+#pragma unroll 1  // a third of the code: instruction fetch shows here
+                for (int c = 0; c < 3; ++c) {
+                    auto lines = [&](auto zero, int k) {
+                        decltype(zero) v[NG];
+                        float* l = line + c * S::SC + k;
+#pragma unroll
+                        for (int t = 0; t < NG; ++t) vload(l + t * S::PI, 1, v[t]);
+#pragma unroll
+                        for (int s = 0; s < NG; ++s) {
+                            decltype(zero) x = vmul(coef(zero, s, 0), v[0]);
+#pragma unroll
+                            for (int t = 1; t < NG; ++t) x = vfma(coef(zero, s, t), v[t], x);
+                            vstore(l + s * S::PI, 1, x);
+                        }
+                    };
+                    lines(float2{}, 0);
+                    lines(float2{}, 2);
+                    lines(0.f, 4);
+                }
+            };
+            struct Coef {
+                const GatherArgs<float>& A;
+                __device__ __forceinline__ float2 operator()(float2, int a, int b) const { return A.D2[a * 5 + b]; }
+                __device__ __forceinline__ float operator()(float, int a, int b) const { return A.D[a * 5 + b]; }
+            };
+            const Coef D{A};
+            if (lane_ok) contract([&](auto z, int s, int t) { return D(z, s, t); });
+            if (g0 == d0 && __any_sync(0xffffffffu, !mbar_wait(bar, pg))) {
+                give_up(pg, next < n_item ? 2 - st : -1, (unsigned)((it + 1) >> 1) & 1u, -1, 0);
+                return;
+            }
+            __syncwarp();
+            float2 r2[3][NG][2];
+            float r1[3][NG];
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int j = 0; j < NG; ++j) {
+                    r2[c][j][0] = r2[c][j][1] = make_float2(0.f, 0.f);
+                    r1[c][j] = 0.f;
+                }
+            if (lane_ok) {
+#pragma unroll
+                for (int j = 0; j < NG; ++j) {
+                    float z[3][NG];  // the zeta fluxes of the row
+                    // d/d-zeta at k: a scalar contraction along the row
+                    auto dz = [&](int c, int k) -> float {
+                        float x = A.D[k * NG] * u_at(c, j, 0);
+#pragma unroll
+                        for (int s = 1; s < NG; ++s) x = vfma(A.D[k * NG + s], u_at(c, j, s), x);
+                        return x;
+                    };
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int k = 2 * h, p = j * NG + k;
+                        float2 g[3][3], fl[3][3];
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            vload(own + c * S::SC + p, 1, g[c][0]);
+                            g[c][1] = vmul(A.D2[j * NG], u2[c][0][h]);
+#pragma unroll
+                            for (int s = 1; s < NG; ++s) g[c][1] = vfma(A.D2[j * NG + s], u2[c][s][h], g[c][1]);
+                            g[c][2] = make_float2(dz(c, k), dz(c, k + 1));
+                        }
+                        point_fluxes(geo + p, NN, 1, g, fl);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            vstore(own + c * S::SC + p, 1, fl[0][c]);
+#pragma unroll
+                            for (int s = 0; s < NG; ++s) r2[c][s][h] = vfma(A.D2[j * NG + s], fl[1][c], r2[c][s][h]);
+                            z[c][k] = fl[2][c].x;
+                            z[c][k + 1] = fl[2][c].y;
+                        }
+                    }
+                    {
+                        const int p = j * NG + 4;
+                        float g[3][3], fl[3][3];
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            g[c][0] = own[c * S::SC + p];
+                            g[c][1] = A.D[j * NG] * u1[c][0];
+#pragma unroll
+                            for (int s = 1; s < NG; ++s) g[c][1] = vfma(A.D[j * NG + s], u1[c][s], g[c][1]);
+                            g[c][2] = dz(c, 4);
+                        }
+                        point_fluxes(geo + p, NN, 1, g, fl);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            own[c * S::SC + p] = fl[0][c];
+#pragma unroll
+                            for (int s = 0; s < NG; ++s) r1[c][s] = vfma(A.D[j * NG + s], fl[1][c], r1[c][s]);
+                            z[c][4] = fl[2][c];
+                        }
+                    }
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+#pragma unroll
+                        for (int k = 0; k < NG; ++k) {
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                r2[c][j][h].x = vfma(A.D[k * NG + 2 * h], z[c][k], r2[c][j][h].x);
+                                r2[c][j][h].y = vfma(A.D[k * NG + 2 * h + 1], z[c][k], r2[c][j][h].y);
+                            }
+                            r1[c][j] = vfma(A.D[k * NG + 4], z[c][k], r1[c][j]);
+                        }
+                }
+            }
+            __syncwarp();  // and the geometry has been read
+            if (g0 + 3 >= d1 && next < n_item) copy_geo(next);
+            if (lane_ok) contract([&](auto z, int s, int t) { return D(z, t, s); });
+            __syncwarp();
+            float r[3][25];
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int j = 0; j < NG; ++j)
+#pragma unroll
+                    for (int k = 0; k < NG; ++k) {
+                        const float x = k == 4 ? r1[c][j] : (k & 1 ? r2[c][j][k / 2].y : r2[c][j][k / 2].x);
+                        r[c][j * NG + k] = -(x + own[c * S::SC + j * NG + k]);
+                    }
+            // point force (solver.cpp:577-605)
+            if (src0 >= 0 && A.mstf) {
+                const int d = g0 + f, fs = A.fset[d], dir = A.dir[d];
+                const float stf = __ldg(A.mstf + mdl * A.n_set + fs);
+                for (int sl = stf != 0.f ? src0 : -1; sl >= 0; sl = __ldg(A.src_next + sl)) {
+                    if (A.src_set && __ldg(A.src_set + sl) != fs) continue;
+#pragma unroll
+                    for (int p = 0; p < 25; ++p) {
+                        const float sw = stf * __ldg(A.src_w + (size_t)sl * NN + i * 25 + p);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c)
+                            if (c == dir) r[c][p] += sw;
+                    }
+                }
+            }
+            __syncwarp();  // every lane has read the exchange array
+            if (lane_ok) {
+                float* out = xch + cl * S::CHUNK_W + i * 225 + 3 * f;
+#pragma unroll
+                for (int p = 0; p < 25; ++p)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) out[p * 9 + c] = r[c][p];
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                const int nc = min(S::CELLS, n_cell - e0);
+                for (int c = 0; c < nc; ++c)
+                    bulk_copy_s2g(A.contrib + ((size_t)(e0 + c) * row_u + (size_t)(g0 / 3) * (S::CHUNK_W / 3)) * 3,
+                                  xch + c * S::CHUNK_W, (unsigned)(S::CHUNK_W * 4));
+                bulk_commit();
+            }
+        }
+    }
+    if (lane == 0) bulk_wait_all();
 }
 
 // Predictor only (start of a run or after a state overwrite).

@@ -264,6 +264,7 @@ struct gfb_solver {
     uint4* touch = nullptr;         // [node] (gfb::NodeGather)
     uint4* touch_more = nullptr;
     int gather_blocks = 0;          // persistent grid of the gather kernel
+    int plane_blocks = 0;           // of the plane kernel (0: not used)
     bool has_cpml = false, has_damping = false, has_src = false;
     int n_pml = 0, n_src = 0, n_rec = 0, slots = 0;
     double c1 = 0.0, c2 = 0.0;
@@ -741,9 +742,25 @@ gfb_status launch_gather_t(gfb_solver* s) {
     A.mc = s->d_mc;
     A.err = reinterpret_cast<unsigned*>(s->d_kernel_err);
     for (int q = 0; q < 36; ++q) A.D[q] = q < NG * NG ? (Real)s->dmat_host[q] : Real(0);
+    for (int q = 0; q < 36; ++q) A.D2[q] = make_float2((float)A.D[q], (float)A.D[q]);
     // a work item is a group's cells with all their wavefields (the geometry
     // read once), or one wavefield of them where that would leave more than
     // half of the resident groups without work
+    // wavefields in threes at ngll 5 in FP32: the plane kernel (faster from
+    // 20 x 20 x 10 cells up, 76 against 82 us per step, level below)
+    if constexpr (std::is_same<Real, float>::value && NG == 5) {
+        if (s->plane_blocks > 0) {
+            using PS = gfb::PlaneShape;
+            const int pairs = (s->n_cell + PS::CELLS - 1) / PS::CELLS;
+            A.nfld_item = 2 * pairs <= s->plane_blocks * PS::WARPS ? 3 : s->nfld;
+            const int n = pairs * (s->nfld / A.nfld_item);
+            const int blocks = std::max(1, std::min((n + PS::WARPS - 1) / PS::WARPS, s->plane_blocks));
+            gfb::elem_plane_kernel<<<blocks, PS::THREADS, PS::SMEM, s->stream>>>(A);
+            CU(cudaGetLastError());
+            s->launches++;
+            return GFB_OK;
+        }
+    }
     const int groups = (s->n_cell + S::CELLS - 1) / S::CELLS;
     A.nfld_item = 2 * groups <= s->gather_blocks * S::GROUPS ? 1 : s->nfld;
     const int items = groups * (s->nfld / A.nfld_item);
@@ -767,6 +784,14 @@ gfb_status gather_grid_t(gfb_solver* s) {
     CU(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, s->device));
     if (per_sm < 1) return fail(GFB_ERR_UNSUPPORTED, "gather element kernel does not fit on an SM");
     s->gather_blocks = per_sm * n_sm;
+    if constexpr (std::is_same<Real, float>::value && NG == 5) {
+        if (s->nfld % 3 == 0 && !(s->has_cpml && !s->node_pml)) {
+            using PS = gfb::PlaneShape;
+            CU(cudaFuncSetAttribute(gfb::elem_plane_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PS::SMEM));
+            CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gfb::elem_plane_kernel, PS::THREADS, PS::SMEM));
+            s->plane_blocks = per_sm * n_sm;
+        }
+    }
     return GFB_OK;
 }
 

@@ -63,6 +63,7 @@ def states(prob, dirs, prec, flags):
 
 @pytest.mark.parametrize("prec,tol", [(gfb.FP64, 1e-12), (gfb.FP32, 4e-5)])
 @pytest.mark.parametrize("ngll,n_cell,dirs", [(3, 1, [0]), (3, 7, [0, 1, 2]), (4, 5, [2, 0]), (5, 1, [1]),
+                                              (5, 1, [2, 1, 0]),
                                               (5, 13, [0, 1, 2]), (5, 37, [2]), (6, 2, [0]), (6, 7, [1, 2, 0])])
 def test_gather_assembly_equals_assembly_by_colour(ngll, n_cell, dirs, prec, tol):
     for cpml in (False, True):
