@@ -433,6 +433,19 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 
+// Programmatic dependent launch along a step: step start -> element kernel ->
+// node passes -> next step's start.  A kernel launched this way may start
+// before the one before it has finished: it sets itself up from arrays no
+// kernel writes (node words, geometry, touches, C-PML coefficients), then
+// pdl_wait() returns when the kernel before has completed and its writes are
+// visible.  Every kernel of the chain calls pdl_wait() before it ends, so its
+// completion implies that of all before it.  pdl_launch(): the next kernel may
+// start now; it comes after pdl_wait(), so no kernel starts before the one
+// two before it has completed.  What a kernel of the chain writes is read with
+// ordinary or L2 loads, not through the read-only path.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Real operations rounded the same way wherever the node update is inlined
 // (node passes, fused update).
 __device__ __forceinline__ float rfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
@@ -592,7 +605,7 @@ __device__ __forceinline__ bool node_constants(const NodeArgs<Real>& A, const No
         return true;
     }
     const int m = __ldg(A.node_model + g);
-    if (!__ldg(A.mlive + m)) return false;
+    if (!__ldcg(A.mlive + m)) return false;
     K = A.mc[m];
     full = A.mnext ? A.mnext[m] != 0 : true;
     return true;
@@ -610,7 +623,7 @@ struct ForceParts {
     static __device__ __forceinline__ void touch(const Real* base, uint32_t q, bool on, Real (&x)[3]) {
         const Real* p = base + (size_t)q * 3;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) x[k] = on ? __ldg(p + k) : Real(0);
+        for (int k = 0; k < 3; ++k) x[k] = on ? p[k] : Real(0);
     }
     __device__ __forceinline__ void load(const NodeArgs<Real>& A, long long g, int d, const uint4& t, bool add) {
         const Real* base = touches(A, d);
@@ -665,14 +678,22 @@ struct ForceParts {
 // nodes [g0, n_node), node_pml_kernel over the C-PML nodes [0, g0).
 constexpr int kNodeThreads = 128, kNodeTile = 32;
 
+// wait: the element phase may still run when this pass starts.  The C-PML
+// pass, which follows the plain pass, does not wait for it: the plain pass
+// lets it start once its own wait is over, and the two write different nodes.
 template <typename Real, int NFLD, bool MULTI, bool PML, bool HALF_V>
-__device__ __forceinline__ void node_pass(const NodeArgs<Real>& A, const NodePml<Real>& P, long long g0, long long g1) {
+__device__ __forceinline__ void node_pass(const NodeArgs<Real>& A, const NodePml<Real>& P, long long g0, bool wait) {
     constexpr int TN = kNodeTile, WARPS = kNodeThreads / 32;
     constexpr int COEF_W = 16 / (int)sizeof(Real), COEF_N = PML ? TN * 14 : COEF_W;
     __shared__ __align__(16) uint4 s_touch[WARPS][3][TN];
     __shared__ __align__(16) Real s_cf[PML ? WARPS : 1][3][COEF_N];
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     const bool gather = A.gather.touch != nullptr;
+    long long g1 = PML ? P.n_slot : A.n_node;
+    if (MULTI && A.live_node_end) {  // this step's bounds
+        if (wait) pdl_wait();
+        g1 = min(g1, A.live_node_end[PML ? 0 : 1]);
+    }
     const long long n_tile = (g1 - g0 + TN - 1) / TN;
     const long long step = (long long)gridDim.x * WARPS;
     auto fetch = [&](long long tile, int st) {
@@ -686,15 +707,17 @@ __device__ __forceinline__ void node_pass(const NodeArgs<Real>& A, const NodePml
         }
         cp_async_commit();
     };
+    const long long first = (long long)blockIdx.x * WARPS + wp;
+    fetch(first, 0);
+    fetch(first + step, 1);
+    if (wait) pdl_wait();
+    pdl_launch();
     ModelConst K;
     bool full, add = false;
     if (!MULTI) {
         node_constants<Real, MULTI>(A, P, 0, K, full);
-        add = A.gather.keep && A.gather.mdirect && __ldg(A.gather.mdirect) == 0;
+        add = A.gather.keep && A.gather.mdirect && __ldcg(A.gather.mdirect) == 0;
     }
-    const long long first = (long long)blockIdx.x * WARPS + wp;
-    fetch(first, 0);
-    fetch(first + step, 1);
     int st = 0;
     for (long long tile = first; tile < n_tile; tile += step) {
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
@@ -715,7 +738,7 @@ __device__ __forceinline__ void node_pass(const NodeArgs<Real>& A, const NodePml
             ForceParts<Real, NFLD> p;
             if (gather) {
                 if (MULTI)
-                    add = A.gather.keep && A.gather.mdirect && __ldg(A.gather.mdirect + __ldg(A.node_model + g)) == 0;
+                    add = A.gather.keep && A.gather.mdirect && __ldcg(A.gather.mdirect + __ldg(A.node_model + g)) == 0;
                 p.load(A, g, d, t, add);
             } else {
                 load4(A.force + ((size_t)g * NFLD + d) * 4, p.old);
@@ -729,6 +752,7 @@ __device__ __forceinline__ void node_pass(const NodeArgs<Real>& A, const NodePml
         st = st == 2 ? 0 : st + 1;
     }
     cp_async_wait_all();
+    if (!wait) pdl_wait();
 }
 
 // Resident blocks per SM.  The passes are bound by DRAM and by the loads in
@@ -746,15 +770,13 @@ constexpr int node_blocks_per_sm(bool pml) {
 template <typename Real, int NFLD, bool MULTI, bool HALF_V>
 __global__ void __launch_bounds__(kNodeThreads, node_blocks_per_sm<Real>(false))
     node_update_kernel(const __grid_constant__ NodeArgs<Real> A, const __grid_constant__ NodePml<Real> P, long long g0) {
-    node_pass<Real, NFLD, MULTI, false, HALF_V>(A, P, g0,
-                                                (MULTI && A.live_node_end) ? min(A.n_node, A.live_node_end[1]) : A.n_node);
+    node_pass<Real, NFLD, MULTI, false, HALF_V>(A, P, g0, true);
 }
 
 template <int NFLD, bool MULTI>
 __global__ void __launch_bounds__(kNodeThreads, node_blocks_per_sm<float>(true))
-    node_pml_kernel(const __grid_constant__ NodeArgs<float> A, const __grid_constant__ NodePml<float> P) {
-    node_pass<float, NFLD, MULTI, true, false>(A, P, 0,
-                                               (MULTI && A.live_node_end) ? min(P.n_slot, A.live_node_end[0]) : P.n_slot);
+    node_pml_kernel(const __grid_constant__ NodeArgs<float> A, const __grid_constant__ NodePml<float> P, bool wait) {
+    node_pass<float, NFLD, MULTI, true, false>(A, P, 0, wait);
 }
 
 // The assembled force alone (a learned layer adds to it between the element
@@ -798,6 +820,8 @@ __global__ void step_begin_kernel(int n_model, int n_set, int* mstep, const int*
                                   const long long* stf_off, const Real* stf_all, Real* mstf, int* mlive, int period,
                                   int* force_direct, int* mdirect, int* mnext) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
+    pdl_launch();
     if (m >= n_model) return;
     const int t = mstep[m];
     const bool live = t < nsteps[m];
@@ -829,6 +853,8 @@ __global__ void step_begin_kernel(int n_model, int n_set, int* mstep, const int*
 static __global__ void live_bounds_kernel(int n_model, int n_colour, const int* mlive, const int* cell_end,
                                    const int* colour_first, const long long* node_end, long long plain_first,
                                    int* live_cell_end, long long* live_node_end) {
+    pdl_wait();
+    pdl_launch();
     for (int c = threadIdx.x; c < n_colour + 2; c += blockDim.x) {
         if (c < n_colour) {
             int e = colour_first[c];
@@ -1810,7 +1836,8 @@ __global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Re
     const int cl = lane_ok ? gt / NG2 : 0;
     const int col = lane_ok ? gt - cl * NG2 : 0;
     const int j = col / NG, k = col - j * NG;
-    const int n_cell = A.live_end ? min(A.n_cell, __ldg(A.live_end)) : A.n_cell;
+    if (A.live_end) pdl_wait();
+    const int n_cell = A.live_end ? min(A.n_cell, __ldcg(A.live_end)) : A.n_cell;
     const int split = A.nfld / A.nfld_item;
     const int fc = gather_chunk_fields<Real>(A.nfld), chunk_u = gather_chunk_units<Real>(NN, A.nfld);
     const bool staged = A.nfld_item % fc == 0;  // an item fills whole chunks
@@ -1844,11 +1871,11 @@ __global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Re
         for (int i = 0; i < NG; ++i) {
             const Real* src = A.ut + ((size_t)(w[i] & kNodeMask) * A.nfld + d) * 4;
             if constexpr (sizeof(Real) == 4) {
-                const float4 t = ok ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 t = ok ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
                 x[0][i] = t.x, x[1][i] = t.y, x[2][i] = t.z;
             } else {
-                const double2 t = ok ? __ldg(reinterpret_cast<const double2*>(src)) : make_double2(0.0, 0.0);
-                x[0][i] = t.x, x[1][i] = t.y, x[2][i] = ok ? __ldg(src + 2) : 0.0;
+                const double2 t = ok ? *reinterpret_cast<const double2*>(src) : make_double2(0.0, 0.0);
+                x[0][i] = t.x, x[1][i] = t.y, x[2][i] = ok ? src[2] : 0.0;
             }
         }
     };
@@ -1858,12 +1885,14 @@ __global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Re
     load_words(first, nw);
     load_words(first + step, nw2);
     if (first < n_item) copy_geo(first);
+    pdl_wait();
+    pdl_launch();
     load_vectors(nw, cell_of(first) >= 0, first % split * A.nfld_item, pre);
     unsigned phase = 0;
     for (int item = first; item < n_item; item += step) {
         const int e = cell_of(item), next = item + step;
         const int mdl = A.multi && e >= 0 ? (int)__ldg(A.ibool_padded + (size_t)e * IB_W + NN) : 0;
-        const bool act = e >= 0 && __ldg(A.mlive + mdl) != 0;
+        const bool act = e >= 0 && __ldcg(A.mlive + mdl) != 0;
         const int src0 = act && A.src_head ? __ldg(A.src_head + e) : -1;
         const int slot = PML && act ? __ldg(A.pml_slot + e) : -1;
 #pragma unroll
@@ -2012,7 +2041,7 @@ __global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Re
             // point force (solver.cpp:577-605)
             if (src0 >= 0 && A.mstf) {
                 const int fs = A.fset[d], dir = A.dir[d];
-                const Real stf = __ldg(A.mstf + mdl * A.n_set + fs);
+                const Real stf = __ldcg(A.mstf + mdl * A.n_set + fs);
                 for (int sl = stf != Real(0) ? src0 : -1; sl >= 0; sl = __ldg(A.src_next + sl)) {
                     if (A.src_set && __ldg(A.src_set + sl) != fs) continue;
 #pragma unroll
@@ -2116,7 +2145,8 @@ static __global__ void __launch_bounds__(PlaneShape::THREADS, 2)
     const bool lane_ok = lane < 30;
     const int q = lane_ok ? lane / 5 : 0, i = lane_ok ? lane - 5 * q : 0;
     const int cl = q / 3, f = q - 3 * cl;
-    const int n_cell = A.live_end ? min(A.n_cell, __ldg(A.live_end)) : A.n_cell;
+    if (A.live_end) pdl_wait();
+    const int n_cell = A.live_end ? min(A.n_cell, __ldcg(A.live_end)) : A.n_cell;
     const int split = A.nfld / A.nfld_item;
     const int n_item = (n_cell + S::CELLS - 1) / S::CELLS * split;
     const int step = gridDim.x * S::WARPS;
@@ -2157,6 +2187,8 @@ static __global__ void __launch_bounds__(PlaneShape::THREADS, 2)
         copy_words(first, 0);
         copy_geo(first);
     }
+    pdl_wait();
+    pdl_launch();
     int it = 0;
     for (int item = first; item < n_item; item += step, ++it) {
         const int st = it & 1, next = item + step;
@@ -2182,7 +2214,7 @@ static __global__ void __launch_bounds__(PlaneShape::THREADS, 2)
 #pragma unroll
                 for (int k = 0; k < NG; ++k) {
                     const uint32_t w = in ? words[i * 25 + j * NG + k] & kNodeMask : 0u;
-                    t[k] = __ldg(reinterpret_cast<const float4*>(A.ut) + (size_t)w * A.nfld + g0 + f);
+                    t[k] = reinterpret_cast<const float4*>(A.ut)[(size_t)w * A.nfld + g0 + f];
                 }
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
@@ -2330,7 +2362,7 @@ static __global__ void __launch_bounds__(PlaneShape::THREADS, 2)
             // point force (solver.cpp:577-605)
             if (src0 >= 0 && A.mstf) {
                 const int d = g0 + f, fs = A.fset[d], dir = A.dir[d];
-                const float stf = __ldg(A.mstf + mdl * A.n_set + fs);
+                const float stf = __ldcg(A.mstf + mdl * A.n_set + fs);
                 for (int sl = stf != 0.f ? src0 : -1; sl >= 0; sl = __ldg(A.src_next + sl)) {
                     if (A.src_set && __ldg(A.src_set + sl) != fs) continue;
 #pragma unroll

@@ -330,7 +330,8 @@ struct gfb_solver {
     long long* d_stf_off = nullptr;
     void *d_mstf = nullptr, *d_stf_all = nullptr;
     bool use_graph = true;
-    cudaGraphExec_t gexec = nullptr;   // one step: step start, colours, node pass
+    cudaGraphExec_t gexec = nullptr;   // one step: step start, element phase, node phase
+    cudaGraphExec_t gexec_n = nullptr; // kGraphSteps steps
     gfb::Layer* layer = nullptr;       // learned absorbing layer (or none)
     long long graph_launches = 0;
     void* ring = nullptr;              // device snapshot ring [slots]
@@ -352,6 +353,13 @@ struct gfb_solver {
     void *npml_coef = nullptr, *npml_mem = nullptr, *npml_prev = nullptr;
     long long device_bytes = 0, upload_bytes = 0, launches = 0;
 
+    // the captured steps, which hold launch arguments that have changed
+    void drop_graphs() {
+        if (gexec) cudaGraphExecDestroy(gexec);
+        if (gexec_n) cudaGraphExecDestroy(gexec_n);
+        gexec = gexec_n = nullptr;
+    }
+
     template <typename T>
     gfb_status alloc(T** out, size_t count) {
         auto b = std::make_unique<DevBuf>();
@@ -366,7 +374,7 @@ struct gfb_solver {
         return GFB_OK;
     }
     ~gfb_solver() {
-        if (gexec) cudaGraphExecDestroy(gexec);
+        drop_graphs();
         if (layer) gfb::layer_free(layer);
         for (auto e : rec_evt) cudaEventDestroy(e);
         for (auto e : copy_evt) cudaEventDestroy(e);
@@ -513,6 +521,24 @@ struct StageClock {
 // ---------------------------------------------------------------------------
 // kernel dispatch
 // ---------------------------------------------------------------------------
+
+// Launch a kernel of the step's programmatic chain (gfb::pdl_wait); early:
+// it may start before the kernel before it has completed.
+template <typename... Params, typename... Args>
+cudaError_t launch_chained(bool early, void (*fn)(Params...), int blocks, int threads, size_t smem, cudaStream_t stream,
+                           Args&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, fn, Params(args)...);
+}
 
 // The gather kernel runs unless the fused node update,
 // GFB_FLAG_POINT_KERNEL or another FP32 variant asks for assembly by colour.
@@ -755,8 +781,7 @@ gfb_status launch_gather_t(gfb_solver* s) {
             A.nfld_item = 2 * pairs <= s->plane_blocks * PS::WARPS ? 3 : s->nfld;
             const int n = pairs * (s->nfld / A.nfld_item);
             const int blocks = std::max(1, std::min((n + PS::WARPS - 1) / PS::WARPS, s->plane_blocks));
-            gfb::elem_plane_kernel<<<blocks, PS::THREADS, PS::SMEM, s->stream>>>(A);
-            CU(cudaGetLastError());
+            CU(launch_chained(true, gfb::elem_plane_kernel, blocks, PS::THREADS, PS::SMEM, s->stream, A));
             s->launches++;
             return GFB_OK;
         }
@@ -765,9 +790,8 @@ gfb_status launch_gather_t(gfb_solver* s) {
     A.nfld_item = 2 * groups <= s->gather_blocks * S::GROUPS ? 1 : s->nfld;
     const int items = groups * (s->nfld / A.nfld_item);
     const int blocks = std::max(1, std::min((items + S::GROUPS - 1) / S::GROUPS, s->gather_blocks));
-    if (pml) gfb::elem_gather_kernel<Real, NG, true><<<blocks, S::THREADS, S::SMEM, s->stream>>>(A);
-    else gfb::elem_gather_kernel<Real, NG, false><<<blocks, S::THREADS, S::SMEM, s->stream>>>(A);
-    CU(cudaGetLastError());
+    CU(launch_chained(true, pml ? gfb::elem_gather_kernel<Real, NG, true> : gfb::elem_gather_kernel<Real, NG, false>, blocks,
+                      S::THREADS, S::SMEM, s->stream, A));
     s->launches++;
     return GFB_OK;
 }
@@ -997,21 +1021,27 @@ gfb_status launch_node_m(gfb_solver* s) {
     node_args(s, A, P);
     // node-form C-PML nodes are device nodes [0, n_pml_node)
     const long long g0 = s->node_pml ? s->n_pml_node : 0;
-    if (g0 < s->n_node) {
-        const int grid = node_grid(s->n_node - g0, gfb::node_blocks_per_sm<Real>(false));
-        bool done = false;
+    const bool plain = g0 < s->n_node;
+    if (plain) {
+        auto* fn = gfb::node_update_kernel<Real, NFLD, MULTI, false>;
         if constexpr (std::is_same<Real, float>::value)
-            if ((done = A.half_v))
-                gfb::node_update_kernel<Real, NFLD, MULTI, true><<<grid, gfb::kNodeThreads, 0, s->stream>>>(A, P, g0);
-        if (!done) gfb::node_update_kernel<Real, NFLD, MULTI, false><<<grid, gfb::kNodeThreads, 0, s->stream>>>(A, P, g0);
-        CU(cudaGetLastError());
+            if (A.half_v) fn = gfb::node_update_kernel<Real, NFLD, MULTI, true>;
+        // Starting early the pass finds the SM set up for the element kernel:
+        // most of the L1 as shared memory.  Where that is 200 KB and more
+        // (line kernel at ngll 5 and 6, FP64) the pass then misses the L1 it
+        // reads its contributions through: 498 against 480 us per step (FP64,
+        // 40 x 40 x 20), 187 / 177 (ngll 6, 22 x 21 x 13).  Beside the plane
+        // kernel and at ngll 3 it gains: 400 / 405 (40 x 40 x 20 x 3), 68 / 72
+        // (20 x 20 x 10 x 3), 72 / 81 (six small models), 69.5 / 72.5 (ngll 3).
+        const bool early = use_gather(s) && s->prec == GFB_FP32 && (s->plane_blocks > 0 || s->ng == 3);
+        CU(launch_chained(early, fn, node_grid(s->n_node - g0, gfb::node_blocks_per_sm<Real>(false)), gfb::kNodeThreads, 0,
+                          s->stream, A, P, g0));
         s->launches++;
     }
     if constexpr (std::is_same<Real, float>::value) {
         if (g0 > 0) {
-            const int gp = node_grid(g0, gfb::node_blocks_per_sm<float>(true));
-            gfb::node_pml_kernel<NFLD, MULTI><<<gp, gfb::kNodeThreads, 0, s->stream>>>(A, P);
-            CU(cudaGetLastError());
+            CU(launch_chained(true, gfb::node_pml_kernel<NFLD, MULTI>, node_grid(g0, gfb::node_blocks_per_sm<float>(true)),
+                              gfb::kNodeThreads, 0, s->stream, A, P, !plain));
             s->launches++;
         }
     }
@@ -1115,10 +1145,7 @@ gfb_status leave_half_v(gfb_solver* s) {
     CU(cudaStreamSynchronize(s->stream));
     s->half_v = false;
     s->hv_begin = s->n_node;
-    if (s->gexec) {
-        cudaGraphExecDestroy(s->gexec);
-        s->gexec = nullptr;
-    }
+    s->drop_graphs();
     return GFB_OK;
 }
 
@@ -1846,19 +1873,16 @@ template <typename Real>
 gfb_status launch_step_begin_t(gfb_solver* s) {
     const int threads = 128;
     const int blocks = (s->n_model + threads - 1) / threads;
-    gfb::step_begin_kernel<Real><<<blocks, threads, 0, s->stream>>>(
-        s->n_model, s->n_set, s->d_mstep, s->d_nsteps, s->d_nstf, s->d_stf_off, static_cast<const Real*>(s->d_stf_all),
+    CU(launch_chained(
+        true, gfb::step_begin_kernel<Real>, blocks, threads, 0, s->stream, s->n_model, s->n_set, s->d_mstep, s->d_nsteps, s->d_nstf, s->d_stf_off, static_cast<const Real*>(s->d_stf_all),
         static_cast<Real*>(s->d_mstf), s->d_mlive, s->refresh, s->d_force_direct,
-        s->refresh > 1 ? s->d_mdirect : nullptr, s->d_mnext);
-    CU(cudaGetLastError());
+        s->refresh > 1 ? s->d_mdirect : nullptr, s->d_mnext));
     s->launches++;
     if (s->d_live_cell_end) {
         const int nc = (int)s->colour_begin.size();  // the colours, then all cells in mesh order
-        gfb::live_bounds_kernel<<<1, 128, 0, s->stream>>>(s->n_model, nc, s->d_mlive, s->d_cell_end,
-                                                          s->d_colour_first, s->d_node_end,
-                                                          s->node_pml ? (long long)s->n_pml_node : 0LL,
-                                                          s->d_live_cell_end, s->d_live_node_end);
-        CU(cudaGetLastError());
+        CU(launch_chained(true, gfb::live_bounds_kernel, 1, 128, 0, s->stream, s->n_model, nc, s->d_mlive, s->d_cell_end,
+                          s->d_colour_first, s->d_node_end, s->node_pml ? (long long)s->n_pml_node : 0LL,
+                          s->d_live_cell_end, s->d_live_node_end));
         s->launches++;
     }
     return GFB_OK;
@@ -1881,41 +1905,68 @@ gfb_status step_body(gfb_solver* s, cudaEvent_t* ev) {
     return GFB_OK;
 }
 
-// Capture step_body once as a CUDA graph; every argument it launches with
-// (device pointers, colour ranges, grid sizes) is fixed for the solver's
-// lifetime, and the step-dependent values live on the device.
-gfb_status capture_step(gfb_solver* s) {
+// Steps of one multi-step graph: between graphs the GPU idles for a couple of
+// microseconds and the programmatic chain is cut.
+constexpr int kGraphSteps = 5;
+
+// Capture n steps of step_body as a CUDA graph; every argument it launches
+// with (device pointers, colour ranges, grid sizes) is fixed until
+// drop_graphs(), and the step-dependent values live on the device.
+gfb_status capture_steps(gfb_solver* s, int n, cudaGraphExec_t* exec) {
     const long long l0 = s->launches;
     CU(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    gfb_status st = step_body(s, nullptr);
+    gfb_status st = GFB_OK;
+    for (int k = 0; k < n && !st; ++k) st = step_body(s, nullptr);
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(s->stream, &g);
+    s->graph_launches = (s->launches - l0) / n;
+    s->launches = l0;
     if (st) {
         if (g) cudaGraphDestroy(g);
         return st;
     }
     if (e != cudaSuccess) return fail(GFB_ERR_CUDA, "step capture failed: %s", cudaGetErrorString(e));
-    const cudaError_t ei = cudaGraphInstantiate(&s->gexec, g, 0);
+    const cudaError_t ei = cudaGraphInstantiate(exec, g, 0);
     cudaGraphDestroy(g);
-    if (ei != cudaSuccess) return fail(GFB_ERR_CUDA, "step graph instantiation failed: %s", cudaGetErrorString(ei));
-    s->graph_launches = s->launches - l0;
-    s->launches = l0;
+    if (ei != cudaSuccess) {
+        *exec = nullptr;
+        return fail(GFB_ERR_CUDA, "step graph instantiation failed: %s", cudaGetErrorString(ei));
+    }
     return GFB_OK;
 }
 
-// One solver step: the device work (a graph launch, or eager launches when
-// phases are timed), then the snapshot when the step is a snapshot step.
-gfb_status one_step(gfb_solver* s, cudaEvent_t* ev) {
+// The device work of n steps before the next snapshot: replayed graphs.
+gfb_status replay_steps(gfb_solver* s, int n) {
     gfb_status st;
-    const int step = s->step;
-    if (!ev && s->use_graph) {
-        if (!s->gexec && (st = capture_step(s))) return st;
-        CU(cudaGraphLaunch(s->gexec, s->stream));
-        s->launches += s->graph_launches;
-    } else if ((st = step_body(s, ev))) {
-        return st;
+    while (n > 0) {
+        const bool many = n >= kGraphSteps;
+        cudaGraphExec_t* exec = many ? &s->gexec_n : &s->gexec;
+        const int k = many ? kGraphSteps : 1;
+        if (!*exec && (st = capture_steps(s, k, exec))) return st;
+        CU(cudaGraphLaunch(*exec, s->stream));
+        s->launches += s->graph_launches * k;
+        n -= k;
     }
-    if (s->stride > 0 && s->n_rec > 0 && step % s->stride == 0) {
+    return GFB_OK;
+}
+
+// Up to n solver steps: their device work (graph launches, or eager launches
+// when phases are timed), up to and with the next snapshot step, then that
+// snapshot.  *done: the steps taken.
+gfb_status some_steps(gfb_solver* s, int n, cudaEvent_t* ev, int* done) {
+    gfb_status st;
+    const bool records = s->stride > 0 && s->n_rec > 0;
+    if (!ev && s->use_graph) {
+        // steps up to the next snapshot step (step % stride == 0)
+        const int to_snap = records ? (s->stride - s->step % s->stride) % s->stride + 1 : n;
+        n = std::min(n, to_snap);
+        if ((st = replay_steps(s, n))) return st;
+    } else {
+        n = 1;
+        if ((st = step_body(s, ev))) return st;
+    }
+    const int step = s->step + n - 1;  // the last one
+    if (records && step % s->stride == 0) {
         // round-robin slot; an unread snapshot still in it moves to pageable
         // memory first.  The record kernel waits (on the GPU) for the last
         // device->host copy out of the slot; the copy of this snapshot runs
@@ -1976,9 +2027,16 @@ gfb_status one_step(gfb_solver* s, cudaEvent_t* ev) {
         s->pending.push_back(std::move(snap));
     }
     if (ev) CU(cudaEventRecord(ev[3], s->stream));
-    s->step++;
+    s->step += n;
     s->a_in_force = true;
+    *done = n;
     return GFB_OK;
+}
+
+gfb_status all_steps(gfb_solver* s, int n) {
+    gfb_status st = GFB_OK;
+    for (int done = 0; n > 0 && !st; n -= done) st = some_steps(s, n, nullptr, &done);
+    return st;
 }
 
 }  // namespace
@@ -2385,11 +2443,7 @@ gfb_status gfb_advance(gfb_solver* s, int32_t n_steps) {
     if (!s) return fail(GFB_ERR_INVALID, "solver is NULL");
     if (n_steps < 0) return fail(GFB_ERR_INVALID, "n_steps must be >= 0");
     CU(cudaSetDevice(s->device));
-    for (int it = 0; it < n_steps; ++it) {
-        gfb_status st = one_step(s, nullptr);
-        if (st) return st;
-    }
-    return GFB_OK;
+    return all_steps(s, n_steps);
 }
 
 gfb_status gfb_advance_timed(gfb_solver* s, int32_t n_steps, double* ms) {
@@ -2404,7 +2458,7 @@ gfb_status gfb_advance_timed(gfb_solver* s, int32_t n_steps, double* ms) {
     }
     gfb_status st = GFB_OK;
     if (cudaEventRecord(e0, s->stream) != cudaSuccess) st = fail(GFB_ERR_CUDA, "cudaEventRecord failed");
-    for (int it = 0; it < n_steps && !st; ++it) st = one_step(s, nullptr);
+    if (!st) st = all_steps(s, n_steps);
     float t = 0.0f;
     if (!st && (cudaEventRecord(e1, s->stream) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
                 cudaEventElapsedTime(&t, e0, e1) != cudaSuccess))
@@ -2428,7 +2482,7 @@ gfb_status gfb_advance_profiled(gfb_solver* s, int32_t n_steps, double* ms_eleme
             break;
         }
     }
-    for (int it = 0; it < n_steps && !st; ++it) st = one_step(s, ev.data() + (size_t)it * 4);
+    for (int it = 0, done = 0; it < n_steps && !st; ++it) st = some_steps(s, 1, ev.data() + (size_t)it * 4, &done);
     double acc[3] = {0, 0, 0};
     if (!st && n_steps > 0) {
         if (cudaEventSynchronize(ev.back()) != cudaSuccess) st = fail(GFB_ERR_CUDA, "event synchronize failed");
@@ -2491,10 +2545,7 @@ gfb_status gfb_set_force_refresh(gfb_solver* s, int32_t steps) {
     // the next step evaluates the force in full (from a period of 1 the
     // stored force is this step's, but the next step must not add to it)
     if (steps > 1) CU(cudaMemsetAsync(s->d_force_direct, 1, (size_t)s->n_model * sizeof(int), s->stream));
-    if (s->gexec) {
-        cudaGraphExecDestroy(s->gexec);
-        s->gexec = nullptr;
-    }
+    s->drop_graphs();
     return GFB_OK;
 }
 
@@ -2512,10 +2563,7 @@ gfb_status gfb_select_element_kernel(gfb_solver* s, int32_t variant) {
     // the predicted displacement rewritten in full (between full
     // evaluations the node pass leaves its increment there)
     if (s->refresh > 1 && (st = launch_predict(s))) return st;
-    if (s->gexec) {
-        cudaGraphExecDestroy(s->gexec);
-        s->gexec = nullptr;
-    }
+    s->drop_graphs();
     return GFB_OK;
 }
 
@@ -3014,10 +3062,7 @@ gfb_status solver_set_layer(gfb_solver* s, Layer* layer) {
         if (st) return st;
     }
     // the captured step graph does not contain the layer's launch
-    if (s->gexec) {
-        cudaGraphExecDestroy(s->gexec);
-        s->gexec = nullptr;
-    }
+    s->drop_graphs();
     return GFB_OK;
 }
 
