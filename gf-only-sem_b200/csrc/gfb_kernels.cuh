@@ -5,10 +5,12 @@
 //   elem_gather_kernel -- for every cell: gather the predicted displacement
 //       through ibool, GLL derivative contractions, stress, weighted
 //       transposed-derivative divergence (forward/elastic/src/
-//       element_cpu.cpp:19-162), C-PML acceleration term and memory update on
-//       C-PML cells (forward/share/src/pml.cpp:55-216; per-cell form), point-
-//       force injection (forward/share/src/solver.cpp:577-605).  The cell's
-//       force contributions are stored cell by cell.
+//       element_cpu.cpp:19-162), point-force injection (forward/share/src/
+//       solver.cpp:577-605).  The cell's force contributions are stored cell
+//       by cell.  elem_plane_kernel: the same for wavefields in threes.
+//   cell_pml_kernel -- per-cell C-PML (FP64, or FP32 where cells disagree):
+//       acceleration term and memory update (forward/share/src/
+//       pml.cpp:55-216).
 //   node_update_kernel, node_pml_kernel -- sum of the contributions of a
 //       node's cells in mesh order (no atomics, bit-reproducible run to run),
 //       node-form C-PML, Newmark corrector with the diagonal mass and the
@@ -1667,7 +1669,7 @@ struct GatherShape : GatherPad<NG, sizeof(Real) == 8> {
     static_assert(!OUT_IN_XCH || CHUNK_MAX_B <= 3 * Pad::SE * (int)sizeof(Real), "a chunk fits in the eta array");
     static constexpr int GROUP_B = CELLS * GEO_SLOT + XCH_B + (OUT_IN_XCH ? 0 : CELLS * CHUNK_MAX_B);
     static constexpr int SMEM = GROUPS * GROUP_B;
-    // registers: 104 a thread in FP32, 168 in FP64
+    // at most 128 registers a thread in FP32, 168 in FP64
     static constexpr int MIN_BLOCKS = (sizeof(Real) == 4 ? 608 : 384) / THREADS;
 };
 
@@ -1692,65 +1694,110 @@ struct GatherArgs {
     int n_set;
     int dir[kMaxFields];
     int fset[kMaxFields];
-    // C-PML per cell
-    const int* pml_slot;           // [cell] -1 if not a C-PML cell
-    const Real* pml_coef;          // [slot][15][NN]
-    Real* pml_mem;                 // [slot][9*nfld][NN]
-    Real* pml_prev;                // [slot][3*nfld][NN]
-    const double* u;               // [node][3*nfld]
-    const double* v;
-    const Real* a;
-    const ModelConst* mc;          // [model]
     unsigned* err;                 // set to 1 when a bulk copy's wait gave up (the launch did not finish)
     Real D[36];                    // D[i*NG+s], read with compile-time indices only
     float2 D2[36];                 // the same twice, for packed operations (FP32)
 };
 
-// C-PML of one wavefield at the points of this thread's line (pml.cpp:55-216):
-// the term with last step's memory added to r, then the memory update, which
-// only uses values fixed at the start of the step.
+// C-PML per cell (pml.cpp:55-216), after the element kernel: the term with
+// last step's memory is added to the cells' contributions, and the memory
+// moves on, which only uses values fixed at the start of the step.  A block
+// takes a C-PML cell at a time, one thread per (component, point); the arrays
+// are streams of whole rows.  An axis
+// that is live nowhere in a cell (its A_k are 0 there) has a memory nothing
+// reads: it is neither loaded nor updated, which is more than half of the
+// traffic in the one-axis cells that most C-PML cells are.  Inside the element
+// kernel, with 12 warps per SM and every axis, the same work took 220 us on
+// 40 x 40 x 20 cells (15,600 of them C-PML, FP64, one wavefield).
+template <typename Real>
+struct CellPmlArgs {
+    int n_slot;
+    const int2* cell;              // [slot] cell, live axes (bits 0..2)
+    const uint32_t* ibool_padded;
+    Real* contrib;
+    int nfld;
+    const int* mlive;
+    bool multi;                    // several models
+    bool early;                    // launched before the element kernel has completed
+    const Real* coef;              // [slot][15][NN]
+    Real* mem;                     // [slot][9*nfld][NN]
+    Real* prev;                    // [slot][3*nfld][NN]
+    const double* u;               // [node][3*nfld]
+    const double* v;
+    const Real* a;
+    const ModelConst* mc;          // [model]
+};
+
+constexpr int cell_pml_threads(int nn) { return (3 * nn + 31) / 32 * 32; }
+// Threads per SM, for 80 registers: with 1280 (56 registers, spills) the pass
+// takes 164 us on the mesh above, with 768 about 139 (575 MB of DRAM traffic).
+constexpr int kCellPmlThreads = 768;
+
 template <typename Real, int NG>
-__device__ __forceinline__ void line_cell_pml(const GatherArgs<Real>& A, int slot, int mdl, int d, int col,
-                                              const uint32_t (&w)[NG], Real (&r)[3][NG]) {
-    constexpr int NN = NG * NG * NG, NG2 = NG * NG;
-    const double k1 = A.mc[mdl].c1;
-    const Real k2 = (Real)A.mc[mdl].c2;
-    const int F = 3 * A.nfld;
+__global__ void __launch_bounds__(cell_pml_threads(NG * NG * NG), kCellPmlThreads / cell_pml_threads(NG * NG * NG))
+    cell_pml_kernel(const __grid_constant__ CellPmlArgs<Real> A) {
+    constexpr int NN = NG * NG * NG;
+    const int F = 3 * A.nfld, fc = gather_chunk_fields<Real>(A.nfld);
+    const int chunk_u = gather_chunk_units<Real>(NN, A.nfld);
+    const int c = threadIdx.x / NN, p = threadIdx.x - c * NN;
+    // only the contributions come from the element kernel: with one cell per
+    // block all else is done while it runs
+    if (!A.early) pdl_wait();
+    pdl_launch();
+    const int step = gridDim.x;
+    auto cell_at = [&](int slot) { return slot < A.n_slot ? __ldg(A.cell + slot) : make_int2(0, 0); };
+    auto node_at = [&](int cell) { return c < 3 ? __ldg(A.ibool_padded + (size_t)cell * ib_row_words(NN) + p) & kNodeMask : 0u; };
+    int2 ce = cell_at(blockIdx.x);
+    uint32_t g = node_at(ce.x);
+    for (int slot = blockIdx.x; slot < A.n_slot; slot += step) {
+        // the next cell's index and nodes are on their way during this one
+        const int2 ce1 = cell_at(slot + step);
+        const int mdl = A.multi ? (int)__ldg(A.ibool_padded + (size_t)ce.x * ib_row_words(NN) + NN) : 0;
+        if (c < 3 && __ldcg(A.mlive + mdl)) {
+            const size_t at = (size_t)g * F + c;
+            const Real* cf = A.coef + (size_t)slot * 15 * NN + p;
+            const Real scale = __ldg(cf + 14 * NN), b0 = __ldg(cf + 9 * NN), b1 = __ldg(cf + 10 * NN);
+            Real bq[3], al[3][3];
 #pragma unroll
-    for (int i = 0; i < NG; ++i) {
-        const int p = i * NG2 + col;
-        const Real* cf = A.pml_coef + (size_t)slot * 15 * NN + p;
-        Real* mem = A.pml_mem + ((size_t)slot * 3 * F + 9 * d) * NN + p;
-        Real* prev = A.pml_prev + ((size_t)slot * F + 3 * d) * NN + p;
-        const size_t at = (size_t)(w[i] & kNodeMask) * F + 3 * d;
-        Real al[9], ab[5], m[9], pr[3], an[3];
-        double un[3], vn[3];
+            for (int q = 0; q < 3; ++q) {
+                const bool live = ce.y >> q & 1;
+                bq[q] = live ? __ldg(cf + (11 + q) * NN) : Real(0);
 #pragma unroll
-        for (int q = 0; q < 9; ++q) al[q] = __ldg(cf + q * NN);
+                for (int x = 0; x < 3; ++x) al[q][x] = live ? __ldg(cf + (3 * q + x) * NN) : Real(0);
+            }
+            const double k1 = A.mc[mdl].c1;
+            const Real k2 = (Real)A.mc[mdl].c2;
+            for (int d = 0; d < A.nfld; ++d) {
+                Real* mem = A.mem + ((size_t)slot * 3 * F + 9 * d + 3 * c) * NN + p;
+                Real* prev = A.prev + ((size_t)slot * F + 3 * d + c) * NN + p;
+                Real* out = A.contrib + ((size_t)ce.x * (A.nfld / fc) * chunk_u + (size_t)(d / fc) * chunk_u + p * fc + d % fc) * 3 + c;
+                const Real pr = *prev, an = A.a[at + 3 * d];
+                const double un = A.u[at + 3 * d], vn = A.v[at + 3 * d];
+                Real m[3];
 #pragma unroll
-        for (int q = 0; q < 5; ++q) ab[q] = __ldg(cf + (9 + q) * NN);
-        const Real scale = __ldg(cf + 14 * NN);
+                for (int q = 0; q < 3; ++q) m[q] = ce.y >> q & 1 ? mem[q * NN] : Real(0);
+                const Real old = A.early ? Real(0) : *out;
+                const Real nv = Real(un + k1 * vn), ov = pr + k2 * an;
+                Real r = b0 * Real(vn) + b1 * Real(un);
 #pragma unroll
-        for (int q = 0; q < 9; ++q) m[q] = mem[q * NN];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            pr[c] = prev[c * NN];
-            un[c] = A.u[at + c];
-            vn[c] = A.v[at + c];
-            an[c] = A.a[at + c];
+                for (int q = 0; q < 3; ++q)
+                    if (ce.y >> q & 1) {
+                        r += bq[q] * m[q];
+                        mem[q * NN] = al[q][0] * m[q] + al[q][1] * nv + al[q][2] * ov;
+                    }
+                *prev = nv;
+                if (A.early) {
+                    pdl_wait();
+                    *out += scale * r;
+                } else {
+                    *out = old + scale * r;
+                }
+            }
         }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const Real nv = Real(un[c] + k1 * vn[c]);
-            const Real ov = pr[c] + k2 * an[c];
-            r[c][i] += scale * (ab[0] * Real(vn[c]) + ab[1] * Real(un[c]) + ab[2] * m[3 * c] + ab[3] * m[3 * c + 1] +
-                                ab[4] * m[3 * c + 2]);
-#pragma unroll
-            for (int q = 0; q < 3; ++q)
-                mem[(3 * c + q) * NN] = al[3 * q] * m[3 * c + q] + al[3 * q + 1] * nv + al[3 * q + 2] * ov;
-            prev[c * NN] = nv;
-        }
+        ce = ce1;
+        g = node_at(ce.x);
     }
+    if (A.early) pdl_wait();
 }
 
 // Packed pairs of FP32 operations (one instruction for two, sm_100) beside the
@@ -1804,7 +1851,7 @@ __device__ __forceinline__ void point_fluxes(const Real* geo, int nn, int step, 
             fl[b][c] = vfma(st[c][2], dd[6 + b], vfma(st[c][1], dd[3 + b], vmul(st[c][0], dd[b])));
 }
 
-template <typename Real, int NG, bool PML>
+template <typename Real, int NG>
 __global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Real, NG>::MIN_BLOCKS)
     elem_gather_kernel(const __grid_constant__ GatherArgs<Real> A) {
     using S = GatherShape<Real, NG>;
@@ -1880,7 +1927,7 @@ __global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Re
         }
     };
 
-    uint32_t cw[NG], nw[NG], nw2[NG];  // node words: this item's (C-PML), the next one's, the one's after
+    uint32_t nw[NG], nw2[NG];  // node words: the next item's, the one's after
     Real pre[3][NG];                   // displacement of the wavefield to come
     load_words(first, nw);
     load_words(first + step, nw2);
@@ -1894,12 +1941,8 @@ __global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Re
         const int mdl = A.multi && e >= 0 ? (int)__ldg(A.ibool_padded + (size_t)e * IB_W + NN) : 0;
         const bool act = e >= 0 && __ldcg(A.mlive + mdl) != 0;
         const int src0 = act && A.src_head ? __ldg(A.src_head + e) : -1;
-        const int slot = PML && act ? __ldg(A.pml_slot + e) : -1;
 #pragma unroll
-        for (int i = 0; i < NG; ++i) {
-            if (PML) cw[i] = nw[i];
-            nw[i] = nw2[i];
-        }
+        for (int i = 0; i < NG; ++i) nw[i] = nw2[i];
         load_words(next + step, nw2);
         if (any(!mbar_wait(bar, phase))) {
             // the copy never came: flag it, give it a second bounded wait, leave
@@ -1925,14 +1968,9 @@ __global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Re
                 }
             sync();
             if (d + 1 < d1) {
-                // the same cells' next wavefield: the words are PML's cw or read again
-                if constexpr (PML) {
-                    load_vectors(cw, e >= 0, d + 1, pre);
-                } else {
-                    uint32_t w[NG];
-                    load_words(item, w);
-                    load_vectors(w, e >= 0, d + 1, pre);
-                }
+                uint32_t w[NG];
+                load_words(item, w);
+                load_vectors(w, e >= 0, d + 1, pre);
             } else {
                 load_vectors(nw, cell_of(next) >= 0, next % split * A.nfld_item, pre);
             }
@@ -2036,8 +2074,6 @@ __global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Re
                     x += xz[c * CELLS * SZ + own_z + i * PZ];
                     r[c][i] = -x;
                 }
-            if constexpr (PML)
-                if (slot >= 0) line_cell_pml<Real, NG>(A, slot, mdl, d, col, cw, r);
             // point force (solver.cpp:577-605)
             if (src0 >= 0 && A.mstf) {
                 const int fs = A.fset[d], dir = A.dir[d];

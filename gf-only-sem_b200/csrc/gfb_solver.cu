@@ -264,6 +264,7 @@ struct gfb_solver {
     uint4* touch = nullptr;         // [node] (gfb::NodeGather)
     uint4* touch_more = nullptr;
     int gather_blocks = 0;          // persistent grid of the gather kernel
+    int gather_sm = 0;              // multiprocessors
     int plane_blocks = 0;           // of the plane kernel (0: not used)
     bool has_cpml = false, has_damping = false, has_src = false;
     int n_pml = 0, n_src = 0, n_rec = 0, slots = 0;
@@ -287,6 +288,7 @@ struct gfb_solver {
     void* inv_mass = nullptr;
     double* damping = nullptr;
     int* pml_slot = nullptr;
+    int2* pml_cell = nullptr;          // [slot] cell, axes that are live in it
     void *pml_coef = nullptr, *pml_mem = nullptr, *pml_prev = nullptr;
     int *src_head = nullptr, *src_next = nullptr;
     void* src_w = nullptr;
@@ -521,6 +523,11 @@ struct StageClock {
 // ---------------------------------------------------------------------------
 // kernel dispatch
 // ---------------------------------------------------------------------------
+
+int grid_for(long long n, int threads) {
+    long long b = (n + threads - 1) / threads;
+    return (int)std::max(1LL, std::min(b, 148LL * 32));
+}
 
 // Launch a kernel of the step's programmatic chain (gfb::pdl_wait); early:
 // it may start before the kernel before it has completed.
@@ -757,15 +764,6 @@ gfb_status launch_gather_t(gfb_solver* s) {
         A.dir[d] = s->dirs[d];
         A.fset[d] = s->fset[d];
     }
-    const bool pml = s->has_cpml && !s->node_pml;
-    A.pml_slot = s->pml_slot;
-    A.pml_coef = static_cast<const Real*>(s->pml_coef);
-    A.pml_mem = static_cast<Real*>(s->pml_mem);
-    A.pml_prev = static_cast<Real*>(s->pml_prev);
-    A.u = s->u;
-    A.v = s->v;
-    A.a = static_cast<const Real*>(s->a);
-    A.mc = s->d_mc;
     A.err = reinterpret_cast<unsigned*>(s->d_kernel_err);
     for (int q = 0; q < 36; ++q) A.D[q] = q < NG * NG ? (Real)s->dmat_host[q] : Real(0);
     for (int q = 0; q < 36; ++q) A.D2[q] = make_float2((float)A.D[q], (float)A.D[q]);
@@ -790,9 +788,34 @@ gfb_status launch_gather_t(gfb_solver* s) {
     A.nfld_item = 2 * groups <= s->gather_blocks * S::GROUPS ? 1 : s->nfld;
     const int items = groups * (s->nfld / A.nfld_item);
     const int blocks = std::max(1, std::min((items + S::GROUPS - 1) / S::GROUPS, s->gather_blocks));
-    CU(launch_chained(true, pml ? gfb::elem_gather_kernel<Real, NG, true> : gfb::elem_gather_kernel<Real, NG, false>, blocks,
-                      S::THREADS, S::SMEM, s->stream, A));
+    CU(launch_chained(true, gfb::elem_gather_kernel<Real, NG>, blocks, S::THREADS, S::SMEM, s->stream, A));
     s->launches++;
+    if (s->has_cpml && !s->node_pml && s->n_pml > 0) {
+        gfb::CellPmlArgs<Real> P;
+        P.n_slot = s->n_pml;
+        P.cell = s->pml_cell;
+        P.ibool_padded = s->ibool_padded;
+        P.contrib = static_cast<Real*>(s->contrib);
+        P.nfld = s->nfld;
+        P.mlive = s->d_mlive;
+        P.coef = static_cast<const Real*>(s->pml_coef);
+        P.mem = static_cast<Real*>(s->pml_mem);
+        P.prev = static_cast<Real*>(s->pml_prev);
+        P.u = s->u;
+        P.v = s->v;
+        P.a = static_cast<const Real*>(s->a);
+        P.mc = s->d_mc;
+        // early beside an element kernel that leaves room on the SMs: 18.4
+        // against 20.8 us per step (11 x 9 x 7 cells); otherwise it would run
+        // with the little L1 the element kernel leaves (486 / 391 us,
+        // 40 x 40 x 20)
+        constexpr int threads = gfb::cell_pml_threads(S::NN);
+        const int cells = std::min(s->n_pml, s->gather_sm * (gfb::kCellPmlThreads / threads));
+        P.multi = s->n_model > 1;
+        P.early = 2 * blocks <= s->gather_blocks;
+        CU(launch_chained(P.early, gfb::cell_pml_kernel<Real, NG>, cells, threads, 0, s->stream, P));
+        s->launches++;
+    }
     return GFB_OK;
 }
 
@@ -800,14 +823,14 @@ gfb_status launch_gather_t(gfb_solver* s) {
 template <typename Real, int NG>
 gfb_status gather_grid_t(gfb_solver* s) {
     using S = gfb::GatherShape<Real, NG>;
-    auto* fn = s->has_cpml && !s->node_pml ? gfb::elem_gather_kernel<Real, NG, true>
-                                           : gfb::elem_gather_kernel<Real, NG, false>;
+    auto* fn = gfb::elem_gather_kernel<Real, NG>;
     CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
     int per_sm = 0, n_sm = 0;
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, S::THREADS, S::SMEM));
     CU(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, s->device));
     if (per_sm < 1) return fail(GFB_ERR_UNSUPPORTED, "gather element kernel does not fit on an SM");
     s->gather_blocks = per_sm * n_sm;
+    s->gather_sm = n_sm;
     if constexpr (std::is_same<Real, float>::value && NG == 5) {
         if (s->nfld % 3 == 0 && !(s->has_cpml && !s->node_pml)) {
             using PS = gfb::PlaneShape;
@@ -1003,10 +1026,6 @@ gfb_status launch_record(gfb_solver* s, void* out) {
     return dispatch<float, RecOp>(s->ng, s->nfld, s, out);
 }
 
-int grid_for(long long n, int threads) {
-    long long b = (n + threads - 1) / threads;
-    return (int)std::max(1LL, std::min(b, 148LL * 32));
-}
 
 // Blocks of a node pass over n nodes: resident ones, looping over tiles.
 int node_grid(long long n, int per_sm) {
@@ -1642,6 +1661,21 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
             if ((st = s->alloc(&d, slot.size()))) return st;
             if ((st = h2d(s, d, slot.data(), slot.size() * 4))) return st;
             s->pml_slot = d;
+        }
+        {
+            std::vector<int2> cells(s->n_pml);
+            parallel_for(s->n_pml, [&](long long s0, long long s1) {
+                for (long long i = s0; i < s1; ++i) {
+                    const double* A = m->pml_coef_abar + (size_t)slot_cell[i] * nn * 5;
+                    int live = 0;
+                    for (int p = 0; p < nn; ++p)
+                        for (int q = 0; q < 3; ++q)
+                            if (A[p * 5 + 2 + q] != 0.0) live |= 1 << q;
+                    cells[i] = int2{(int)slot_cell[i], live};
+                }
+            }, 256);
+            if ((st = s->alloc(&s->pml_cell, cells.size()))) return st;
+            if ((st = h2d(s, s->pml_cell, cells.data(), cells.size() * sizeof(int2)))) return st;
         }
         Real* dcoef = nullptr;
         if ((st = s->alloc(&dcoef, (size_t)s->n_pml * 15 * nn))) return st;
