@@ -22,8 +22,7 @@
 // one launch per colour with a plain read-modify-write of the global force:
 // cells of one colour share no node and colours run in a fixed order, and the
 // first colour touching a node stores instead of adding, which replaces the
-// memset of the global residual (cuda_step.cu:289-290).  elem_step_kernel
-// serves the residual of independent elements.
+// memset of the global residual (cuda_step.cu:289-290).
 //
 // Layouts on the device (cells in mesh order):
 //   ibool  [cell][NN]            node id | FIRST_TOUCH, LAST_TOUCH bits (by colour)
@@ -189,7 +188,7 @@ struct NodePml {
 
 template <typename Real>
 struct ElemArgs {
-    int e_begin, e_end;     // range of `cells` (elem_step_kernel: of the cells themselves)
+    int e_begin, e_end;     // range of `cells`
     const int* cells;       // the cells colour after colour
     const uint32_t* ibool;
     const Real* geom;
@@ -226,183 +225,6 @@ struct ElemArgs {
     NodeArgs<Real> nu;
     NodePml<Real> np;
 };
-
-template <typename Real, int NG, int NFLD>
-__device__ __forceinline__ void elem_body(const ElemArgs<Real>& A, Real* smem) {
-    using S = Shape<NG>;
-    constexpr int NN = S::NN, NNP = S::NNP, EPB = S::EPB, F = 3 * NFLD;
-    Real* sD = smem;                       // NG*NG, padded to 64
-    Real* su = smem + 64;                  // [EPB][F][NNP]
-    Real* sG = su + EPB * F * NNP;         // [EPB][3*F][NNP]
-    const int tid = threadIdx.x;
-    const int el = tid / NNP, p = tid - el * NNP;
-    const int e = A.e_begin + blockIdx.x * EPB + el;
-    const bool active = (p < NN) && (e < A.e_end);
-    if (tid < NG * NG) sD[tid] = A.dmat[tid];
-    Real* mu_s = su + el * F * NNP;
-    Real* mG = sG + el * 3 * F * NNP;
-
-    uint32_t gword = 0;
-    Real dd[9], jw = Real(0), lam = Real(0), mu = Real(0);
-    if (active) {
-        gword = __ldg(A.ibool + (size_t)e * NN + p);
-        const uint32_t g = gword & kNodeMask;
-        const Real* src = A.ut + (size_t)g * F;
-#pragma unroll
-        for (int f = 0; f < F; ++f) mu_s[f * NNP + p] = src[f];
-        const Real* gp = A.geom + (size_t)e * 12 * NN + p;
-#pragma unroll
-        for (int f = 0; f < 9; ++f) dd[f] = __ldg(gp + f * NN);
-        jw = __ldg(gp + 9 * NN);
-        lam = __ldg(gp + 10 * NN);
-        mu = __ldg(gp + 11 * NN);
-    }
-    __syncthreads();
-    const int i = p / (NG * NG), j = (p / NG) % NG, k = p % NG;
-    if (active) {
-#pragma unroll
-        for (int d = 0; d < NFLD; ++d) {
-            if (mu <= Real(0)) {  // element_cpu.cpp:42-43: the point adds nothing
-#pragma unroll
-                for (int q = 0; q < 9; ++q) mG[((q / 3) * F + d * 3 + (q % 3)) * NNP + p] = Real(0);
-                continue;
-            }
-            Real gx[3] = {0, 0, 0}, gy[3] = {0, 0, 0}, gz[3] = {0, 0, 0};
-#pragma unroll
-            for (int s = 0; s < NG; ++s) {
-                const Real Di = sD[i * NG + s], Dj = sD[j * NG + s], Dk = sD[k * NG + s];
-                const int pa = (s * NG + j) * NG + k, pb = (i * NG + s) * NG + k,
-                          pc = (i * NG + j) * NG + s;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const Real* uc = mu_s + (d * 3 + c) * NNP;
-                    gx[c] += Di * uc[pa];
-                    gy[c] += Dj * uc[pb];
-                    gz[c] += Dk * uc[pc];
-                }
-            }
-            // physical gradient with the reference's reading of dxi_dx
-            Real gr[3][3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                gr[c][0] = gx[c] * dd[0] + gy[c] * dd[1] + gz[c] * dd[2];
-                gr[c][1] = gx[c] * dd[3] + gy[c] * dd[4] + gz[c] * dd[5];
-                gr[c][2] = gx[c] * dd[6] + gy[c] * dd[7] + gz[c] * dd[8];
-            }
-            const Real exx = gr[0][0], eyy = gr[1][1], ezz = gr[2][2];
-            const Real exy = Real(0.5) * (gr[0][1] + gr[1][0]);
-            const Real exz = Real(0.5) * (gr[0][2] + gr[2][0]);
-            const Real eyz = Real(0.5) * (gr[1][2] + gr[2][1]);
-            const Real tr = exx + eyy + ezz;
-            const Real m2 = Real(2) * mu;
-            Real sg[3][3];
-            sg[0][0] = m2 * exx + lam * tr;
-            sg[1][1] = m2 * eyy + lam * tr;
-            sg[2][2] = m2 * ezz + lam * tr;
-            sg[0][1] = sg[1][0] = m2 * exy;
-            sg[0][2] = sg[2][0] = m2 * exz;
-            sg[1][2] = sg[2][1] = m2 * eyz;
-            // flux along reference axis a: jw * sigma . (dd[a], dd[3+a], dd[6+a])
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-                    mG[(a * F + d * 3 + c) * NNP + p] =
-                        jw * (sg[c][0] * dd[a] + sg[c][1] * dd[3 + a] + sg[c][2] * dd[6 + a]);
-            }
-        }
-    }
-    __syncthreads();
-    if (!active) return;
-
-    Real r[F];
-#pragma unroll
-    for (int f = 0; f < F; ++f) {
-        Real acc = Real(0);
-#pragma unroll
-        for (int s = 0; s < NG; ++s) {
-            acc += sD[s * NG + i] * mG[(0 * F + f) * NNP + (s * NG + j) * NG + k];
-            acc += sD[s * NG + j] * mG[(1 * F + f) * NNP + (i * NG + s) * NG + k];
-            acc += sD[s * NG + k] * mG[(2 * F + f) * NNP + (i * NG + j) * NG + s];
-        }
-        r[f] = -acc;
-    }
-    const uint32_t g = gword & kNodeMask;
-
-    // C-PML acceleration term with last step's memory, then the memory
-    // update that the reference performs after the corrector (it only uses
-    // values fixed at the start of the step).
-    const int slot = A.pml_slot ? __ldg(A.pml_slot + e) : -1;
-    if (slot >= 0) {
-        const Real* cf = A.pml_coef + (size_t)slot * 15 * NN + p;
-        Real al[9], ab[5];
-#pragma unroll
-        for (int q = 0; q < 9; ++q) al[q] = __ldg(cf + q * NN);
-#pragma unroll
-        for (int q = 0; q < 5; ++q) ab[q] = __ldg(cf + (9 + q) * NN);
-        const Real scale = __ldg(cf + 14 * NN);
-        Real* mem = A.pml_mem + (size_t)slot * (F * 3) * NN + p;
-        Real* prev = A.pml_prev + (size_t)slot * F * NN + p;
-#pragma unroll
-        for (int f = 0; f < F; ++f) {
-            const double un = A.u[(size_t)g * F + f];
-            const double vn = A.v[(size_t)g * F + f];
-            const Real an = A.a[(size_t)g * F + f];
-            const Real nv = Real(un + A.c1 * vn);
-            const Real ov = prev[f * NN] + Real(A.c2) * an;
-            Real m0 = mem[(f * 3 + 0) * NN], m1 = mem[(f * 3 + 1) * NN], m2 = mem[(f * 3 + 2) * NN];
-            r[f] += scale * (ab[0] * Real(vn) + ab[1] * Real(un) + ab[2] * m0 + ab[3] * m1 + ab[4] * m2);
-            m0 = al[0] * m0 + al[1] * nv + al[2] * ov;
-            m1 = al[3] * m1 + al[4] * nv + al[5] * ov;
-            m2 = al[6] * m2 + al[7] * nv + al[8] * ov;
-            mem[(f * 3 + 0) * NN] = m0;
-            mem[(f * 3 + 1) * NN] = m1;
-            mem[(f * 3 + 2) * NN] = m2;
-            prev[f * NN] = nv;
-        }
-    }
-    // point-force source (one model): wavefield d takes the slots of its
-    // source set, scaled by that set's source time function
-    if (A.mstf) {
-        int s = A.src_head ? __ldg(A.src_head + e) : -1;
-        while (s >= 0) {
-            const Real w = __ldg(A.src_w + (size_t)s * NN + p);
-            const int ks = A.src_set ? __ldg(A.src_set + s) : 0;
-            if (w != Real(0)) {
-#pragma unroll
-                for (int d = 0; d < NFLD; ++d) {
-                    const Real stf = A.mstf[A.fset[d]];
-                    if (stf == Real(0) || A.fset[d] != ks) continue;
-#pragma unroll
-                    for (int c = 0; c < 3; ++c)
-                        if (c == A.dir[d]) r[d * 3 + c] += stf * w;
-                }
-            }
-            s = __ldg(A.src_next + s);
-        }
-    }
-    // colour-ordered assembly: exclusive access to node g in this launch
-    Real* out = A.force + (size_t)g * F;
-    if (gword & kFirstTouch) {
-#pragma unroll
-        for (int f = 0; f < F; ++f) out[f] = r[f];
-    } else {
-#pragma unroll
-        for (int f = 0; f < F; ++f) out[f] += r[f];
-    }
-}
-
-template <typename Real, int NG, int NFLD>
-__global__ void __launch_bounds__(Shape<NG>::THREADS) elem_step_kernel(ElemArgs<Real> A) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    elem_body<Real, NG, NFLD>(A, reinterpret_cast<Real*>(smem_raw));
-}
-
-template <typename Real, int NG, int NFLD>
-constexpr size_t elem_smem_bytes() {
-    using S = Shape<NG>;
-    return sizeof(Real) * (64 + (size_t)S::EPB * 3 * NFLD * S::NNP * 4);
-}
 
 // 16-byte vector helpers (a float4, or two double2 for FP64 vectors).
 __device__ __forceinline__ void load4(const float* p, float (&v)[4]) {

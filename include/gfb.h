@@ -390,19 +390,12 @@ gfb_status gfb_element_residual(int32_t n_elem, const double* dxi_dx, const doub
  * Work is queued on `stream` (a cudaStream_t; NULL = legacy default stream)
  * of the current device; the call does not wait for it.
  *
- * The kernel's scratch (cell geometry repacked for the kernel, the node
- * table and the derivative table) lives in one fixed 8 MiB device array
- * inside the library; every GPU that loads the library holds it until the
- * process exits.  n_elem is limited to what fits: 3106 cells at ngll=3,
- * 1310 at ngll=4, 671 at ngll=5, 388 at ngll=6; larger calls are rejected
- * with GFB_ERR_INVALID and a message giving the maximum (split the call).
- * The first call on a device looks up the array's device address, and so
- * does the first call after a device reset (cudaDeviceReset, or the
- * primary context released and created again), where the array can move;
- * make those calls before any CUDA stream capture.  All calls on a device
- * share the one array and each call rewrites the part it reads, so calls
- * that may overlap on the GPU (different streams, or host threads without
- * ordering) race; serialise them on one stream.  FP64 only.
+ * One kernel reads the caller's arrays and writes r; it needs no scratch, so
+ * calls on different streams or from different threads do not disturb each
+ * other, and calls can be captured.  n_elem is limited to 3106 cells at
+ * ngll=3, 1310 at ngll=4, 671 at ngll=5, 388 at ngll=6; larger calls are
+ * rejected with GFB_ERR_INVALID and a message giving the maximum (split the
+ * call).  FP64 only.
  */
 gfb_status gfb_element_residual_noalloc(int32_t n_elem, const double* dxi_dx, const double* jacobian,
                                         const double* lambda_, const double* mu, int32_t ngll,
