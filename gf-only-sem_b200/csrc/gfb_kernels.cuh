@@ -2393,6 +2393,36 @@ __global__ void half_v_kernel(long long n_node, int F, long long hv_begin, bool 
     }
 }
 
+// u, v or a of wavefield `field` in the mesh's node order, out[node][3] as
+// double: one thread per value, the scattered side the read.  inv: node ->
+// device node (nullptr: the same).  what: 0 u, 1 v, 2 a; nodes >= hv_begin
+// hold the half-step velocity, as in half_v_kernel.
+template <typename Real>
+__global__ void state_kernel(long long n_node, int F, int field, int what, const int* inv, const double* u,
+                             const double* v, const Real* a, long long hv_begin, bool a_from_force, const float* w32,
+                             const Real* force, const Real* inv_mass, const uint8_t* node_model, const ModelConst* mc,
+                             double dt, double* out) {
+    const long long total = n_node * 3;
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
+         t += (long long)gridDim.x * blockDim.x) {
+        const long long n = t / 3;
+        const int f = field * 3 + (int)(t - n * 3);
+        const long long g = inv ? inv[n] : n;
+        const size_t i = (size_t)g * F + f;
+        double x;
+        if (what == 0) {
+            x = u[i];
+        } else if (g < hv_begin) {
+            x = what == 1 ? v[i] : (double)a[i];
+        } else {
+            const double h = node_model ? mc[node_model[g]].dt : dt;
+            const double an = a_from_force ? (double)(Real)(force[padded_index(g, f, F)] * inv_mass[g]) : (double)a[i];
+            x = what == 1 ? (double)w32[i] - 0.5 * h * an : (double)(Real)an;
+        }
+        out[t] = x;
+    }
+}
+
 // Recording nodes merged across the recording cells that share them (the
 // strain Green's-function extraction of postprocess/cpp/main.cpp:300-425):
 // strain mass-weighted, sum(m_p e_p) / sum(m_p) over the node's (cell, point)

@@ -261,6 +261,8 @@ struct gfb_solver {
     // and its buffer fits on the device)
     bool gather_ok = false;
     void* contrib = nullptr;        // Real [cell][chunk][nn][fields of the chunk][3] (gfb::NodeGather)
+    size_t contrib_bytes = 0;
+    int* d_node_inv = nullptr;      // node_inv on the device (gfb_get_state)
     uint4* touch = nullptr;         // [node] (gfb::NodeGather)
     uint4* touch_more = nullptr;
     int gather_blocks = 0;          // persistent grid of the gather kernel
@@ -1402,6 +1404,7 @@ gfb_status build_gather(gfb_solver* s, const gfb_mesh* m, const NodeBuckets& nb,
     s->touch = dt;
     s->touch_more = dm;
     s->contrib = dc;
+    s->contrib_bytes = contrib;
     s->gather_ok = true;
     return GFB_OK;
 }
@@ -2619,49 +2622,40 @@ gfb_status gfb_get_state(gfb_solver* s, int32_t field, double* u, double* v, dou
     if (field < 0 || field >= s->nfld) return fail(GFB_ERR_INVALID, "field %d out of range", field);
     CU(cudaSetDevice(s->device));
     CU(cudaStreamSynchronize(s->stream));
-    const size_t nF = (size_t)s->n_node * s->F;
-    std::vector<double> tmp(nF);
     gfb_status st;
-    auto pick = [&](double* dst) {  // device layout [device node][3*n_field]
-        for (long long g = 0; g < s->n_node; ++g) {
-            const long long d = s->node_inv.empty() ? g : s->node_inv[g];
-            for (int c = 0; c < 3; ++c) dst[g * 3 + c] = tmp[d * s->F + field * 3 + c];
-        }
-    };
-    if (u) {
-        if ((st = d2h(s, tmp.data(), s->u, nF * 8))) return st;
-        pick(u);
+    // node -> device node on the device, from the first call on
+    if (!s->node_inv.empty() && !s->d_node_inv) {
+        if ((st = s->alloc(&s->d_node_inv, s->node_inv.size()))) return st;
+        if ((st = h2d(s, s->d_node_inv, s->node_inv.data(), s->node_inv.size() * 4))) return st;
     }
-    // half-step velocity form: (v, a) of the plain nodes recovered into
-    // temporary device arrays (the C-PML nodes copied as they are)
-    double* dv = s->v;
-    void* da = s->a;
-    std::unique_ptr<DevBuf> tv, ta;
-    if (s->half_v && (v || a)) {
-        tv = std::make_unique<DevBuf>();
-        ta = std::make_unique<DevBuf>();
-        CU(cudaMalloc(&tv->p, nF * 8));
-        CU(cudaMalloc(&ta->p, nF * 4));
-        CU(cudaMemcpyAsync(tv->p, s->v, nF * 8, cudaMemcpyDeviceToDevice, s->stream));
-        CU(cudaMemcpyAsync(ta->p, s->a, nF * 4, cudaMemcpyDeviceToDevice, s->stream));
-        if ((st = half_v_to_full(s, static_cast<double*>(tv->p), static_cast<float*>(ta->p)))) return st;
-        CU(cudaStreamSynchronize(s->stream));
-        dv = static_cast<double*>(tv->p);
-        da = ta->p;
+    // gathered on the device into one array in the mesh's node order: the
+    // contribution buffer, which every step writes anew, where it is large
+    // enough (more than one point per node)
+    const size_t bytes = (size_t)s->n_node * 3 * sizeof(double);
+    DevBuf own;
+    double* out = static_cast<double*>(s->contrib);
+    if (s->contrib_bytes < bytes) {
+        CU(cudaMalloc(&own.p, bytes));
+        out = static_cast<double*>(own.p);
     }
-    if (v) {
-        if ((st = d2h(s, tmp.data(), dv, nF * 8))) return st;
-        pick(v);
-    }
-    if (a) {
-        if (s->prec == GFB_FP64) {
-            if ((st = d2h(s, tmp.data(), da, nF * 8))) return st;
-        } else {
-            std::vector<float> f(nF);
-            if ((st = d2h(s, f.data(), da, nF * 4))) return st;
-            for (size_t i = 0; i < nF; ++i) tmp[i] = f[i];
-        }
-        pick(a);
+    double* const dst[3] = {u, v, a};
+    for (int what = 0; what < 3; ++what) {
+        if (!dst[what]) continue;
+        const int grid = grid_for((long long)s->n_node * 3, 256);
+        const long long hv = s->half_v ? s->hv_begin : (long long)s->n_node;
+        if (s->prec == GFB_FP64)
+            gfb::state_kernel<double><<<grid, 256, 0, s->stream>>>(
+                s->n_node, s->F, field, what, s->d_node_inv, s->u, s->v, static_cast<const double*>(s->a), hv, s->a_in_force,
+                s->w32, static_cast<const double*>(s->force), static_cast<const double*>(s->inv_mass), s->d_node_model,
+                s->d_mc, s->dt, out);
+        else
+            gfb::state_kernel<float><<<grid, 256, 0, s->stream>>>(
+                s->n_node, s->F, field, what, s->d_node_inv, s->u, s->v, static_cast<const float*>(s->a), hv, s->a_in_force,
+                s->w32, static_cast<const float*>(s->force), static_cast<const float*>(s->inv_mass), s->d_node_model,
+                s->d_mc, s->dt, out);
+        CU(cudaGetLastError());
+        s->launches++;
+        if ((st = d2h(s, dst[what], out, bytes))) return st;
     }
     return GFB_OK;
 }
