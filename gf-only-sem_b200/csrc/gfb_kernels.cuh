@@ -2288,7 +2288,7 @@ struct RecArgs {
     const double* v;
     const Real* a;
     long long n_node;
-    Out* out;               // [NFLD][n_rec][NN][15]
+    Out* out;               // [NFLD] of strain [n_rec][NN][6], u, v, a [n_rec][NN][3]
     // nodes g >= hv_begin hold the half-step velocity w (w32): a = f/m from
     // the step's assembled force, v = w - dt/2 a
     long long hv_begin;
@@ -2340,7 +2340,10 @@ __global__ void record_kernel(RecArgs<Real, Out> A) {
             gr[c][1] = gx[c] * dd[3] + gy[c] * dd[4] + gz[c] * dd[5];
             gr[c][2] = gx[c] * dd[6] + gy[c] * dd[7] + gz[c] * dd[8];
         }
-        Out* o = A.out + (((size_t)d * A.n_rec + ci) * NN + p) * 15;
+        const size_t points = (size_t)A.n_rec * NN, q = (size_t)ci * NN + p;
+        Out* o = A.out + (size_t)d * points * 15 + q * 6;
+        Out* ou = A.out + ((size_t)d * 15 + 6) * points + q * 3;
+        Out *ov = ou + 3 * points, *oa = ov + 3 * points;
         o[0] = (Out)gr[0][0];
         o[1] = (Out)gr[1][1];
         o[2] = (Out)gr[2][2];
@@ -2352,15 +2355,15 @@ __global__ void record_kernel(RecArgs<Real, Out> A) {
             const Real im = A.inv_mass[g];
             for (int c = 0; c < 3; ++c) {
                 const double an = (double)(Real)(A.force[((size_t)g * NFLD + d) * 4 + c] * im);
-                o[6 + c] = (Out)A.u[(size_t)g * F + d * 3 + c];
-                o[9 + c] = (Out)((double)A.w32[(size_t)g * F + d * 3 + c] - 0.5 * h * an);
-                o[12 + c] = (Out)an;
+                ou[c] = (Out)A.u[(size_t)g * F + d * 3 + c];
+                ov[c] = (Out)((double)A.w32[(size_t)g * F + d * 3 + c] - 0.5 * h * an);
+                oa[c] = (Out)an;
             }
         } else {
             for (int c = 0; c < 3; ++c) {
-                o[6 + c] = (Out)A.u[(size_t)g * F + d * 3 + c];
-                o[9 + c] = (Out)A.v[(size_t)g * F + d * 3 + c];
-                o[12 + c] = (Out)A.a[(size_t)g * F + d * 3 + c];
+                ou[c] = (Out)A.u[(size_t)g * F + d * 3 + c];
+                ov[c] = (Out)A.v[(size_t)g * F + d * 3 + c];
+                oa[c] = (Out)A.a[(size_t)g * F + d * 3 + c];
             }
         }
     }
@@ -2427,23 +2430,25 @@ __global__ void state_kernel(long long n_node, int F, int field, int what, const
 // strain Green's-function extraction of postprocess/cpp/main.cpp:300-425):
 // strain mass-weighted, sum(m_p e_p) / sum(m_p) over the node's (cell, point)
 // occurrences; u, v, a averaged.  One thread per (wavefield, node, value),
-// reading the snapshot's cell-point records (out[field][rec][NN][15]) and
-// writing merged[field][node][15] behind them in the same slot.
+// reading the snapshot's cell-point records (RecArgs::out, per_field points)
+// and writing merged[field][node][15] behind them in the same slot.
 template <typename Out>
 __global__ void merge_nodes_kernel(int n_field, int n_unique, long long per_field, const int* ptr, const int* occ,
                                    const double* w, Out* slot) {
     const long long total = (long long)n_field * n_unique * 15;
-    Out* merged = slot + (size_t)n_field * per_field;
+    Out* merged = slot + (size_t)n_field * per_field * 15;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
         const int c = (int)(t % 15);
         const long long fn = t / 15;
         const int node = (int)(fn % n_unique), f = (int)(fn / n_unique);
-        const Out* src = slot + (size_t)f * per_field;
+        // component c of the field's points, `w0` values apart
+        const int w0 = c < 6 ? 6 : 3;
+        const Out* src = slot + (size_t)f * per_field * 15 + (c < 6 ? c : per_field * (c / 3 * 3) + c % 3);
         double acc = 0.0, ws = 0.0;
         for (int k = ptr[node]; k < ptr[node + 1]; ++k) {
             const double wk = c < 6 ? w[k] : 1.0;
-            acc += wk * (double)src[(size_t)occ[k] * 15 + c];
+            acc += wk * (double)src[(size_t)occ[k] * w0];
             ws += wk;
         }
         merged[((size_t)f * n_unique + node) * 15 + c] = (Out)(ws > 0.0 ? acc / ws : 0.0);

@@ -342,6 +342,7 @@ struct gfb_solver {
     std::vector<void*> pinned;         // pinned host copy of each slot
     bool rec_f32 = false;              // snapshot values stored as float
     std::vector<cudaEvent_t> rec_evt;  // record kernel of the slot done
+    std::vector<cudaEvent_t> cell_evt; // the records' part of the slot is on the host
     std::vector<cudaEvent_t> copy_evt; // device->host copy of the slot done
     std::vector<char> copy_issued;
     int next_slot = 0;
@@ -381,6 +382,7 @@ struct gfb_solver {
         drop_graphs();
         if (layer) gfb::layer_free(layer);
         for (auto e : rec_evt) cudaEventDestroy(e);
+        for (auto e : cell_evt) cudaEventDestroy(e);
         for (auto e : copy_evt) cudaEventDestroy(e);
         for (auto p : pinned) cudaFreeHost(p);
         bufs.clear();
@@ -1180,7 +1182,8 @@ gfb_status launch_predict(gfb_solver* s) {
     return GFB_OK;
 }
 
-// A snapshot: the recording cells' records [field][rec][NN][15], then the
+// A snapshot: per wavefield the recording cells' strain [rec][NN][6], u, v and
+// a [rec][NN][3] (the arrays of a record, so reading one is a copy), then the
 // same values merged per recording node [field][node][15].
 size_t snapshot_cell_values(const gfb_solver* s) { return (size_t)s->nfld * s->n_rec * s->nn * 15; }
 size_t snapshot_values(const gfb_solver* s) {
@@ -1210,6 +1213,31 @@ void unpack_points(const gfb_solver* s, const void* raw, long long n_out, Index 
                 }
             }
         }, 16384);
+    };
+    if (s->rec_f32) run(static_cast<const float*>(raw));
+    else run(static_cast<const double*>(raw));
+}
+
+// Wavefield `field` of a raw snapshot into the caller's arrays (NULL: skipped),
+// converted where the types differ; the threads split the values.
+template <typename Out>
+void unpack_record(const gfb_solver* s, const void* raw, int field, Out* strain, Out* u, Out* v, Out* a) {
+    const long long P = (long long)s->n_rec * s->nn;
+    auto run = [&](auto* src0) {
+        const auto* src = src0 + (size_t)field * P * 15;
+        Out* const dst[4] = {strain, u, v, a};
+        const long long first[5] = {0, 6 * P, 9 * P, 12 * P, 15 * P};
+        parallel_for(15 * P, [&](long long i0, long long i1) {
+            for (int k = 0; k < 4; ++k) {
+                const long long b = std::max(i0, first[k]), e = std::min(i1, first[k + 1]);
+                if (!dst[k] || e <= b) continue;
+                Out* to = dst[k] + (b - first[k]);
+                if constexpr (std::is_same<decltype(src), const Out*>::value)
+                    std::memcpy(to, src + b, (size_t)(e - b) * sizeof(Out));
+                else
+                    for (long long i = 0; i < e - b; ++i) to[i] = (Out)src[b + i];
+            }
+        }, 262144);
     };
     if (s->rec_f32) run(static_cast<const float*>(raw));
     else run(static_cast<const double*>(raw));
@@ -1863,10 +1891,12 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
         if ((st = s->alloc(&ring, snapshot_bytes(s) * s->slots))) return st;
         s->ring = ring;
         s->rec_evt.assign(s->slots, nullptr);
+        s->cell_evt.assign(s->slots, nullptr);
         s->copy_evt.assign(s->slots, nullptr);
         s->copy_issued.assign(s->slots, 0);
         for (int k = 0; k < s->slots; ++k) {
             CU(cudaEventCreateWithFlags(&s->rec_evt[k], cudaEventDisableTiming));
+            CU(cudaEventCreateWithFlags(&s->cell_evt[k], cudaEventDisableTiming));
             CU(cudaEventCreateWithFlags(&s->copy_evt[k], cudaEventDisableTiming));
         }
         CU(host_ring.finish());
@@ -2039,22 +2069,29 @@ gfb_status some_steps(gfb_solver* s, int n, cudaEvent_t* ev, int* done) {
         if (s->copy_issued[slot]) CU(cudaStreamWaitEvent(s->stream, s->copy_evt[slot], 0));
         void* dslot = static_cast<unsigned char*>(s->ring) + (size_t)slot * snapshot_bytes(s);
         if ((st = launch_record(s, dslot))) return st;
+        // on the copy stream, beside the following steps: the records to the
+        // host, then the merge and its part
+        CU(cudaEventRecord(s->rec_evt[slot], s->stream));
+        CU(cudaStreamWaitEvent(s->copy_stream, s->rec_evt[slot], 0));
+        const size_t cell_bytes = snapshot_cell_values(s) * (s->rec_f32 ? 4 : 8);
+        unsigned char* host = static_cast<unsigned char*>(s->pinned[slot]);
+        CU(cudaMemcpyAsync(host, dslot, cell_bytes, cudaMemcpyDeviceToHost, s->copy_stream));
+        CU(cudaEventRecord(s->cell_evt[slot], s->copy_stream));
         {
             const long long total = (long long)s->nfld * s->n_unique * 15;
             const int grid = grid_for(total, 256);
-            const long long per_field = (long long)s->n_rec * s->nn * 15;
+            const long long per_field = (long long)s->n_rec * s->nn;
             if (s->rec_f32)
-                gfb::merge_nodes_kernel<float><<<grid, 256, 0, s->stream>>>(s->nfld, s->n_unique, per_field, s->gf_ptr,
-                                                                              s->gf_occ, s->gf_w, static_cast<float*>(dslot));
+                gfb::merge_nodes_kernel<float><<<grid, 256, 0, s->copy_stream>>>(
+                    s->nfld, s->n_unique, per_field, s->gf_ptr, s->gf_occ, s->gf_w, static_cast<float*>(dslot));
             else
-                gfb::merge_nodes_kernel<double><<<grid, 256, 0, s->stream>>>(
+                gfb::merge_nodes_kernel<double><<<grid, 256, 0, s->copy_stream>>>(
                     s->nfld, s->n_unique, per_field, s->gf_ptr, s->gf_occ, s->gf_w, static_cast<double*>(dslot));
             CU(cudaGetLastError());
             s->launches++;
         }
-        CU(cudaEventRecord(s->rec_evt[slot], s->stream));
-        CU(cudaStreamWaitEvent(s->copy_stream, s->rec_evt[slot], 0));
-        CU(cudaMemcpyAsync(s->pinned[slot], dslot, snapshot_bytes(s), cudaMemcpyDeviceToHost, s->copy_stream));
+        CU(cudaMemcpyAsync(host + cell_bytes, static_cast<unsigned char*>(dslot) + cell_bytes, snapshot_bytes(s) - cell_bytes,
+                           cudaMemcpyDeviceToHost, s->copy_stream));
         CU(cudaEventRecord(s->copy_evt[slot], s->copy_stream));
         s->copy_issued[slot] = 1;
         Snapshot snap;
@@ -2460,6 +2497,7 @@ gfb_status gfb_destroy(gfb_solver* s) {
     if (!s) return GFB_OK;
     cudaSetDevice(s->device);
     cudaStreamSynchronize(s->stream);
+    cudaStreamSynchronize(s->copy_stream);
     delete s;
     return GFB_OK;
 }
@@ -2864,14 +2902,12 @@ gfb_status read_record_t(gfb_solver* s, int32_t field, int32_t* step, Out* strai
     }
     // copy out without holding the lock (the stepping thread may go on)
     gfb_status st = GFB_OK;
-    if (slot >= 0 && cudaEventSynchronize(s->copy_evt[slot]) != cudaSuccess)
+    if (slot >= 0 && cudaEventSynchronize(s->cell_evt[slot]) != cudaSuccess)
         st = fail(GFB_ERR_CUDA, "snapshot copy failed");
     if (step) *step = snap->step;
     if (!st && (strain || u || v || a)) {
         const void* raw = slot >= 0 ? s->pinned[slot] : (const void*)snap->host.get();
-        const long long first = (long long)field * s->n_rec * s->nn;  // points of the earlier fields
-        unpack_points(s, raw, (long long)s->n_rec * s->nn, [first](long long q) { return first + q; }, strain, u,
-                      v, a);
+        unpack_record(s, raw, field, strain, u, v, a);
     }
     {
         std::lock_guard<std::mutex> lk(s->rec_mu);
