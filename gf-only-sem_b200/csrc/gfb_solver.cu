@@ -1056,7 +1056,8 @@ gfb_status launch_node_m(gfb_solver* s) {
         // 40 x 40 x 20), 187 / 177 (ngll 6, 22 x 21 x 13).  Beside the plane
         // kernel and at ngll 3 it gains: 400 / 405 (40 x 40 x 20 x 3), 68 / 72
         // (20 x 20 x 10 x 3), 72 / 81 (six small models), 69.5 / 72.5 (ngll 3).
-        const bool early = use_gather(s) && s->prec == GFB_FP32 && (s->plane_blocks > 0 || s->ng == 3);
+        const bool early = use_gather(s) && s->prec == GFB_FP32 && !(s->has_cpml && !s->node_pml) &&
+                           (s->plane_blocks > 0 || s->ng == 3);
         CU(launch_chained(early, fn, node_grid(s->n_node - g0, gfb::node_blocks_per_sm<Real>(false)), gfb::kNodeThreads, 0,
                           s->stream, A, P, g0));
         s->launches++;
