@@ -111,8 +111,8 @@ def build_batch(threads: int = 8):
 
 
 def run_batch(args):
-    """32 models of uneven size in one solver: one element launch per colour
-    over all of them, the step replayed as a CUDA graph, kernel variant picked
+    """32 models of uneven size in one solver: one element launch over all of
+    them, the step replayed as a CUDA graph, kernel variant picked
     by the autotuner.  Reported: aggregate GLL-point updates/s over the whole
     run (every model to its last step) and each model's completion time."""
     import gfb
@@ -436,27 +436,35 @@ def node_pml_live_axes(prob):
 
 
 def elem_bytes_per_step(prob, info, n_field, prec):
-    """Algorithmic DRAM bytes of one step's element/assembly launches
-    (unpadded component bytes; the [node][field][4] layout moves 4/3 of the
-    gather/force bytes, visible in the ncu traffic).  With the force updated
-    by increments (all but one step in the refresh period) every touch of a
-    node reads and writes its force."""
+    """Algorithmic DRAM bytes of one step's element phase (unpadded component
+    bytes): geometry and node numbers per point, the predicted displacement
+    (or its increment) once per node, and the force: the cells' contributions
+    written, or, in the kernels that assemble by colour, read and written at
+    every touch (in full: the first touch of a node only writes)."""
     nn = 125
     P = prob["n_cell"] * nn
     G = prob["n_node"]
     sr = 4 if prec == 1 else 8
     F = 3 * n_field
-    geom = P * 12 * sr + P * 4                      # geometry + ibool
-    gather = P * F * sr                              # predicted displacement (or its increment)
-    if info.get("force_refresh", 1) > 1:             # force by increments: every touch reads and writes
+    geom = P * 11 * sr + P * 4                      # geometry + ibool
+    gather = G * F * sr                              # predicted displacement (or its increment)
+    if not by_colour(info, prec):                    # contributions
+        force = P * F * sr
+    elif info.get("force_refresh", 1) > 1:           # force by increments: every touch reads and writes
         force = P * F * sr * 2
     else:                                            # in full: first touch writes, others read+write
         force = G * F * sr + (P - G) * F * sr * 2
     pml = 0
-    if info["n_pml_node"] == 0:                      # per-cell C-PML in this kernel
+    if info["n_pml_node"] == 0:                      # per-cell C-PML (one live axis)
         Ppml = info["n_pml_cell"] * nn
-        pml = Ppml * (15 * sr + F * 3 * sr * 2 + F * sr * 2 + F * 16 + F * sr)
+        pml = Ppml * (7 * sr + F * sr * 2 + F * sr * 2 + F * 16 + F * sr)
     return geom + gather + force + pml
+
+
+def by_colour(info, prec):
+    """Whether the element phase assembles by colour (FP32 kernels selected
+    instead of the default one)."""
+    return prec == 1 and info.get("elem_variant", 0) != 0
 
 
 def node_bytes_per_step(prob, info, n_field, prec):
@@ -474,6 +482,8 @@ def node_bytes_per_step(prob, info, n_field, prec):
     state = 16 + 8 if info.get("half_v") else 16 + 16 + 2 * sr   # u (+ w | v, a) read and written
     mass = 4 if prec == 1 else 8
     base = n_plain * (F * (state + 2 * sr) + mass) + n_pml * (F * (32 + 4 * sr) + mass)
+    if not by_colour(info, prec):                    # contributions and touches read, the force kept (FP32)
+        base += prob["n_cell"] * 125 * F * sr + prob["n_node"] * (16 + (F * sr if prec == 1 else -F * sr))
     if n_pml > 0:                                    # node-form C-PML in this kernel
         n_live, live = node_pml_live_axes(prob)
         base += n_live * (14 * sr + F * sr * 2) + live * F * sr * 2
@@ -481,7 +491,7 @@ def node_bytes_per_step(prob, info, n_field, prec):
 
 
 def committed_traffic():
-    path = os.path.join(REPO, "profiles", "elem_col_traffic_deformed_64x64x32.json")
+    path = os.path.join(REPO, "profiles", "elem_plane_traffic_deformed_64x64x32.json")
     try:
         with open(path) as f:
             return json.load(f)
@@ -518,7 +528,7 @@ def fp64_plain_sample(prob, device, args, fp32_value_per_gpu, peak):
             "phases_ms_per_step": {"element": ms_e / k, "node": ms_n / k, "record": ms_r / k},
             "roofline_element": {"achieved": eb / (ms_e / k / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                                  "frac": eb / (ms_e / k / 1e3) / 1e9 / peak, "algorithmic_bytes_per_step": eb,
-                                 "kernel": "elem_pipe_kernel<double,5,1> (all colour launches of a step)"},
+                                 "kernel": "elem_gather_kernel<double,5> and cell_pml_kernel<double,5>"},
             "roofline_node": {"achieved": nb / (ms_n / k / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                               "algorithmic_bytes_per_step": nb},
             "fp32_batched_over_fp64_plain": fp32_value_per_gpu / val}
@@ -726,10 +736,12 @@ def run_gfb(args):
     flags = (gfb.FLAG_RECORD_F32 if args.record_f32 else 0) | (gfb.FLAG_POINT_KERNEL if args.point_kernel else 0)
     s = gfb.Solver(prob, dirs=dirs, precision=prec, device=device, record_slots=8, flags=flags)
     info = s.info()
-    if prec == gfb.FP32 and not args.point_kernel:
-        kname = f"elem_col_kernel<5,{len(dirs)}>"
+    if args.point_kernel:
+        kname = f"elem_pipe_kernel<{'float' if prec == gfb.FP32 else 'double'},5,{len(dirs)}> (by colour)"
+    elif prec == gfb.FP32 and len(dirs) == 3:
+        kname = "elem_plane_kernel"
     else:
-        kname = f"elem_pipe_kernel<{'float' if prec == gfb.FP32 else 'double'},5,{len(dirs)}>"
+        kname = f"elem_gather_kernel<{'float' if prec == gfb.FP32 else 'double'},5>"
     s.advance(args.warmup)
     s.drain()
     s.synchronize()
@@ -841,11 +853,11 @@ def run_gfb(args):
                                "note": f"phases from {n_prof} eagerly launched steps; value from the graph-replayed K"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind,
-                     "kernel": f"{kname} (all colour launches of a step)",
+                     "kernel": kname,
                      "algorithmic_bytes_per_step": eb,
                      "traffic": (traffic["bytes_per_cell"] * prob["n_cell"]
-                                 if traffic and prec == gfb.FP32 and not args.point_kernel else None),
-                     "traffic_source": (traffic or {}).get("source") if traffic else None},
+                                 if traffic and kname == "elem_plane_kernel" else None),
+                     "traffic_source": traffic["source"] if traffic and kname == "elem_plane_kernel" else None},
         "roofline_node": {"achieved": nb / (ms_node / args.steps / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                           "algorithmic_bytes_per_step": nb},
         "e2e": {"value": e2e_val, "unit": UNIT, "h2d_bytes_per_step": up / args.steps,
