@@ -1369,6 +1369,11 @@ gfb_status build_gather(gfb_solver* s, const gfb_mesh* m, const NodeBuckets& nb,
     size_t free_b = 0, total_b = 0;
     CU(cudaMemGetInfo(&free_b, &total_b));
     if (free_b < contrib + (size_t)s->n_node * (24 + 4 * s->F) + (size_t(1) << 30)) return GFB_OK;
+    Real* dc = nullptr;
+    if (s->alloc(&dc, units * 3)) {  // taken by someone else meanwhile
+        (void)cudaGetLastError();
+        return GFB_OK;
+    }
     // the second to fourth touch of each node, or where the touches from the
     // fourth on are
     struct Rest {
@@ -1428,8 +1433,6 @@ gfb_status build_gather(gfb_solver* s, const gfb_mesh* m, const NodeBuckets& nb,
     if ((st = s->alloc(&dm, base.back()))) return st;
     for (int t = 0; t < nb.n_owner; ++t)
         if (!more[t].empty() && (st = h2d(s, dm + base[t], more[t].data(), more[t].size() * sizeof(uint4)))) return st;
-    Real* dc = nullptr;
-    if ((st = s->alloc(&dc, units * 3))) return st;
     s->touch = dt;
     s->touch_more = dm;
     s->contrib = dc;
