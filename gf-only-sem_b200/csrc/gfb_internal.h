@@ -48,6 +48,10 @@ gfb_status solver_predict(gfb_solver* s);
 // that reads or writes v and a of any node between steps.
 gfb_status solver_full_state(gfb_solver* s);
 
+// GFB_ERR_CUDA once a kernel of the solver has given up a wait on its own
+// copies (its state is invalid); call after synchronising with the solver.
+gfb_status solver_check(gfb_solver* s);
+
 // Learned absorbing layer attached to a solver (gfb_layer.cu): launched
 // between the element phase and the node phase of every step; freed with the
 // solver.
@@ -58,3 +62,8 @@ Layer* solver_layer(gfb_solver* s);
 gfb_status solver_set_layer(gfb_solver* s, Layer* layer);
 
 }  // namespace gfb
+
+// Leaves the solver as a kernel whose bounded wait gave up would (no kernel
+// can be made to: the wait is for its own copies).  For the error paths'
+// tests; not part of the interface.
+extern "C" gfb_status gfb_inject_kernel_error(gfb_solver* solver);

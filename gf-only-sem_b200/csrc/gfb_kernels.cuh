@@ -1767,10 +1767,12 @@ __global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Re
         for (int i = 0; i < NG; ++i) nw[i] = nw2[i];
         load_words(next + step, nw2);
         if (any(!mbar_wait(bar, phase))) {
-            // the copy never came: flag it, give it a second bounded wait, leave
+            // the copy never came: flag it, give it a second bounded wait, let
+            // the stores on their way read their shared memory, leave
             if (gt == 0) {
                 atomicOr(A.err, 1u);
                 mbar_wait(bar, phase);
+                bulk_wait_all();
             }
             return;
         }

@@ -991,6 +991,7 @@ gfb_status gfb_trainer_collect(gfb_trainer* t, gfb_solver* thin, gfb_solver* thi
         }
     }
     LCU(cudaStreamSynchronize(a.stream));
+    if ((st = solver_check(thick)) || (st = solver_check(thin))) return st;
     return GFB_OK;
 }
 

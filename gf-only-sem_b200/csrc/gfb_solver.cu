@@ -322,7 +322,10 @@ struct gfb_solver {
     int refresh = 1;
     bool by_increments_ok = false;     // the force may be updated by increments (FP32, node-form or no C-PML, ...)
     int *d_mdirect = nullptr, *d_mnext = nullptr, *d_force_direct = nullptr;
-    int* d_kernel_err = nullptr;       // set by a kernel whose bounded wait gave up
+    // set by a kernel whose bounded wait gave up: a word of mapped host memory,
+    // so that every call that hands out results can look at it without a copy
+    // (after the synchronisation that the results need anyway)
+    unsigned *kernel_err = nullptr, *d_kernel_err = nullptr;
     // plain nodes (device nodes >= hv_begin) keep the half-step velocity
     // v + dt/2 a in v and no acceleration (FP32 path); a_in_force: the
     // assembled force holds the last step's (a = f/m), else a is the stored
@@ -385,6 +388,7 @@ struct gfb_solver {
         for (auto e : cell_evt) cudaEventDestroy(e);
         for (auto e : copy_evt) cudaEventDestroy(e);
         for (auto p : pinned) cudaFreeHost(p);
+        if (kernel_err) cudaFreeHost(kernel_err);
         bufs.clear();
         if (stream) cudaStreamDestroy(stream);
         if (copy_stream) cudaStreamDestroy(copy_stream);
@@ -702,7 +706,7 @@ gfb_status launch_col_e(gfb_solver* s, int c) {
     }
     for (int q = 0; q < 36; ++q) A.D[q] = q < NG * NG ? s->dmat_host[q] : 0.0;
     const int blocks = std::max(1, std::min(A.n_groups, s->col_blocks));
-    A.err = reinterpret_cast<unsigned*>(s->d_kernel_err);
+    A.err = s->d_kernel_err;
     const int smem = S::SMEM + gfb::col_model_smem(s->n_model, s->n_set);
     gfb::elem_col_kernel<NG, NFLD, EPB><<<blocks, S::THREADS, smem, s->stream>>>(A);
     CU(cudaGetLastError());
@@ -768,7 +772,7 @@ gfb_status launch_gather_t(gfb_solver* s) {
         A.dir[d] = s->dirs[d];
         A.fset[d] = s->fset[d];
     }
-    A.err = reinterpret_cast<unsigned*>(s->d_kernel_err);
+    A.err = s->d_kernel_err;
     for (int q = 0; q < 36; ++q) A.D[q] = q < NG * NG ? (Real)s->dmat_host[q] : Real(0);
     for (int q = 0; q < 36; ++q) A.D2[q] = make_float2((float)A.D[q], (float)A.D[q]);
     // a work item is a group's cells with all their wavefields (the geometry
@@ -1827,7 +1831,6 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
         if ((st = put_int(&s->d_mdirect, one))) return st;
         if ((st = put_int(&s->d_mnext, one))) return st;
         if ((st = put_int(&s->d_force_direct, zero))) return st;
-        if ((st = put_int(&s->d_kernel_err, std::vector<int>(1, 0)))) return st;
         if ((st = s->alloc(&s->d_stf_off, off.size()))) return st;
         if ((st = h2d(s, s->d_stf_off, off.data(), off.size() * 8))) return st;
         if ((st = upload(s, &s->d_stf_all, stf_all))) return st;
@@ -1956,6 +1959,16 @@ gfb_status launch_step_begin_t(gfb_solver* s) {
                           s->d_live_cell_end, s->d_live_node_end));
         s->launches++;
     }
+    return GFB_OK;
+}
+
+// A kernel whose bounded wait on its own bulk copies gave up left its step
+// unfinished, and every step after it built on that: no result leaves the
+// solver from then on.  Called where the work that the result comes from has
+// been synchronised with.
+gfb_status check_kernel_err(const gfb_solver* s) {
+    if (s->kernel_err && *static_cast<volatile const unsigned*>(s->kernel_err))
+        return fail(GFB_ERR_CUDA, "element kernel: a bulk copy did not complete; the state is invalid");
     return GFB_OK;
 }
 
@@ -2232,6 +2245,9 @@ gfb_status create_impl(const gfb_mesh* m, const gfb_config* c, const gfb_source*
     s->c2 = (1.0 - theta) * 0.5 * c->dt * c->dt;
     CU(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     CU(cudaStreamCreateWithFlags(&s->copy_stream, cudaStreamNonBlocking));
+    CU(cudaHostAlloc(reinterpret_cast<void**>(&s->kernel_err), sizeof(unsigned), cudaHostAllocMapped));
+    *s->kernel_err = 0;
+    CU(cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->d_kernel_err), s->kernel_err, 0));
 
     StageClock clk;
     const int nn = s->nn;
@@ -2506,18 +2522,6 @@ gfb_status gfb_destroy(gfb_solver* s) {
     return GFB_OK;
 }
 
-namespace {
-// A kernel whose bounded wait on its own bulk copies gave up left the step
-// unfinished: report it at the next synchronisation.
-gfb_status check_kernel_err(gfb_solver* s) {
-    if (!s->d_kernel_err) return GFB_OK;
-    int e = 0;
-    CU(cudaMemcpy(&e, s->d_kernel_err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (e) return fail(GFB_ERR_CUDA, "element kernel: a bulk copy did not complete; the state is invalid");
-    return GFB_OK;
-}
-}  // namespace
-
 gfb_status gfb_advance(gfb_solver* s, int32_t n_steps) {
     if (!s) return fail(GFB_ERR_INVALID, "solver is NULL");
     if (n_steps < 0) return fail(GFB_ERR_INVALID, "n_steps must be >= 0");
@@ -2578,7 +2582,7 @@ gfb_status gfb_advance_profiled(gfb_solver* s, int32_t n_steps, double* ms_eleme
     }
     for (auto e : ev)
         if (e) cudaEventDestroy(e);
-    if (st) return st;
+    if (st || (st = check_kernel_err(s))) return st;
     if (ms_element) *ms_element += acc[0];
     if (ms_node) *ms_node += acc[1];
     if (ms_record) *ms_record += acc[2];
@@ -2665,6 +2669,7 @@ gfb_status gfb_get_state(gfb_solver* s, int32_t field, double* u, double* v, dou
     CU(cudaSetDevice(s->device));
     CU(cudaStreamSynchronize(s->stream));
     gfb_status st;
+    if ((st = check_kernel_err(s))) return st;
     // node -> device node on the device, from the first call on
     if (!s->node_inv.empty() && !s->d_node_inv) {
         if ((st = s->alloc(&s->d_node_inv, s->node_inv.size()))) return st;
@@ -2837,6 +2842,7 @@ gfb_status gfb_checkpoint_save(gfb_solver* s, void* buf, int64_t bytes) {
     if (!buf || bytes < need) return fail(GFB_ERR_INVALID, "checkpoint buffer needs %lld bytes", (long long)need);
     CU(cudaSetDevice(s->device));
     CU(cudaStreamSynchronize(s->stream));
+    if ((st = check_kernel_err(s))) return st;
     CheckpointHeader h;
     checkpoint_header(s, need, h);
     unsigned char* p = static_cast<unsigned char*>(buf);
@@ -2908,6 +2914,7 @@ gfb_status read_record_t(gfb_solver* s, int32_t field, int32_t* step, Out* strai
     gfb_status st = GFB_OK;
     if (slot >= 0 && cudaEventSynchronize(s->cell_evt[slot]) != cudaSuccess)
         st = fail(GFB_ERR_CUDA, "snapshot copy failed");
+    if (!st) st = check_kernel_err(s);
     if (step) *step = snap->step;
     if (!st && (strain || u || v || a)) {
         const void* raw = slot >= 0 ? s->pinned[slot] : (const void*)snap->host.get();
@@ -2969,6 +2976,7 @@ gfb_status gfb_read_green(gfb_solver* s, int32_t* step, double* strain, double* 
     gfb_status st = GFB_OK;
     if (slot >= 0 && cudaEventSynchronize(s->copy_evt[slot]) != cudaSuccess)
         st = fail(GFB_ERR_CUDA, "snapshot copy failed");
+    if (!st) st = check_kernel_err(s);
     if (step) *step = snap->step;
     if (!st) {
         // merged part [field][node][15] after the cell part, read out as
@@ -3049,6 +3057,7 @@ gfb_status gfb_element_residual(int32_t n_elem, const double* dxi_dx, const doub
     }
     if ((st = launch_elem(s))) return st;
     CU(cudaStreamSynchronize(s->stream));
+    if ((st = check_kernel_err(s))) return st;
     if (use_gather(s)) {  // one touch per node: the contributions are the residual
         auto read = [&](auto zero) -> gfb_status {
             const size_t row = (size_t)gfb::gather_chunk_units<decltype(zero)>(nn, 1) * 3;
@@ -3112,6 +3121,8 @@ gfb_status solver_predict(gfb_solver* s) { return launch_predict(s); }
 
 gfb_status solver_full_state(gfb_solver* s) { return leave_half_v(s); }
 
+gfb_status solver_check(gfb_solver* s) { return check_kernel_err(s); }
+
 Layer* solver_layer(gfb_solver* s) { return s->layer; }
 
 gfb_status solver_set_layer(gfb_solver* s, Layer* layer) {
@@ -3135,3 +3146,9 @@ gfb_status solver_set_layer(gfb_solver* s, Layer* layer) {
 }
 
 }  // namespace gfb
+
+extern "C" gfb_status gfb_inject_kernel_error(gfb_solver* s) {
+    if (!s) return fail(GFB_ERR_INVALID, "solver is NULL");
+    *s->kernel_err = 1;
+    return GFB_OK;
+}
