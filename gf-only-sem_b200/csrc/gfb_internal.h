@@ -67,3 +67,8 @@ gfb_status solver_set_layer(gfb_solver* s, Layer* layer);
 // can be made to: the wait is for its own copies).  For the error paths'
 // tests; not part of the interface.
 extern "C" gfb_status gfb_inject_kernel_error(gfb_solver* solver);
+
+// Whether any work of the solver is still queued or running on the device
+// (1) or not (0), without waiting.  For the tests of what the interface's
+// calls wait for; not part of the interface.
+extern "C" gfb_status gfb_work_queued(gfb_solver* solver, int32_t* queued);

@@ -239,7 +239,8 @@ struct Snapshot {
 struct gfb_solver {
     int device = 0;
     cudaStream_t stream = nullptr;
-    cudaStream_t copy_stream = nullptr;
+    cudaStream_t copy_stream = nullptr;   // snapshots to the host
+    cudaStream_t merge_stream = nullptr;  // their merge per recording node
     int prec = GFB_FP64;
     int ng = 0, nn = 0, nfld = 1, F = 3;
     int n_cell = 0, n_node = 0;
@@ -345,6 +346,7 @@ struct gfb_solver {
     std::vector<void*> pinned;         // pinned host copy of each slot
     bool rec_f32 = false;              // snapshot values stored as float
     std::vector<cudaEvent_t> rec_evt;  // record kernel of the slot done
+    std::vector<cudaEvent_t> merge_evt;  // merge kernel of the slot done
     std::vector<cudaEvent_t> cell_evt; // the records' part of the slot is on the host
     std::vector<cudaEvent_t> copy_evt; // device->host copy of the slot done
     std::vector<char> copy_issued;
@@ -385,6 +387,7 @@ struct gfb_solver {
         drop_graphs();
         if (layer) gfb::layer_free(layer);
         for (auto e : rec_evt) cudaEventDestroy(e);
+        for (auto e : merge_evt) cudaEventDestroy(e);
         for (auto e : cell_evt) cudaEventDestroy(e);
         for (auto e : copy_evt) cudaEventDestroy(e);
         for (auto p : pinned) cudaFreeHost(p);
@@ -392,6 +395,7 @@ struct gfb_solver {
         bufs.clear();
         if (stream) cudaStreamDestroy(stream);
         if (copy_stream) cudaStreamDestroy(copy_stream);
+        if (merge_stream) cudaStreamDestroy(merge_stream);
     }
 };
 
@@ -1898,11 +1902,13 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
         if ((st = s->alloc(&ring, snapshot_bytes(s) * s->slots))) return st;
         s->ring = ring;
         s->rec_evt.assign(s->slots, nullptr);
+        s->merge_evt.assign(s->slots, nullptr);
         s->cell_evt.assign(s->slots, nullptr);
         s->copy_evt.assign(s->slots, nullptr);
         s->copy_issued.assign(s->slots, 0);
         for (int k = 0; k < s->slots; ++k) {
             CU(cudaEventCreateWithFlags(&s->rec_evt[k], cudaEventDisableTiming));
+            CU(cudaEventCreateWithFlags(&s->merge_evt[k], cudaEventDisableTiming));
             CU(cudaEventCreateWithFlags(&s->cell_evt[k], cudaEventDisableTiming));
             CU(cudaEventCreateWithFlags(&s->copy_evt[k], cudaEventDisableTiming));
         }
@@ -2086,9 +2092,10 @@ gfb_status some_steps(gfb_solver* s, int n, cudaEvent_t* ev, int* done) {
         if (s->copy_issued[slot]) CU(cudaStreamWaitEvent(s->stream, s->copy_evt[slot], 0));
         void* dslot = static_cast<unsigned char*>(s->ring) + (size_t)slot * snapshot_bytes(s);
         if ((st = launch_record(s, dslot))) return st;
-        // on the copy stream, beside the following steps: the records to the
-        // host, then the merge and its part
+        // beside the following steps: the merge on its own stream, the records
+        // and then the merged part to the host on the copy stream
         CU(cudaEventRecord(s->rec_evt[slot], s->stream));
+        CU(cudaStreamWaitEvent(s->merge_stream, s->rec_evt[slot], 0));
         CU(cudaStreamWaitEvent(s->copy_stream, s->rec_evt[slot], 0));
         const size_t cell_bytes = snapshot_cell_values(s) * (s->rec_f32 ? 4 : 8);
         unsigned char* host = static_cast<unsigned char*>(s->pinned[slot]);
@@ -2099,14 +2106,17 @@ gfb_status some_steps(gfb_solver* s, int n, cudaEvent_t* ev, int* done) {
             const int grid = grid_for(total, 256);
             const long long per_field = (long long)s->n_rec * s->nn;
             if (s->rec_f32)
-                gfb::merge_nodes_kernel<float><<<grid, 256, 0, s->copy_stream>>>(
+                gfb::merge_nodes_kernel<float><<<grid, 256, 0, s->merge_stream>>>(
                     s->nfld, s->n_unique, per_field, s->gf_ptr, s->gf_occ, s->gf_w, static_cast<float*>(dslot));
             else
-                gfb::merge_nodes_kernel<double><<<grid, 256, 0, s->copy_stream>>>(
+                gfb::merge_nodes_kernel<double><<<grid, 256, 0, s->merge_stream>>>(
                     s->nfld, s->n_unique, per_field, s->gf_ptr, s->gf_occ, s->gf_w, static_cast<double*>(dslot));
             CU(cudaGetLastError());
             s->launches++;
         }
+        CU(cudaEventRecord(s->merge_evt[slot], s->merge_stream));
+        if (ev) CU(cudaStreamWaitEvent(s->stream, s->merge_evt[slot], 0));  // in the phase's time
+        CU(cudaStreamWaitEvent(s->copy_stream, s->merge_evt[slot], 0));
         CU(cudaMemcpyAsync(host + cell_bytes, static_cast<unsigned char*>(dslot) + cell_bytes, snapshot_bytes(s) - cell_bytes,
                            cudaMemcpyDeviceToHost, s->copy_stream));
         CU(cudaEventRecord(s->copy_evt[slot], s->copy_stream));
@@ -2245,6 +2255,7 @@ gfb_status create_impl(const gfb_mesh* m, const gfb_config* c, const gfb_source*
     s->c2 = (1.0 - theta) * 0.5 * c->dt * c->dt;
     CU(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     CU(cudaStreamCreateWithFlags(&s->copy_stream, cudaStreamNonBlocking));
+    CU(cudaStreamCreateWithFlags(&s->merge_stream, cudaStreamNonBlocking));
     CU(cudaHostAlloc(reinterpret_cast<void**>(&s->kernel_err), sizeof(unsigned), cudaHostAllocMapped));
     *s->kernel_err = 0;
     CU(cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->d_kernel_err), s->kernel_err, 0));
@@ -2518,6 +2529,7 @@ gfb_status gfb_destroy(gfb_solver* s) {
     cudaSetDevice(s->device);
     cudaStreamSynchronize(s->stream);
     cudaStreamSynchronize(s->copy_stream);
+    cudaStreamSynchronize(s->merge_stream);
     delete s;
     return GFB_OK;
 }
@@ -2542,6 +2554,9 @@ gfb_status gfb_advance_timed(gfb_solver* s, int32_t n_steps, double* ms) {
     gfb_status st = GFB_OK;
     if (cudaEventRecord(e0, s->stream) != cudaSuccess) st = fail(GFB_ERR_CUDA, "cudaEventRecord failed");
     if (!st) st = all_steps(s, n_steps);
+    // the merges of the snapshots among these steps are part of their time
+    for (auto e : s->merge_evt)
+        if (!st && cudaStreamWaitEvent(s->stream, e, 0) != cudaSuccess) st = fail(GFB_ERR_CUDA, "cudaStreamWaitEvent failed");
     float t = 0.0f;
     if (!st && (cudaEventRecord(e1, s->stream) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
                 cudaEventElapsedTime(&t, e0, e1) != cudaSuccess))
@@ -2654,6 +2669,8 @@ gfb_status gfb_synchronize(gfb_solver* s) {
     if (!s) return fail(GFB_ERR_INVALID, "solver is NULL");
     CU(cudaSetDevice(s->device));
     CU(cudaStreamSynchronize(s->stream));
+    CU(cudaStreamSynchronize(s->merge_stream));
+    CU(cudaStreamSynchronize(s->copy_stream));
     return check_kernel_err(s);
 }
 
@@ -2921,15 +2938,25 @@ gfb_status read_record_t(gfb_solver* s, int32_t field, int32_t* step, Out* strai
         unpack_record(s, raw, field, strain, u, v, a);
     }
     {
-        std::lock_guard<std::mutex> lk(s->rec_mu);
-        snap->readers--;
+        std::unique_lock<std::mutex> lk(s->rec_mu);
         if (!st) {
             if (!snap->read_mask[field]) {
                 snap->read_mask[field] = 1;
                 snap->fields_read++;
             }
-            if (release || snap->fields_read == s->nfld) snap->done = true;
+            if (release || snap->fields_read == s->nfld) {
+                // with its last read nothing of the snapshot stays queued: its
+                // merged part, if nobody has read it, has arrived too (the
+                // slot is this reader's until readers goes down)
+                if (slot >= 0) {
+                    lk.unlock();
+                    if (cudaEventSynchronize(s->copy_evt[slot]) != cudaSuccess) st = fail(GFB_ERR_CUDA, "snapshot copy failed");
+                    lk.lock();
+                }
+                if (!st) snap->done = true;
+            }
         }
+        snap->readers--;
         while (!s->pending.empty() && s->pending.front().done && s->pending.front().readers == 0)
             s->pending.pop_front();
     }
@@ -3146,6 +3173,17 @@ gfb_status solver_set_layer(gfb_solver* s, Layer* layer) {
 }
 
 }  // namespace gfb
+
+extern "C" gfb_status gfb_work_queued(gfb_solver* s, int32_t* queued) {
+    if (!s || !queued) return fail(GFB_ERR_INVALID, "NULL argument");
+    *queued = 0;
+    for (cudaStream_t q : {s->stream, s->merge_stream, s->copy_stream}) {
+        const cudaError_t e = cudaStreamQuery(q);
+        if (e == cudaErrorNotReady) *queued = 1;
+        else CU(e);
+    }
+    return GFB_OK;
+}
 
 extern "C" gfb_status gfb_inject_kernel_error(gfb_solver* s) {
     if (!s) return fail(GFB_ERR_INVALID, "solver is NULL");

@@ -224,15 +224,17 @@ gfb_status gfb_advance(gfb_solver* solver, int32_t n_steps);
 
 /*
  * gfb_advance with one pair of CUDA events on the solver's stream around the
- * n_steps steps; adds their device milliseconds to *ms and synchronises.
+ * n_steps steps and the recording and merging of their snapshots; adds their
+ * device milliseconds to *ms and synchronises with them.  The snapshots'
+ * copies to the host are not part of the time.
  */
 gfb_status gfb_advance_timed(gfb_solver* solver, int32_t n_steps, double* ms);
 
 /*
  * gfb_advance with CUDA events on the solver's stream around each phase of
  * every step; adds the device milliseconds spent in the element/assembly
- * launches, the node update and the snapshot kernel to the three outputs
- * (any may be NULL).  Synchronises before returning.  The reference times
+ * launches, the node update and the snapshot kernels (recording and merge) to
+ * the three outputs (any may be NULL).  Synchronises before returning.  The reference times
  * its loop with std::chrono only (solver.cpp:342-348, 729-732).
  */
 gfb_status gfb_advance_profiled(gfb_solver* solver, int32_t n_steps, double* ms_element,
@@ -282,7 +284,7 @@ gfb_status gfb_set_force_refresh(gfb_solver* solver, int32_t steps);
  * update); GFB_ERR_INVALID for a variant outside [-1, n_elem_variants). */
 gfb_status gfb_select_element_kernel(gfb_solver* solver, int32_t variant);
 
-/* Wait for all queued work. */
+/* Wait for all queued work: steps, and the snapshots' merges and copies. */
 gfb_status gfb_synchronize(gfb_solver* solver);
 
 /* Next solver step index (number of steps taken since step 0). */

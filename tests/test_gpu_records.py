@@ -106,3 +106,35 @@ def test_mesh_check_reports_first_offending_entry(prob):
     bad["ibool"] = ib2
     with pytest.raises(gfb.GfbError, match=r"ibool\[%d\]=-1 outside" % (5 * nn + 10)):
         gfb.Solver(bad, dirs=[0], precision=gfb.FP32)
+
+
+def queued(s):
+    import ctypes as C
+
+    fn = s.lib.gfb_work_queued
+    fn.restype, fn.argtypes = C.c_int, [C.c_void_p, C.POINTER(C.c_int32)]
+    q = C.c_int32(-1)
+    assert fn(s.h, C.byref(q)) == 0
+    return q.value
+
+
+@pytest.mark.parametrize("prec", [gfb.FP64, gfb.FP32])
+def test_nothing_stays_queued(prec):
+    """Every cell records and every step is a snapshot step, so the merge of a
+    snapshot and the merged part's copy end well after the records' copy:
+    neither a synchronisation, nor a run that has read its snapshots, nor a
+    released snapshot leaves them queued."""
+    spec = mesh.MeshSpec(nx=16, ny=16, nz=10, dx=500.0, dy=500.0, dz=500.0, order=4, seed=2)
+    prob = mesh.build_problem(spec, mesh.seeded_layers(2, 10 * 500.0), np.asarray([4100.0, 4200.0, 800.0]), nsteps=40,
+                              snapshot_stride=1, record_depth_max_m=500.0, with_cpml=False)
+    prob["recording"] = {"rec_cell_local": np.arange(prob["n_cell"], dtype=np.int32)}
+    s = gfb.Solver(prob, dirs=[0, 1], precision=prec, record_slots=4)
+    s.advance(2)
+    s.synchronize()
+    assert queued(s) == 0
+    s.run(3)
+    assert s.pending() == 0 and queued(s) == 0
+    s.advance(1)
+    s.read_record(0, release=True, out={})
+    assert queued(s) == 0
+    s.close()
