@@ -241,6 +241,11 @@ struct gfb_solver {
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;   // snapshots to the host
     cudaStream_t merge_stream = nullptr;  // their merge per recording node
+    // the C-PML node pass runs beside the plain one: elem_evt, the element
+    // phase it follows; pml_evt, its end, which the next step waits for
+    cudaStream_t node_stream = nullptr;
+    cudaEvent_t elem_evt = nullptr, pml_evt = nullptr;
+    bool capturing = false;
     int prec = GFB_FP64;
     int ng = 0, nn = 0, nfld = 1, F = 3;
     int n_cell = 0, n_node = 0;
@@ -396,6 +401,9 @@ struct gfb_solver {
         if (stream) cudaStreamDestroy(stream);
         if (copy_stream) cudaStreamDestroy(copy_stream);
         if (merge_stream) cudaStreamDestroy(merge_stream);
+        if (elem_evt) cudaEventDestroy(elem_evt);
+        if (pml_evt) cudaEventDestroy(pml_evt);
+        if (node_stream) cudaStreamDestroy(node_stream);
     }
 };
 
@@ -542,27 +550,63 @@ int grid_for(long long n, int threads) {
 }
 
 // Launch a kernel of the step's programmatic chain (gfb::pdl_wait); early:
-// it may start before the kernel before it has completed.
+// it may start before the kernel before it has completed.  lets: an event that
+// lets a kernel on another stream start as early as the next one on this
+// stream may (nullptr: none); that kernel's pdl_wait() is for this one.
 template <typename... Params, typename... Args>
-cudaError_t launch_chained(bool early, void (*fn)(Params...), int blocks, int threads, size_t smem, cudaStream_t stream,
-                           Args&&... args) {
+cudaError_t launch_forked(bool early, cudaEvent_t lets, void (*fn)(Params...), int blocks, int threads, size_t smem,
+                          cudaStream_t stream, Args&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = early ? 1 : 0;
+    cudaLaunchAttribute at[2] = {};
+    if (early) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (lets) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticEvent;
+        at[cfg.numAttrs].val.programmaticEvent.event = lets;
+        at[cfg.numAttrs].val.programmaticEvent.flags = 0;
+        at[cfg.numAttrs++].val.programmaticEvent.triggerAtBlockStart = 0;
+    }
+    cfg.attrs = at;
     return cudaLaunchKernelEx(&cfg, fn, Params(args)...);
+}
+template <typename... Params, typename... Args>
+cudaError_t launch_chained(bool early, void (*fn)(Params...), int blocks, int threads, size_t smem, cudaStream_t stream,
+                           Args&&... args) {
+    return launch_forked(early, nullptr, fn, blocks, threads, smem, stream, args...);
 }
 
 // The gather kernel runs unless the fused node update,
 // GFB_FLAG_POINT_KERNEL or another FP32 variant asks for assembly by colour.
 bool use_gather(const gfb_solver* s) {
     return s->gather_ok && !s->fuse && !s->point_kernel && (s->prec == GFB_FP64 || s->col_variant == 0);
+}
+
+// Whether the node passes may start before the element kernel has completed.
+// They then find the SM set up for it: most of the L1 as shared memory.  Where
+// that is 200 KB and more (line kernel at ngll 5 and 6, FP64) a pass then misses
+// the L1 it reads its contributions through: 498 against 480 us per step (FP64,
+// 40 x 40 x 20 cells), 187 / 177 (ngll 6, 22 x 21 x 13), 178 / 166 (one FP32
+// wavefield, 40 x 40 x 20).  Beside the plane kernel and at ngll 3 it gains:
+// 400 / 405 (40 x 40 x 20 x 3), 68 / 72 (20 x 20 x 10 x 3), 72 / 81 (six small
+// models), 69.5 / 72.5 (ngll 3).
+bool node_early(const gfb_solver* s) {
+    return use_gather(s) && !s->layer && s->prec == GFB_FP32 && !(s->has_cpml && !s->node_pml) &&
+           (s->plane_blocks > 0 || s->ng == 3);
+}
+
+// Both node passes of a step (plain nodes, node-form C-PML nodes) have nodes.
+bool two_node_passes(const gfb_solver* s) { return s->node_pml && s->n_pml_node > 0 && s->n_pml_node < s->n_node; }
+
+// The event by which a captured element kernel lets the C-PML node pass start
+// early.  Outside a graph that pass follows a plain event record.
+cudaEvent_t elem_lets(const gfb_solver* s) {
+    return s->capturing && node_early(s) && two_node_passes(s) ? s->elem_evt : nullptr;
 }
 
 // Whether the assembled force outlives the step: the stored force of the
@@ -791,7 +835,7 @@ gfb_status launch_gather_t(gfb_solver* s) {
             A.nfld_item = 2 * pairs <= s->plane_blocks * PS::WARPS ? 3 : s->nfld;
             const int n = pairs * (s->nfld / A.nfld_item);
             const int blocks = std::max(1, std::min((n + PS::WARPS - 1) / PS::WARPS, s->plane_blocks));
-            CU(launch_chained(true, gfb::elem_plane_kernel, blocks, PS::THREADS, PS::SMEM, s->stream, A));
+            CU(launch_forked(true, elem_lets(s), gfb::elem_plane_kernel, blocks, PS::THREADS, PS::SMEM, s->stream, A));
             s->launches++;
             return GFB_OK;
         }
@@ -800,7 +844,7 @@ gfb_status launch_gather_t(gfb_solver* s) {
     A.nfld_item = 2 * groups <= s->gather_blocks * S::GROUPS ? 1 : s->nfld;
     const int items = groups * (s->nfld / A.nfld_item);
     const int blocks = std::max(1, std::min((items + S::GROUPS - 1) / S::GROUPS, s->gather_blocks));
-    CU(launch_chained(true, gfb::elem_gather_kernel<Real, NG>, blocks, S::THREADS, S::SMEM, s->stream, A));
+    CU(launch_forked(true, elem_lets(s), gfb::elem_gather_kernel<Real, NG>, blocks, S::THREADS, S::SMEM, s->stream, A));
     s->launches++;
     if (s->has_cpml && !s->node_pml && s->n_pml > 0) {
         gfb::CellPmlArgs<Real> P;
@@ -817,15 +861,16 @@ gfb_status launch_gather_t(gfb_solver* s) {
         P.v = s->v;
         P.a = static_cast<const Real*>(s->a);
         P.mc = s->d_mc;
-        // early beside an element kernel that leaves room on the SMs: 18.4
-        // against 20.8 us per step (11 x 9 x 7 cells); otherwise it would run
+        // early beside an element kernel that leaves room on the SMs: 17.9
+        // against 18.3 us per step (11 x 9 x 7 cells); otherwise it would run
         // with the little L1 the element kernel leaves (486 / 391 us,
         // 40 x 40 x 20)
         constexpr int threads = gfb::cell_pml_threads(S::NN);
         const int cells = std::min(s->n_pml, s->gather_sm * (gfb::kCellPmlThreads / threads));
         P.multi = s->n_model > 1;
-        P.early = 2 * blocks <= s->gather_blocks;
-        CU(launch_chained(P.early, gfb::cell_pml_kernel<Real, NG>, cells, threads, 0, s->stream, P));
+        const bool early = 2 * blocks <= s->gather_blocks;
+        auto* fn = early ? gfb::cell_pml_kernel<Real, NG, true> : gfb::cell_pml_kernel<Real, NG, false>;
+        CU(launch_chained(early, fn, cells, threads, 0, s->stream, P));
         s->launches++;
     }
     return GFB_OK;
@@ -1052,29 +1097,32 @@ gfb_status launch_node_m(gfb_solver* s) {
     node_args(s, A, P);
     // node-form C-PML nodes are device nodes [0, n_pml_node)
     const long long g0 = s->node_pml ? s->n_pml_node : 0;
-    const bool plain = g0 < s->n_node;
-    if (plain) {
+    const bool early = node_early(s), two = two_node_passes(s);
+    if (two && !elem_lets(s)) CU(cudaEventRecord(s->elem_evt, s->stream));
+    if (g0 < s->n_node) {
         auto* fn = gfb::node_update_kernel<Real, NFLD, MULTI, false>;
         if constexpr (std::is_same<Real, float>::value)
             if (A.half_v) fn = gfb::node_update_kernel<Real, NFLD, MULTI, true>;
-        // Starting early the pass finds the SM set up for the element kernel:
-        // most of the L1 as shared memory.  Where that is 200 KB and more
-        // (line kernel at ngll 5 and 6, FP64) the pass then misses the L1 it
-        // reads its contributions through: 498 against 480 us per step (FP64,
-        // 40 x 40 x 20), 187 / 177 (ngll 6, 22 x 21 x 13).  Beside the plane
-        // kernel and at ngll 3 it gains: 400 / 405 (40 x 40 x 20 x 3), 68 / 72
-        // (20 x 20 x 10 x 3), 72 / 81 (six small models), 69.5 / 72.5 (ngll 3).
-        const bool early = use_gather(s) && s->prec == GFB_FP32 && !(s->has_cpml && !s->node_pml) &&
-                           (s->plane_blocks > 0 || s->ng == 3);
         CU(launch_chained(early, fn, node_grid(s->n_node - g0, gfb::node_blocks_per_sm<Real>(false)), gfb::kNodeThreads, 0,
                           s->stream, A, P, g0));
         s->launches++;
     }
     if constexpr (std::is_same<Real, float>::value) {
         if (g0 > 0) {
-            CU(launch_chained(true, gfb::node_pml_kernel<NFLD, MULTI>, node_grid(g0, gfb::node_blocks_per_sm<float>(true)),
-                              gfb::kNodeThreads, 0, s->stream, A, P, !plain));
+            // beside the plain pass: its blocks take the SMs that the plain
+            // pass leaves.  One after the other the two cost 445 against 428
+            // us per step (32 x 32 x 16 x 6), 407 / 399 (40 x 40 x 20 x 3), 78.5 /
+            // 73 (20 x 20 x 10 x 3), 82 / 71 (six small models); in one launch,
+            // at the C-PML pass's registers, 433 / 399 (40 x 40 x 20 x 3).
+            cudaStream_t q = two ? s->node_stream : s->stream;
+            if (two) CU(cudaStreamWaitEvent(q, s->elem_evt, 0));
+            CU(launch_chained(two ? elem_lets(s) != nullptr : early, gfb::node_pml_kernel<NFLD, MULTI>,
+                              node_grid(g0, gfb::node_blocks_per_sm<float>(true)), gfb::kNodeThreads, 0, q, A, P));
             s->launches++;
+            if (two) {
+                CU(cudaEventRecord(s->pml_evt, q));
+                CU(cudaStreamWaitEvent(s->stream, s->pml_evt, 0));
+            }
         }
     }
     return GFB_OK;
@@ -2005,8 +2053,10 @@ constexpr int kGraphSteps = 5;
 gfb_status capture_steps(gfb_solver* s, int n, cudaGraphExec_t* exec) {
     const long long l0 = s->launches;
     CU(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+    s->capturing = true;
     gfb_status st = GFB_OK;
     for (int k = 0; k < n && !st; ++k) st = step_body(s, nullptr);
+    s->capturing = false;
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(s->stream, &g);
     s->graph_launches = (s->launches - l0) / n;
@@ -2256,6 +2306,9 @@ gfb_status create_impl(const gfb_mesh* m, const gfb_config* c, const gfb_source*
     CU(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     CU(cudaStreamCreateWithFlags(&s->copy_stream, cudaStreamNonBlocking));
     CU(cudaStreamCreateWithFlags(&s->merge_stream, cudaStreamNonBlocking));
+    CU(cudaStreamCreateWithFlags(&s->node_stream, cudaStreamNonBlocking));
+    CU(cudaEventCreateWithFlags(&s->elem_evt, cudaEventDisableTiming));
+    CU(cudaEventCreateWithFlags(&s->pml_evt, cudaEventDisableTiming));
     CU(cudaHostAlloc(reinterpret_cast<void**>(&s->kernel_err), sizeof(unsigned), cudaHostAllocMapped));
     *s->kernel_err = 0;
     CU(cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->d_kernel_err), s->kernel_err, 0));
