@@ -57,8 +57,8 @@ __host__ __device__ constexpr int ib_row_words(int nn) { return (nn + 1 + 3) / 4
 // Geometry rows of the time loop, [cell][geo_row]: dxi_dx (9 x NN), then
 // lambda and mu times det J w_i w_j w_k (so the stress they give is already
 // the flux's and the weight costs no load or multiply), padded to whole
-// 16-byte copies.  Where mu <= 0 both are 0: the point adds nothing
-// (element_cpu.cpp:42-43).
+// 16-byte copies.  Where mu <= 0 both are 0: the point adds nothing, whatever
+// its other values are (element_cpu.cpp:42-43).
 template <typename Real>
 __host__ __device__ constexpr int geo_row(int nn) {
     return (11 * nn * (int)sizeof(Real) + 15) / 16 * 16 / (int)sizeof(Real);
@@ -875,6 +875,11 @@ __global__ void __launch_bounds__(PipeShape<Real, NG, NFLD>::THREADS, (sizeof(Re
             lam = geo[9 * NN + p];
             mu = geo[10 * NN + p];
         }
+        const bool on = lam != Real(0) || mu != Real(0);  // else the point adds nothing
+        if (!on) {
+#pragma unroll
+            for (int q = 0; q < 9; ++q) dd[q] = Real(0);
+        }
         __syncthreads();  // geometry stage now takes this group's old force vectors
         if (active && !(gword & first_bit)) {
             const uint32_t g = gword & kNodeMask;
@@ -898,7 +903,7 @@ __global__ void __launch_bounds__(PipeShape<Real, NG, NFLD>::THREADS, (sizeof(Re
         for (int d = 0; d < NFLD; ++d)
 #pragma unroll
             for (int q = 0; q < 6; ++q) st[d][q] = Real(0);
-        if (active) {
+        if (active && on) {
 #pragma unroll
             for (int d = 0; d < NFLD; ++d) {
                 Real gx[3] = {0, 0, 0}, gy[3] = {0, 0, 0}, gz[3] = {0, 0, 0};
@@ -1111,7 +1116,7 @@ struct ColArgs {
     const int* live_end;           // [colour] end of the stepping cells (several models), or null
     int colour;
     const uint32_t* ibool_padded;  // [cell][ib_row_words(NN)]: node words, model index
-    const float* geom;             // [cell][12][NN]
+    const float* geom;             // [cell][geo_row]
     const float* ut;               // [node][NFLD][4]
     float* force;                  // [node][NFLD][4]
     const float* dmat;             // [NG*NG]
@@ -1360,16 +1365,17 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_>::THREADS, ColShape<NG
             const float st3 = mu * (gr[0][1] + gr[1][0]);
             const float st4 = mu * (gr[0][2] + gr[2][0]);
             const float st5 = mu * (gr[1][2] + gr[2][1]);
-            // flux along axis a: sigma . (dd[a], dd[3+a], dd[6+a])
-            fx0[i] = (st0 * dd[0] + st3 * dd[3] + st4 * dd[6]);
-            fx1[i] = (st3 * dd[0] + st1 * dd[3] + st5 * dd[6]);
-            fx2[i] = (st4 * dd[0] + st5 * dd[3] + st2 * dd[6]);
-            const float e0 = (st0 * dd[1] + st3 * dd[4] + st4 * dd[7]);
-            const float e1 = (st3 * dd[1] + st1 * dd[4] + st5 * dd[7]);
-            const float e2 = (st4 * dd[1] + st5 * dd[4] + st2 * dd[7]);
-            const float z0 = (st0 * dd[2] + st3 * dd[5] + st4 * dd[8]);
-            const float z1 = (st3 * dd[2] + st1 * dd[5] + st5 * dd[8]);
-            const float z2 = (st4 * dd[2] + st5 * dd[5] + st2 * dd[8]);
+            // flux along axis a: sigma . (dd[a], dd[3+a], dd[6+a]); 0 where the
+            // point adds nothing
+            const bool on = lam != 0.f || mu != 0.f;
+            auto flux = [&](float a, float b, float c, int x) {
+                return on ? a * dd[x] + b * dd[3 + x] + c * dd[6 + x] : 0.f;
+            };
+            fx0[i] = flux(st0, st3, st4, 0);
+            fx1[i] = flux(st3, st1, st5, 0);
+            fx2[i] = flux(st4, st5, st2, 0);
+            const float e0 = flux(st0, st3, st4, 1), e1 = flux(st3, st1, st5, 1), e2 = flux(st4, st5, st2, 1);
+            const float z0 = flux(st0, st3, st4, 2), z1 = flux(st3, st1, st5, 2), z2 = flux(st4, st5, st2, 2);
             fe[0 * GR * SP + ubase + i * NG2] = e0;
             fe[1 * GR * SP + ubase + i * NG2] = e1;
             fe[2 * GR * SP + ubase + i * NG2] = e2;
@@ -1650,11 +1656,19 @@ template <typename Real>
 __device__ __forceinline__ void vstore(Real* p, int, Real x) { p[0] = x; }
 __device__ __forceinline__ void vstore(float* p, int step, float2 x) { p[0] = x.x, p[step] = x.y; }
 __device__ __forceinline__ float2 vpair(float a, float b) { return make_float2(a, b); }
+// x where a or b is not 0, else 0 (also if x is not a number)
+template <typename Real>
+__device__ __forceinline__ Real vwhere(Real a, Real b, Real x) { return a != Real(0) || b != Real(0) ? x : Real(0); }
+__device__ __forceinline__ float2 vwhere(float2 a, float2 b, float2 x) {
+    return make_float2(vwhere(a.x, b.x, x.x), vwhere(a.y, b.y, x.y));
+}
 
 // Gradient to fluxes at one point (V = Real) or, in FP32, two (float2) whose
 // geometry lies `step` apart: g[c][b] the derivatives of component c along
-// reference axis b; fl[b][c] the flux along axis b.
-template <typename Real, typename V>
+// reference axis b; fl[b][c] the flux along axis b.  OFF: 0 at the points that add
+// nothing (lambda and mu stored as 0), where a collapsed cell's infinite dxi_dx
+// would otherwise make 0 * inf of it.
+template <bool OFF, typename Real, typename V>
 __device__ __forceinline__ void point_fluxes(const Real* geo, int nn, int step, const V (&g)[3][3], V (&fl)[3][3]) {
     V dd[9], lam, mu, gr[3][3];
 #pragma unroll
@@ -1678,8 +1692,10 @@ __device__ __forceinline__ void point_fluxes(const Real* geo, int nn, int step, 
 #pragma unroll
     for (int b = 0; b < 3; ++b)
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
+        for (int c = 0; c < 3; ++c) {
             fl[b][c] = vfma(st[c][2], dd[6 + b], vfma(st[c][1], dd[3 + b], vmul(st[c][0], dd[b])));
+            if (OFF) fl[b][c] = vwhere(lam, mu, fl[b][c]);
+        }
 }
 
 template <typename Real, int NG>
@@ -1869,7 +1885,7 @@ __global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Re
                         vload(xe + c * CELLS * SE + own_e + i * PE, PE, g[c][1]);
                         vload(xz + c * CELLS * SZ + own_z + i * PZ, PZ, g[c][2]);
                     }
-                    point_fluxes(geo + i * NG2 + col, NN, NG2, g, fl);
+                    point_fluxes<true>(geo + i * NG2 + col, NN, NG2, g, fl);
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
                         if constexpr (sizeof(V) > sizeof(Real)) {
@@ -1980,7 +1996,9 @@ __global__ void __launch_bounds__(GatherShape<Real, NG>::THREADS, GatherShape<Re
 // at 135 q + 27 i + 5 j + k: a warp's own-point and line accesses fall in
 // distinct banks.  Node words come by bulk copy one item ahead, the geometry
 // as soon as the last one has been read; the contributions leave as one bulk
-// copy per cell, collected in the exchange array.
+// copy per cell, collected in the exchange array.  OFF: the mesh has points with
+// mu <= 0; the selects at every point cost 1.2 % of a step (404 against 399 us,
+// same cells), which the line kernel hides.
 // ---------------------------------------------------------------------------
 struct PlaneShape {
     static constexpr int NG = 5, NN = 125, NG2 = 25, CELLS = 2, WARPS = 4, THREADS = 32 * WARPS;
@@ -1995,6 +2013,7 @@ struct PlaneShape {
     static_assert(CELLS * CHUNK_W * 4 <= XCH_B, "the contributions fit in the exchange array");
 };
 
+template <bool OFF>
 static __global__ void __launch_bounds__(PlaneShape::THREADS, 2)
     elem_plane_kernel(const __grid_constant__ GatherArgs<float> A) {
     using S = PlaneShape;
@@ -2171,7 +2190,7 @@ static __global__ void __launch_bounds__(PlaneShape::THREADS, 2)
                             for (int s = 1; s < NG; ++s) g[c][1] = vfma(A.D2[j * NG + s], u2[c][s][h], g[c][1]);
                             g[c][2] = make_float2(dz(c, k), dz(c, k + 1));
                         }
-                        point_fluxes(geo + p, NN, 1, g, fl);
+                        point_fluxes<OFF>(geo + p, NN, 1, g, fl);
 #pragma unroll
                         for (int c = 0; c < 3; ++c) {
                             vstore(own + c * S::SC + p, 1, fl[0][c]);
@@ -2192,7 +2211,7 @@ static __global__ void __launch_bounds__(PlaneShape::THREADS, 2)
                             for (int s = 1; s < NG; ++s) g[c][1] = vfma(A.D[j * NG + s], u1[c][s], g[c][1]);
                             g[c][2] = dz(c, 4);
                         }
-                        point_fluxes(geo + p, NN, 1, g, fl);
+                        point_fluxes<OFF>(geo + p, NN, 1, g, fl);
 #pragma unroll
                         for (int c = 0; c < 3; ++c) {
                             own[c * S::SC + p] = fl[0][c];

@@ -288,6 +288,7 @@ struct gfb_solver {
     int col_epb = 0;                   // cells per group of the variant in use
     bool point_kernel = false;         // thread-per-point element kernel
     void* geom = nullptr;
+    bool off_points = false;           // some points have mu <= 0 and add nothing
     void* dmat = nullptr;
     double dmat_host[36] = {};         // D of the line kernels' parameters
     double *u = nullptr, *v = nullptr;
@@ -835,7 +836,8 @@ gfb_status launch_gather_t(gfb_solver* s) {
             A.nfld_item = 2 * pairs <= s->plane_blocks * PS::WARPS ? 3 : s->nfld;
             const int n = pairs * (s->nfld / A.nfld_item);
             const int blocks = std::max(1, std::min((n + PS::WARPS - 1) / PS::WARPS, s->plane_blocks));
-            CU(launch_forked(true, elem_lets(s), gfb::elem_plane_kernel, blocks, PS::THREADS, PS::SMEM, s->stream, A));
+            auto* fn = s->off_points ? gfb::elem_plane_kernel<true> : gfb::elem_plane_kernel<false>;
+            CU(launch_forked(true, elem_lets(s), fn, blocks, PS::THREADS, PS::SMEM, s->stream, A));
             s->launches++;
             return GFB_OK;
         }
@@ -891,8 +893,9 @@ gfb_status gather_grid_t(gfb_solver* s) {
     if constexpr (std::is_same<Real, float>::value && NG == 5) {
         if (s->nfld % 3 == 0 && !(s->has_cpml && !s->node_pml)) {
             using PS = gfb::PlaneShape;
-            CU(cudaFuncSetAttribute(gfb::elem_plane_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PS::SMEM));
-            CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gfb::elem_plane_kernel, PS::THREADS, PS::SMEM));
+            auto* plane = s->off_points ? gfb::elem_plane_kernel<true> : gfb::elem_plane_kernel<false>;
+            CU(cudaFuncSetAttribute(plane, cudaFuncAttributeMaxDynamicSharedMemorySize, PS::SMEM));
+            CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, plane, PS::THREADS, PS::SMEM));
             s->plane_blocks = per_sm * n_sm;
         }
     }
@@ -1645,6 +1648,7 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
     {
         const int row = gfb::geo_row<Real>(nn);
         Real* dg = nullptr;
+        std::atomic<bool> off(false);
         if ((st = s->alloc(&dg, (size_t)n_cell * row))) return st;
         st = staged_upload(s, dg, (size_t)row * sizeof(Real), n_cell,
                            [&](long long e0, long long e1, unsigned char* out) {
@@ -1652,6 +1656,7 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
                 for (long long i = a0; i < a1; ++i) {
                     const long long e = e0 + i;
                     Real* o = reinterpret_cast<Real*>(out) + i * row;
+                    bool cell_off = false;
                     for (int p = 0; p < nn; ++p) {
                         const long long q = e * nn + p;
                         for (int f = 0; f < 9; ++f) o[f * nn + p] = (Real)m->dxi_dx[q * 9 + f];
@@ -1661,13 +1666,16 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
                         const double f = m->mu[q] > 0.0 ? m->jacobian[q] * w[i0] * w[j] * w[k] : 0.0;
                         o[9 * nn + p] = f != 0.0 ? (Real)(m->lambda_[q] * f) : Real(0);
                         o[10 * nn + p] = f != 0.0 ? (Real)(m->mu[q] * f) : Real(0);
+                        cell_off |= !(m->mu[q] > 0.0);
                     }
+                    if (cell_off) off.store(true);
                     for (int x = 11 * nn; x < row; ++x) o[x] = Real(0);
                 }
             }, 256);
         });
         if (st) return st;
         s->geom = dg;
+        s->off_points = off.load();
     }
     clk.mark("geometry upload");
     {
