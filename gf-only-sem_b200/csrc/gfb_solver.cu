@@ -902,7 +902,7 @@ gfb_status gather_grid_t(gfb_solver* s) {
     return GFB_OK;
 }
 
-int gather_cells(int ng) {
+int gather_cells(int ng) {  // in both precisions
     return ng == 3 ? gfb::GatherShape<float, 3>::CELLS
                    : (ng == 4 ? gfb::GatherShape<float, 4>::CELLS
                               : (ng == 5 ? gfb::GatherShape<float, 5>::CELLS : gfb::GatherShape<float, 6>::CELLS));
@@ -2680,9 +2680,10 @@ gfb_status gfb_get_info(const gfb_solver* s, gfb_info* info) {
     info->kernel_launches = s->launches;
     info->n_pml_node = s->node_pml ? s->n_pml_node : 0;
     const bool gather = use_gather(s), col = use_col_kernel(s);
-    info->elem_blocks = gather ? s->gather_blocks : (col ? s->col_blocks : s->pipe_blocks);
+    const bool plane = gather && s->plane_blocks > 0;
+    info->elem_blocks = plane ? s->plane_blocks : (gather ? s->gather_blocks : (col ? s->col_blocks : s->pipe_blocks));
     info->elem_kernel = gather || col ? 1 : 0;
-    info->cells_per_group = gather ? gather_cells(s->ng) : (col ? s->col_epb : 0);
+    info->cells_per_group = plane ? gfb::PlaneShape::CELLS : (gather ? gather_cells(s->ng) : (col ? s->col_epb : 0));
     info->force_refresh = s->refresh;
     info->half_v = s->half_v ? 1 : 0;
     info->elem_variant = col_kernel_eligible(s) && !s->point_kernel ? s->col_variant : -1;

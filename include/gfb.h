@@ -99,8 +99,8 @@ typedef struct gfb_config {
  * accesses cost far more L1 transactions than the contiguous node pass. */
 #define GFB_FLAG_FUSED_NODE 4
 /* Run the thread-per-GLL-point element kernel with assembly by colour instead
- * of the default thread-per-xi-line kernel (same arithmetic, different
- * summation order; for comparisons). */
+ * of the default kernel, which has a thread per xi-line or xi-plane (same
+ * arithmetic, different summation order; for comparisons). */
 #define GFB_FLAG_POINT_KERNEL 8
 /* Launch each step's kernels one by one instead of replaying the step as a
  * captured CUDA graph. */
@@ -255,8 +255,10 @@ typedef struct gfb_info {
     int64_t kernel_launches; /* kernels launched by this solver so far                     */
     int32_t n_pml_node;      /* global nodes carrying C-PML state (0: per-cell form)        */
     int32_t elem_blocks;     /* blocks in the persistent grid of the element kernel in use  */
-    int32_t elem_kernel;     /* 1: thread-per-xi-line kernel, 0: thread-per-point kernel    */
-    int32_t cells_per_group; /* cells a thread-per-xi-line kernel takes at a time (0 otherwise) */
+    int32_t elem_kernel;     /* 1: thread per xi-line or, for FP32 wavefields in threes at ngll 5,
+                                per xi-plane; 0: thread per point                              */
+    int32_t cells_per_group; /* cells a warp or group of threads of that kernel takes at a time
+                                (0 for thread per point)                                       */
     int32_t force_refresh;   /* steps between full element-force evaluations (1: every step) */
     int32_t half_v;          /* 1: plain nodes keep the half-step velocity, no acceleration */
     int32_t elem_variant;    /* FP32 element kernel in use: -1 thread-per-point by colour; 0 the
