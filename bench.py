@@ -448,7 +448,7 @@ def elem_bytes_per_step(prob, info, n_field, prec):
     F = 3 * n_field
     geom = P * 11 * sr + P * 4                      # geometry + ibool
     gather = G * F * sr                              # predicted displacement (or its increment)
-    if not by_colour(info, prec):                    # contributions
+    if not info["by_colour"]:                        # contributions
         force = P * F * sr
     elif info.get("force_refresh", 1) > 1:           # force by increments: every touch reads and writes
         force = P * F * sr * 2
@@ -459,12 +459,6 @@ def elem_bytes_per_step(prob, info, n_field, prec):
         Ppml = info["n_pml_cell"] * nn
         pml = Ppml * (7 * sr + F * sr * 2 + F * sr * 2 + F * 16 + F * sr)
     return geom + gather + force + pml
-
-
-def by_colour(info, prec):
-    """Whether the element phase assembles by colour (FP32 kernels selected
-    instead of the default one)."""
-    return prec == 1 and info.get("elem_variant", 0) != 0
 
 
 def node_bytes_per_step(prob, info, n_field, prec):
@@ -482,7 +476,7 @@ def node_bytes_per_step(prob, info, n_field, prec):
     state = 16 + 8 if info.get("half_v") else 16 + 16 + 2 * sr   # u (+ w | v, a) read and written
     mass = 4 if prec == 1 else 8
     base = n_plain * (F * (state + 2 * sr) + mass) + n_pml * (F * (32 + 4 * sr) + mass)
-    if not by_colour(info, prec):                    # contributions and touches read, the force kept (FP32)
+    if not info["by_colour"]:                        # contributions and touches read, the force kept (FP32)
         base += prob["n_cell"] * 125 * F * sr + prob["n_node"] * (16 + (F * sr if prec == 1 else -F * sr))
     if n_pml > 0:                                    # node-form C-PML in this kernel
         n_live, live = node_pml_live_axes(prob)
@@ -509,7 +503,7 @@ def fp64_plain_sample(prob, device, args, fp32_value_per_gpu, peak):
 
     s = gfb.Solver(prob, dirs=[0], precision=gfb.FP64, device=device, record_slots=8,
                    flags=gfb.FLAG_RECORD_F32 if args.record_f32 else 0)
-    info = s.info()
+    info = {**s.info(), "by_colour": s.by_colour}
     s.advance(args.warmup)
     s.drain()
     s.synchronize()
@@ -735,8 +729,10 @@ def run_gfb(args):
     t_gen = time.perf_counter() - t_gen
     flags = (gfb.FLAG_RECORD_F32 if args.record_f32 else 0) | (gfb.FLAG_POINT_KERNEL if args.point_kernel else 0)
     s = gfb.Solver(prob, dirs=dirs, precision=prec, device=device, record_slots=8, flags=flags)
-    info = s.info()
-    if args.point_kernel:
+    info = {**s.info(), "by_colour": s.by_colour}
+    if info["by_colour"] and prec == gfb.FP32 and not args.point_kernel:
+        kname = f"elem_col_kernel<5,{len(dirs)}> (by colour)"
+    elif info["by_colour"]:
         kname = f"elem_pipe_kernel<{'float' if prec == gfb.FP32 else 'double'},5,{len(dirs)}> (by colour)"
     elif prec == gfb.FP32 and len(dirs) == 3:
         kname = "elem_plane_kernel"

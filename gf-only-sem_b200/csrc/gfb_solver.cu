@@ -1421,7 +1421,8 @@ gfb_status build_gather(gfb_solver* s, const gfb_mesh* m, const NodeBuckets& nb,
     auto unit_of = [&](long long q) -> uint32_t { return (uint32_t)((size_t)(q / nn) * row_u + (size_t)(q % nn) * fc); };
     // the fused node update keeps to assembly by colour; so does the
     // thread-per-point kernel where no other can be selected later
-    if (units >= (size_t)0x7fffffff || s->fuse || (s->point_kernel && s->prec == GFB_FP64)) return GFB_OK;
+    if (units >= (size_t)0x7fffffff || s->fuse || (s->point_kernel && s->prec == GFB_FP64) || (s->flags & GFB_FLAG_COLOUR))
+        return GFB_OK;
     const size_t contrib = units * 3 * sizeof(Real);
     // beside the buffer: the touches and the half-step velocity (create_impl),
     // and some room for what a user attaches later
@@ -2688,6 +2689,12 @@ gfb_status gfb_get_info(const gfb_solver* s, gfb_info* info) {
     info->half_v = s->half_v ? 1 : 0;
     info->elem_variant = col_kernel_eligible(s) && !s->point_kernel ? s->col_variant : -1;
     info->n_elem_variants = col_kernel_eligible(s) ? s->n_col_variants : 0;
+    return GFB_OK;
+}
+
+gfb_status gfb_assembly(const gfb_solver* s, int32_t* by_colour) {
+    if (!s || !by_colour) return fail(GFB_ERR_INVALID, "NULL argument");
+    *by_colour = use_gather(s) ? 0 : 1;
     return GFB_OK;
 }
 

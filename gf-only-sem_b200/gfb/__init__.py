@@ -30,6 +30,7 @@ FLAG_POINT_KERNEL = 8
 FLAG_NO_GRAPH = 16
 FLAG_AUTOTUNE = 32
 FLAG_DIRECT_FORCE = 64
+FLAG_COLOUR = 128
 
 _dp = C.POINTER(C.c_double)
 _ip = C.POINTER(C.c_int32)
@@ -153,6 +154,7 @@ def load_library(path: str = LIB_PATH) -> C.CDLL:
     lib.gfb_create_sources.argtypes = [C.POINTER(Mesh), C.POINTER(Config), C.c_int32, C.POINTER(Source), C.c_int32,
                                        _ip, _ip, C.POINTER(C.c_void_p)]
     lib.gfb_get_info.argtypes = [C.c_void_p, C.POINTER(Info)]
+    lib.gfb_assembly.argtypes = [C.c_void_p, _ip]
     lib.gfb_select_element_kernel.argtypes = [C.c_void_p, C.c_int32]
     lib.gfb_set_force_refresh.argtypes = [C.c_void_p, C.c_int32]
     lib.gfb_current_step.argtypes = [C.c_void_p, _ip]
@@ -171,7 +173,7 @@ def load_library(path: str = LIB_PATH) -> C.CDLL:
         "gfb_element_residual", "gfb_advance_profiled", "gfb_get_info", "gfb_advance_timed",
         "gfb_create_batch", "gfb_checkpoint_size", "gfb_checkpoint_save", "gfb_checkpoint_load",
         "gfb_rec_nodes", "gfb_read_green", "gfb_read_record_f32", "gfb_create_sources",
-        "gfb_select_element_kernel", "gfb_set_force_refresh",
+        "gfb_select_element_kernel", "gfb_set_force_refresh", "gfb_assembly",
     ):
         getattr(lib, name).restype = C.c_int
     _lib = lib
@@ -349,9 +351,17 @@ class Solver:
         _check(self.lib.gfb_get_info(self.h, C.byref(i)))
         return {name: getattr(i, name) for name, _ in Info._fields_}
 
+    @property
+    def by_colour(self) -> bool:
+        """Whether the element force is assembled colour after colour (gfb_assembly)."""
+        c = C.c_int32()
+        _check(self.lib.gfb_assembly(self.h, C.byref(c)))
+        return c.value != 0
+
     def select_element_kernel(self, variant: int):
         """Use element-kernel variant `variant` from the next step on (-1: the
-        thread-per-point kernel; 0..n_elem_variants-1: the line kernel's)."""
+        thread-per-point kernel; 0: the default; 1..n_elem_variants-1: the
+        line kernel by colour)."""
         _check(self.lib.gfb_select_element_kernel(self.h, int(variant)))
 
     def set_force_refresh(self, steps: int):

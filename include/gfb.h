@@ -122,6 +122,12 @@ typedef struct gfb_config {
  * term is added at the nodes or there is none, and without a learned layer
  * or GFB_FLAG_FUSED_NODE (those evaluate in full every step). */
 #define GFB_FLAG_DIRECT_FORCE 64
+/* Assemble the element force colour after colour instead of through the cells'
+ * contributions (the same sums in another order).  Slower, but without the
+ * contribution buffer and the nodes' lists of it: about 5 KB per cell less
+ * device memory for three FP32 wavefields at ngll 5.  A solver whose buffer
+ * does not fit on the device does this by itself (gfb_assembly). */
+#define GFB_FLAG_COLOUR 128
 
 /* Point-force source (config.h5 /source, io.cpp:681-707). */
 typedef struct gfb_source {
@@ -271,6 +277,13 @@ typedef struct gfb_info {
 
 gfb_status gfb_get_info(const gfb_solver* solver, gfb_info* info);
 
+/* How the element force is assembled now: *by_colour = 0 by the node pass from
+ * the cells' contributions, 1 colour after colour (GFB_FLAG_COLOUR,
+ * GFB_FLAG_POINT_KERNEL, GFB_FLAG_FUSED_NODE, a kernel selected that does so, or
+ * not enough device memory for the contributions when the solver was made).
+ * The two differ in rounding. */
+gfb_status gfb_assembly(const gfb_solver* solver, int32_t* by_colour);
+
 /* FP32 path: steps between full evaluations of the element force (the steps
  * between add the force of the predicted displacement's increment; 800 by
  * default, 1 = in full every step).  The next step evaluates in full.
@@ -330,7 +343,9 @@ gfb_status gfb_read_green(gfb_solver* solver, int32_t* step, double* strain, dou
  * the C-PML memory and previous fields (per cell or per node) and the step
  * counters, in the device layout.  The reference's restart file keeps u, v,
  * a only (restart.cpp:120-152), so its resume restarts C-PML memory from
- * zero; loading a checkpoint continues bit for bit.  A checkpoint loads
+ * zero; loading a checkpoint continues bit for bit where the two solvers
+ * assemble alike (gfb_assembly; it depends on the free device memory too) and
+ * run the same element kernel, to rounding otherwise.  A checkpoint loads
  * into a solver built from the same inputs and flags (checked); snapshots
  * pending in the ring and a learned layer's history are not part of it.
  */
