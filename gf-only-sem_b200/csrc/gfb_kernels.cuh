@@ -2426,21 +2426,21 @@ __global__ void half_v_kernel(long long n_node, int F, long long hv_begin, bool 
     }
 }
 
-// u, v or a of wavefield `field` in the mesh's node order, out[node][3] as
-// double: one thread per value, the scattered side the read.  inv: node ->
-// device node (nullptr: the same).  what: 0 u, 1 v, 2 a; nodes >= hv_begin
+// u, v or a of wavefield `field` at the nodes [n0, n1) of the mesh's order,
+// out[node - n0][3] as double: one thread per value, the scattered side the read.
+// inv: node -> device node (nullptr: device nodes [n0, n1)).  what: 0 u, 1 v, 2 a; nodes >= hv_begin
 // hold the half-step velocity, as in half_v_kernel.
 template <typename Real>
-__global__ void state_kernel(long long n_node, int F, int field, int what, const int* inv, const double* u,
+__global__ void state_kernel(long long n0, long long n1, int F, int field, int what, const int* inv, const double* u,
                              const double* v, const Real* a, long long hv_begin, bool a_from_force, const float* w32,
                              const Real* force, const Real* inv_mass, const uint8_t* node_model, const ModelConst* mc,
                              double dt, double* out) {
-    const long long total = n_node * 3;
+    const long long total = (n1 - n0) * 3;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
         const long long n = t / 3;
         const int f = field * 3 + (int)(t - n * 3);
-        const long long g = inv ? inv[n] : n;
+        const long long g = inv ? inv[n0 + n] : n0 + n;
         const size_t i = (size_t)g * F + f;
         double x;
         if (what == 0) {

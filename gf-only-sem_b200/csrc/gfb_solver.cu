@@ -2756,39 +2756,68 @@ gfb_status gfb_get_state(gfb_solver* s, int32_t field, double* u, double* v, dou
     CU(cudaStreamSynchronize(s->stream));
     gfb_status st;
     if ((st = check_kernel_err(s))) return st;
-    // node -> device node on the device, from the first call on
-    if (!s->node_inv.empty() && !s->d_node_inv) {
-        if ((st = s->alloc(&s->d_node_inv, s->node_inv.size()))) return st;
-        if ((st = h2d(s, s->d_node_inv, s->node_inv.data(), s->node_inv.size() * 4))) return st;
+    // gathered on the device, range after range, into the contribution buffer,
+    // which every step writes anew, in the mesh's node order (node -> device
+    // node on the device from the first call on)
+    if (!s->node_inv.empty() && !s->d_node_inv && s->contrib) {
+        int* inv = nullptr;
+        if (s->alloc(&inv, s->node_inv.size()) == GFB_OK) {
+            if ((st = h2d(s, inv, s->node_inv.data(), s->node_inv.size() * 4))) return st;
+            s->d_node_inv = inv;
+        } else {
+            (void)cudaGetLastError();
+        }
     }
-    // gathered on the device into one array in the mesh's node order: the
-    // contribution buffer, which every step writes anew, where it is large
-    // enough (more than one point per node)
-    const size_t bytes = (size_t)s->n_node * 3 * sizeof(double);
-    DevBuf own;
+    // without that buffer or no memory for the map (a full device): in device
+    // node order into page-locked host memory, put in order by the host
+    struct HostBuf {
+        void* p = nullptr;
+        ~HostBuf() {
+            if (p) cudaFreeHost(p);
+        }
+    } host;
+    const bool direct = s->contrib && (s->node_inv.empty() || s->d_node_inv);
+    const size_t node_bytes = 3 * sizeof(double);
+    long long range = (long long)(s->contrib_bytes / node_bytes);
     double* out = static_cast<double*>(s->contrib);
-    if (s->contrib_bytes < bytes) {
-        CU(cudaMalloc(&own.p, bytes));
-        out = static_cast<double*>(own.p);
+    if (!direct || range < 1) {
+        range = std::min<long long>(s->n_node, (8 << 20) / node_bytes);
+        CU(cudaHostAlloc(&host.p, (size_t)range * node_bytes, cudaHostAllocMapped));
+        CU(cudaHostGetDevicePointer(reinterpret_cast<void**>(&out), host.p, 0));
     }
+    const int* inv = direct ? s->d_node_inv : nullptr;
     double* const dst[3] = {u, v, a};
+    const long long hv = s->half_v ? s->hv_begin : (long long)s->n_node;
     for (int what = 0; what < 3; ++what) {
         if (!dst[what]) continue;
-        const int grid = grid_for((long long)s->n_node * 3, 256);
-        const long long hv = s->half_v ? s->hv_begin : (long long)s->n_node;
-        if (s->prec == GFB_FP64)
-            gfb::state_kernel<double><<<grid, 256, 0, s->stream>>>(
-                s->n_node, s->F, field, what, s->d_node_inv, s->u, s->v, static_cast<const double*>(s->a), hv, s->a_in_force,
-                s->w32, static_cast<const double*>(s->force), static_cast<const double*>(s->inv_mass), s->d_node_model,
-                s->d_mc, s->dt, out);
-        else
-            gfb::state_kernel<float><<<grid, 256, 0, s->stream>>>(
-                s->n_node, s->F, field, what, s->d_node_inv, s->u, s->v, static_cast<const float*>(s->a), hv, s->a_in_force,
-                s->w32, static_cast<const float*>(s->force), static_cast<const float*>(s->inv_mass), s->d_node_model,
-                s->d_mc, s->dt, out);
-        CU(cudaGetLastError());
-        s->launches++;
-        if ((st = d2h(s, dst[what], out, bytes))) return st;
+        for (long long n0 = 0; n0 < s->n_node; n0 += range) {
+            const long long n1 = std::min<long long>(s->n_node, n0 + range);
+            const int grid = grid_for((n1 - n0) * 3, 256);
+            if (s->prec == GFB_FP64)
+                gfb::state_kernel<double><<<grid, 256, 0, s->stream>>>(
+                    n0, n1, s->F, field, what, inv, s->u, s->v, static_cast<const double*>(s->a), hv, s->a_in_force, s->w32,
+                    static_cast<const double*>(s->force), static_cast<const double*>(s->inv_mass), s->d_node_model, s->d_mc,
+                    s->dt, out);
+            else
+                gfb::state_kernel<float><<<grid, 256, 0, s->stream>>>(
+                    n0, n1, s->F, field, what, inv, s->u, s->v, static_cast<const float*>(s->a), hv, s->a_in_force, s->w32,
+                    static_cast<const float*>(s->force), static_cast<const float*>(s->inv_mass), s->d_node_model, s->d_mc,
+                    s->dt, out);
+            CU(cudaGetLastError());
+            s->launches++;
+            if (!host.p) {
+                if ((st = d2h(s, dst[what] + n0 * 3, out, (size_t)(n1 - n0) * node_bytes))) return st;
+                continue;
+            }
+            CU(cudaStreamSynchronize(s->stream));
+            const double* src = static_cast<const double*>(host.p);
+            parallel_for(n1 - n0, [&](long long i0, long long i1) {
+                for (long long i = i0; i < i1; ++i) {
+                    const long long g = direct || s->node_perm.empty() ? n0 + i : s->node_perm[n0 + i];
+                    for (int c = 0; c < 3; ++c) dst[what][g * 3 + c] = src[i * 3 + c];
+                }
+            });
+        }
     }
     return GFB_OK;
 }
