@@ -709,19 +709,20 @@ bool col_kernel_eligible(const gfb_solver* s) {
     return s->prec == GFB_FP32 && !(s->has_cpml && !s->node_pml) && !s->fuse;
 }
 
-// Candidates at ngll 5 with up to three wavefields: 0 the gather kernel, and
-// the line kernel by colour with 1 one fewer cell per group, 2 one more, 3
-// the default count.  Elsewhere the gather kernel only.
+// Candidates at ngll 5 with up to three wavefields: 0 the default (the gather
+// kernel, or the line kernel by colour in a solver without the contribution
+// buffer), and the line kernel by colour with 1 one fewer cell per group, 2 one
+// more, 3 the default count.  Elsewhere the default only.
 constexpr int col_epb_lo(int nfld) { return nfld == 3 ? 1 : (nfld == 2 ? 2 : 4); }
 constexpr int col_epb_hi(int nfld) { return nfld == 3 ? 3 : (nfld == 2 ? 4 : 8); }
 template <int NG, int NFLD>
-constexpr bool kHasCol = NG == 5 && NFLD <= 3;
+constexpr bool kColVariants = NG == 5 && NFLD <= 3;
 
-// Line kernel by colour: a variant of it is selected, or the mesh is too
-// large for the gather kernel.
-bool use_col_kernel(const gfb_solver* s) {
-    return col_kernel_eligible(s) && !s->point_kernel && !use_gather(s) && s->ng == 5 && s->nfld <= 3;
-}
+// Line kernel by colour: a variant of it is selected, or the solver has no
+// contribution buffer (with the point kernel instead, a step takes 136 against 114
+// us at ngll 3, 37 x 29 x 23 x 3; 152 / 118 at ngll 4, 30 x 31 x 17 x 2; 280 / 230 at
+// ngll 6, 22 x 21 x 13 x 3; 1,014 / 538 at ngll 5 with six wavefields, 32 x 32 x 16).
+bool use_col_kernel(const gfb_solver* s) { return col_kernel_eligible(s) && !s->point_kernel && !use_gather(s); }
 
 template <int NG, int NFLD, int EPB>
 gfb_status launch_col_e(gfb_solver* s, int c) {
@@ -765,8 +766,10 @@ gfb_status launch_col_e(gfb_solver* s, int c) {
 
 template <int NG, int NFLD>
 gfb_status launch_col_t(gfb_solver* s, int c) {
-    if (s->col_variant == 1) return launch_col_e<NG, NFLD, col_epb_lo(NFLD)>(s, c);
-    if (s->col_variant == 2) return launch_col_e<NG, NFLD, col_epb_hi(NFLD)>(s, c);
+    if constexpr (kColVariants<NG, NFLD>) {
+        if (s->col_variant == 1) return launch_col_e<NG, NFLD, col_epb_lo(NFLD)>(s, c);
+        if (s->col_variant == 2) return launch_col_e<NG, NFLD, col_epb_hi(NFLD)>(s, c);
+    }
     return launch_col_e<NG, NFLD, gfb::col_default_epb(NG, NFLD)>(s, c);
 }
 
@@ -788,14 +791,12 @@ gfb_status col_grid(gfb_solver* s) {
 
 template <int NG, int NFLD>
 gfb_status col_grid_t(gfb_solver* s) {
-    s->n_col_variants = 1;
-    if constexpr (kHasCol<NG, NFLD>) {
-        s->n_col_variants = 4;
+    s->n_col_variants = kColVariants<NG, NFLD> ? 4 : 1;
+    if constexpr (kColVariants<NG, NFLD>) {
         if (s->col_variant == 1) return col_grid<NG, NFLD, col_epb_lo(NFLD)>(s);
         if (s->col_variant == 2) return col_grid<NG, NFLD, col_epb_hi(NFLD)>(s);
-        return col_grid<NG, NFLD, gfb::col_default_epb(NG, NFLD)>(s);
     }
-    return GFB_OK;
+    return col_grid<NG, NFLD, gfb::col_default_epb(NG, NFLD)>(s);
 }
 
 template <typename Real, int NG>
@@ -999,7 +1000,7 @@ gfb_status dispatch(int ng, int nfld, Args... args) {
 template <typename Real, int NG, int NFLD>
 struct ElemOp {
     static gfb_status run(gfb_solver* s, int c) {
-        if constexpr (std::is_same<Real, float>::value && kHasCol<NG, NFLD>)
+        if constexpr (std::is_same<Real, float>::value)
             if (use_col_kernel(s)) return launch_col_t<NG, NFLD>(s, c);
         return launch_elem_t<Real, NG, NFLD>(s, c);
     }

@@ -112,3 +112,21 @@ def test_selected_kernels_report_their_assembly():
         s = gfb.Solver(prob, dirs=[0], precision=gfb.FP64, flags=flags)
         assert s.by_colour
         s.close()
+
+
+@pytest.mark.parametrize("order,fields", [(2, 1), (2, 3), (3, 2), (4, 3), (4, 6), (4, 9), (4, 12), (5, 3)])
+def test_by_colour_runs_the_line_kernel(order, fields):
+    """Every FP32 shape has it; the point kernel takes up to twice the time."""
+    prob = problem(order)
+    ids, w = np.asarray(prob["src_cell_ids"]), np.asarray(prob["src_weights"])
+    src = {"src_cell_ids": ids, "src_weights": w, "stf": prob["stf"]}
+    more = dict(sources=[src], field_source=[0] * fields) if fields > 3 else {}
+
+    def make(flags):
+        return gfb.Solver(prob, dirs=[f % 3 for f in range(fields)], precision=gfb.FP32, flags=flags, **more)
+
+    a, b = make(0), make(gfb.FLAG_COLOUR)
+    assert b.by_colour and b.info()["elem_kernel"] == 1 and b.info()["cells_per_group"] >= 1
+    close(kick(b, prob["n_node"]), kick(a, prob["n_node"]), TOL[gfb.FP32])
+    a.close()
+    b.close()
