@@ -1212,20 +1212,29 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_>::THREADS, ColShape<NG
         const int e0 = A.e_begin + grp * EPB, nc = min(EPB, e_end - e0);
         fence_proxy_async_smem();
         mbar_expect_tx(&s_bar[st], (unsigned)(nc * S::GEO_B));
-        for (int c = 0; c < nc; ++c)
-            bulk_copy_g2s(gbase + (st * EPB + c) * S::GEO_SLOT,
-                          reinterpret_cast<const unsigned char*>(A.geom) + (size_t)__ldg(A.cells + e0 + c) * S::GEO_B, S::GEO_B,
-                          &s_bar[st]);
+        int cell[EPB];  // looked up together
+#pragma unroll
+        for (int c = 0; c < EPB; ++c) cell[c] = c < nc ? __ldg(A.cells + e0 + c) : 0;
+#pragma unroll
+        for (int c = 0; c < EPB; ++c)
+            if (c < nc)
+                bulk_copy_g2s(gbase + (st * EPB + c) * S::GEO_SLOT,
+                              reinterpret_cast<const unsigned char*>(A.geom) + (size_t)cell[c] * S::GEO_B, S::GEO_B, &s_bar[st]);
     };
     auto tma_ib = [&](int grp, int st) {
         if (tid != 0) return;
         const int e0 = A.e_begin + grp * EPB, nc = min(EPB, e_end - e0);
         fence_proxy_async_smem();
         mbar_expect_tx(&s_bar[2 + st], (unsigned)(nc * S::IB_B));
-        for (int c = 0; c < nc; ++c)
-            bulk_copy_g2s(ibase + (st * EPB + c) * S::IB_B,
-                          reinterpret_cast<const unsigned char*>(A.ibool_padded) + (size_t)__ldg(A.cells + e0 + c) * S::IB_B,
-                          S::IB_B, &s_bar[2 + st]);
+        int cell[EPB];
+#pragma unroll
+        for (int c = 0; c < EPB; ++c) cell[c] = c < nc ? __ldg(A.cells + e0 + c) : 0;
+#pragma unroll
+        for (int c = 0; c < EPB; ++c)
+            if (c < nc)
+                bulk_copy_g2s(ibase + (st * EPB + c) * S::IB_B,
+                              reinterpret_cast<const unsigned char*>(A.ibool_padded) + (size_t)cell[c] * S::IB_B, S::IB_B,
+                              &s_bar[2 + st]);
     };
     // a wait that gave up: flag it, give the copies in flight a second
     // bounded wait, and leave (every thread together)

@@ -719,7 +719,7 @@ template <int NG, int NFLD>
 constexpr bool kColVariants = NG == 5 && NFLD <= 3;
 
 // Line kernel by colour: a variant of it is selected, or the solver has no
-// contribution buffer (with the point kernel instead, a step takes 136 against 114
+// contribution buffer (with the point kernel instead, a step takes 136 against 105
 // us at ngll 3, 37 x 29 x 23 x 3; 152 / 118 at ngll 4, 30 x 31 x 17 x 2; 280 / 230 at
 // ngll 6, 22 x 21 x 13 x 3; 1,014 / 538 at ngll 5 with six wavefields, 32 x 32 x 16).
 bool use_col_kernel(const gfb_solver* s) { return col_kernel_eligible(s) && !s->point_kernel && !use_gather(s); }
