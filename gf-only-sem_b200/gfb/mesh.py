@@ -569,8 +569,13 @@ def _cpml_parameters(coords, is_pml, bounds, widths, vp, f0, dt):
     return regions, coef_alpha, abar
 
 
-def hex_newton(x_target, corners, max_iter=50, tol=1e-12):
-    """Natural coordinates of a point in a trilinear hex (source_locator.py:74-123)."""
+def hex_newton(x_target, corners, max_iter=50, tol=1e-12, transposed=False):
+    """Natural coordinates of a point in a trilinear hex (source_locator.py:74-123).
+
+    With J[a, c] = dx_c / dxi_a, Newton's step solves J^T dxi = res
+    (``transposed``).  The default step solves J dxi = res, as the reference
+    does: the same root, reached at once where J is symmetric (boxes), but
+    linearly and not always within ``max_iter`` on a strongly deformed cell."""
     xi = np.zeros(3)
     for _ in range(max_iter):
         fa = 1 + HEX_CORNERS[:, 0] * xi[0]
@@ -584,7 +589,7 @@ def hex_newton(x_target, corners, max_iter=50, tol=1e-12):
         res = x_target - Nv @ corners
         J = dN.T @ corners
         try:
-            dxi = np.linalg.solve(J, res)
+            dxi = np.linalg.solve(J.T if transposed else J, res)
         except np.linalg.LinAlgError:
             return None
         xi = xi + dxi
@@ -600,7 +605,9 @@ def hex_newton(x_target, corners, max_iter=50, tol=1e-12):
 def locate_point_source(coords, corners, source_xyz, is_pml, order):
     """Buried-mode source location: AABB candidates among non-PML cells,
     Newton, Lagrange weights normalised over all containing cells
-    (source_locator.py:186-213, 295-375)."""
+    (source_locator.py:186-213, 295-375).  A source that the reference's
+    iteration finds in no cell is looked for once more with Newton's own step,
+    which converges in every cell that contains it."""
     ng = order + 1
     pts = gll_points(order)
     lo = coords.reshape(coords.shape[0], -1, 3).min(axis=1)
@@ -608,16 +615,19 @@ def locate_point_source(coords, corners, source_xyz, is_pml, order):
     m = 1e-10
     cand = np.nonzero(np.all((lo - m <= source_xyz) & (source_xyz <= hi + m), axis=1) & ~is_pml)[0]
     ids, ws = [], []
-    for e in cand:
-        xi = hex_newton(np.asarray(source_xyz, dtype=np.float64), corners[e])
-        if xi is None:
-            continue
-        lx, ly, lz = (lagrange_1d(xi[a], pts) for a in range(3))
-        w = lx[:, None, None] * ly[None, :, None] * lz[None, None, :]
-        if np.sum(w) < 1e-12:
-            continue
-        ids.append(int(e))
-        ws.append(w)
+    for transposed in (False, True):
+        for e in cand:
+            xi = hex_newton(np.asarray(source_xyz, dtype=np.float64), corners[e], transposed=transposed)
+            if xi is None:
+                continue
+            lx, ly, lz = (lagrange_1d(xi[a], pts) for a in range(3))
+            w = lx[:, None, None] * ly[None, :, None] * lz[None, None, :]
+            if np.sum(w) < 1e-12:
+                continue
+            ids.append(int(e))
+            ws.append(w)
+        if ids:
+            break
     if not ids:
         raise ValueError(f"source {source_xyz} not inside any non-PML cell")
     total = float(sum(np.sum(w) for w in ws))
