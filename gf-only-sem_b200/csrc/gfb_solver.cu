@@ -224,6 +224,43 @@ struct DevBuf {
     }
 };
 
+// Words of mapped host memory for the solvers' error flags: one page-locked page
+// for the process, allocated by the first solver (page-locking and freeing one
+// on every create costs milliseconds), each word given back by its solver.  A
+// solver past the last word gets memory of its own.
+struct FlagWords {
+    static constexpr int N = 1024;
+    std::mutex mu;
+    unsigned* page = nullptr;
+    std::vector<int> free_words;
+    cudaError_t take(unsigned** word, bool* own) {
+        std::lock_guard<std::mutex> lk(mu);
+        if (!page) {
+            const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&page), N * sizeof(unsigned),
+                                                cudaHostAllocMapped | cudaHostAllocPortable);
+            if (e != cudaSuccess) {
+                page = nullptr;
+                return e;
+            }
+            for (int k = N - 1; k >= 0; --k) free_words.push_back(k);
+        }
+        *own = free_words.empty();
+        if (*own) return cudaHostAlloc(reinterpret_cast<void**>(word), sizeof(unsigned), cudaHostAllocMapped);
+        *word = page + free_words.back();
+        free_words.pop_back();
+        return cudaSuccess;
+    }
+    void give_back(unsigned* word, bool own) {
+        std::lock_guard<std::mutex> lk(mu);
+        if (own) cudaFreeHost(word);
+        else free_words.push_back((int)(word - page));
+    }
+};
+FlagWords& flag_words() {
+    static FlagWords* w = new FlagWords();  // never destroyed: freed with the process
+    return *w;
+}
+
 struct Snapshot {
     int step;
     int slot;                  // ring slot (device + pinned host), -1 once spilled
@@ -240,10 +277,10 @@ struct gfb_solver {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;   // snapshots to the host
-    cudaStream_t merge_stream = nullptr;  // their merge per recording node
-    // the C-PML node pass runs beside the plain one: elem_evt, the element
-    // phase it follows; pml_evt, its end, which the next step waits for
-    cudaStream_t node_stream = nullptr;
+    // beside the steps: the snapshots' merge per recording node, and the C-PML
+    // node pass beside the plain one (elem_evt, the element phase it follows;
+    // pml_evt, its end, which the next step waits for)
+    cudaStream_t side_stream = nullptr;   // null where a solver has neither
     cudaEvent_t elem_evt = nullptr, pml_evt = nullptr;
     bool capturing = false;
     int prec = GFB_FP64;
@@ -333,6 +370,7 @@ struct gfb_solver {
     // so that every call that hands out results can look at it without a copy
     // (after the synchronisation that the results need anyway)
     unsigned *kernel_err = nullptr, *d_kernel_err = nullptr;
+    bool own_err = false;
     // plain nodes (device nodes >= hv_begin) keep the half-step velocity
     // v + dt/2 a in v and no acceleration (FP32 path); a_in_force: the
     // assembled force holds the last step's (a = f/m), else a is the stored
@@ -397,14 +435,13 @@ struct gfb_solver {
         for (auto e : cell_evt) cudaEventDestroy(e);
         for (auto e : copy_evt) cudaEventDestroy(e);
         for (auto p : pinned) cudaFreeHost(p);
-        if (kernel_err) cudaFreeHost(kernel_err);
+        if (kernel_err) flag_words().give_back(kernel_err, own_err);
         bufs.clear();
         if (stream) cudaStreamDestroy(stream);
         if (copy_stream) cudaStreamDestroy(copy_stream);
-        if (merge_stream) cudaStreamDestroy(merge_stream);
         if (elem_evt) cudaEventDestroy(elem_evt);
         if (pml_evt) cudaEventDestroy(pml_evt);
-        if (node_stream) cudaStreamDestroy(node_stream);
+        if (side_stream) cudaStreamDestroy(side_stream);
     }
 };
 
@@ -1118,7 +1155,7 @@ gfb_status launch_node_m(gfb_solver* s) {
             // us per step (32 x 32 x 16 x 6), 407 / 399 (40 x 40 x 20 x 3), 78.5 /
             // 73 (20 x 20 x 10 x 3), 82 / 71 (six small models); in one launch,
             // at the C-PML pass's registers, 433 / 399 (40 x 40 x 20 x 3).
-            cudaStream_t q = two ? s->node_stream : s->stream;
+            cudaStream_t q = two ? s->side_stream : s->stream;
             if (two) CU(cudaStreamWaitEvent(q, s->elem_evt, 0));
             CU(launch_chained(two ? elem_lets(s) != nullptr : early, gfb::node_pml_kernel<NFLD, MULTI>,
                               node_grid(g0, gfb::node_blocks_per_sm<float>(true)), gfb::kNodeThreads, 0, q, A, P));
@@ -2155,7 +2192,7 @@ gfb_status some_steps(gfb_solver* s, int n, cudaEvent_t* ev, int* done) {
         // beside the following steps: the merge on its own stream, the records
         // and then the merged part to the host on the copy stream
         CU(cudaEventRecord(s->rec_evt[slot], s->stream));
-        CU(cudaStreamWaitEvent(s->merge_stream, s->rec_evt[slot], 0));
+        CU(cudaStreamWaitEvent(s->side_stream, s->rec_evt[slot], 0));
         CU(cudaStreamWaitEvent(s->copy_stream, s->rec_evt[slot], 0));
         const size_t cell_bytes = snapshot_cell_values(s) * (s->rec_f32 ? 4 : 8);
         unsigned char* host = static_cast<unsigned char*>(s->pinned[slot]);
@@ -2166,15 +2203,15 @@ gfb_status some_steps(gfb_solver* s, int n, cudaEvent_t* ev, int* done) {
             const int grid = grid_for(total, 256);
             const long long per_field = (long long)s->n_rec * s->nn;
             if (s->rec_f32)
-                gfb::merge_nodes_kernel<float><<<grid, 256, 0, s->merge_stream>>>(
+                gfb::merge_nodes_kernel<float><<<grid, 256, 0, s->side_stream>>>(
                     s->nfld, s->n_unique, per_field, s->gf_ptr, s->gf_occ, s->gf_w, static_cast<float*>(dslot));
             else
-                gfb::merge_nodes_kernel<double><<<grid, 256, 0, s->merge_stream>>>(
+                gfb::merge_nodes_kernel<double><<<grid, 256, 0, s->side_stream>>>(
                     s->nfld, s->n_unique, per_field, s->gf_ptr, s->gf_occ, s->gf_w, static_cast<double*>(dslot));
             CU(cudaGetLastError());
             s->launches++;
         }
-        CU(cudaEventRecord(s->merge_evt[slot], s->merge_stream));
+        CU(cudaEventRecord(s->merge_evt[slot], s->side_stream));
         if (ev) CU(cudaStreamWaitEvent(s->stream, s->merge_evt[slot], 0));  // in the phase's time
         CU(cudaStreamWaitEvent(s->copy_stream, s->merge_evt[slot], 0));
         CU(cudaMemcpyAsync(host + cell_bytes, static_cast<unsigned char*>(dslot) + cell_bytes, snapshot_bytes(s) - cell_bytes,
@@ -2315,11 +2352,7 @@ gfb_status create_impl(const gfb_mesh* m, const gfb_config* c, const gfb_source*
     s->c2 = (1.0 - theta) * 0.5 * c->dt * c->dt;
     CU(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     CU(cudaStreamCreateWithFlags(&s->copy_stream, cudaStreamNonBlocking));
-    CU(cudaStreamCreateWithFlags(&s->merge_stream, cudaStreamNonBlocking));
-    CU(cudaStreamCreateWithFlags(&s->node_stream, cudaStreamNonBlocking));
-    CU(cudaEventCreateWithFlags(&s->elem_evt, cudaEventDisableTiming));
-    CU(cudaEventCreateWithFlags(&s->pml_evt, cudaEventDisableTiming));
-    CU(cudaHostAlloc(reinterpret_cast<void**>(&s->kernel_err), sizeof(unsigned), cudaHostAllocMapped));
+    CU(flag_words().take(&s->kernel_err, &s->own_err));
     *s->kernel_err = 0;
     CU(cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->d_kernel_err), s->kernel_err, 0));
 
@@ -2464,6 +2497,11 @@ gfb_status create_impl(const gfb_mesh* m, const gfb_config* c, const gfb_source*
     if (s->gather_ok) {
         if ((st = s->prec == GFB_FP64 ? gather_grid<double>(s.get()) : gather_grid<float>(s.get()))) return st;
     }
+    if (s->n_rec > 0 || two_node_passes(s.get())) {
+        CU(cudaStreamCreateWithFlags(&s->side_stream, cudaStreamNonBlocking));
+        CU(cudaEventCreateWithFlags(&s->elem_evt, cudaEventDisableTiming));
+        CU(cudaEventCreateWithFlags(&s->pml_evt, cudaEventDisableTiming));
+    }
     CU(cudaStreamSynchronize(s->stream));
     clk.mark("device set-up");
     // FP32 path: the element force of most steps from the predicted
@@ -2592,7 +2630,7 @@ gfb_status gfb_destroy(gfb_solver* s) {
     cudaSetDevice(s->device);
     cudaStreamSynchronize(s->stream);
     cudaStreamSynchronize(s->copy_stream);
-    cudaStreamSynchronize(s->merge_stream);
+    if (s->side_stream) cudaStreamSynchronize(s->side_stream);
     delete s;
     return GFB_OK;
 }
@@ -2739,7 +2777,7 @@ gfb_status gfb_synchronize(gfb_solver* s) {
     if (!s) return fail(GFB_ERR_INVALID, "solver is NULL");
     CU(cudaSetDevice(s->device));
     CU(cudaStreamSynchronize(s->stream));
-    CU(cudaStreamSynchronize(s->merge_stream));
+    if (s->side_stream) CU(cudaStreamSynchronize(s->side_stream));
     CU(cudaStreamSynchronize(s->copy_stream));
     return check_kernel_err(s);
 }
@@ -3276,7 +3314,8 @@ gfb_status solver_set_layer(gfb_solver* s, Layer* layer) {
 extern "C" gfb_status gfb_work_queued(gfb_solver* s, int32_t* queued) {
     if (!s || !queued) return fail(GFB_ERR_INVALID, "NULL argument");
     *queued = 0;
-    for (cudaStream_t q : {s->stream, s->merge_stream, s->copy_stream}) {
+    for (cudaStream_t q : {s->stream, s->side_stream, s->copy_stream}) {
+        if (!q) continue;
         const cudaError_t e = cudaStreamQuery(q);
         if (e == cudaErrorNotReady) *queued = 1;
         else CU(e);
