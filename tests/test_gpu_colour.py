@@ -130,3 +130,22 @@ def test_by_colour_runs_the_line_kernel(order, fields):
     close(kick(b, prob["n_node"]), kick(a, prob["n_node"]), TOL[gfb.FP32])
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("prec", [gfb.FP64, gfb.FP32])
+@pytest.mark.parametrize("ngll,n", [(3, 18518), (3, 18519), (4, 2), (5, 3999), (5, 4000), (6, 2315)])
+def test_element_residual_by_either_assembly(ngll, n, prec):
+    """On both sides of the size where the call changes its assembly: the same
+    cells one by one (K_e is linear, so the sums differ by rounding alone)."""
+    rng = np.random.default_rng(ngll)
+    P = n * ngll**3
+    dxi = rng.uniform(-0.3, 0.3, (P, 9))
+    dxi[:, [0, 4, 8]] += 1.0
+    a = [rng.uniform(0.5, 1.5, P) for _ in range(3)]
+    u = rng.standard_normal((P, 3))
+    r = gfb.element_residual(dxi, *a, u, ngll, prec).reshape(n, -1)
+    k = np.r_[0, n // 2, n - 1]
+    q = (k[:, None] * ngll**3 + np.arange(ngll**3)).ravel()
+    one = gfb.element_residual(dxi[q], *(x[q] for x in a), u[q], ngll, prec).reshape(len(k), -1)
+    assert np.isfinite(r).all()
+    assert np.abs(r[k] - one).max() <= TOL[prec] * np.abs(one).max()
