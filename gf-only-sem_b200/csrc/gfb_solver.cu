@@ -184,7 +184,10 @@ struct NodeBuckets {
 NodeBuckets bucket_points(const int* ibool, long long P, long long n_node) {
     NodeBuckets b;
     const long long hw = std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
-    b.n_owner = (int)std::max(1LL, std::min(hw, n_node / (1LL << 18)));
+    // 16 Ki nodes per owner or more: with 256 Ki a mesh of 4,000 cells had one
+    // owner, and its lists for the assembly made gfb_create 62-72 ms long
+    // instead of 55-60
+    b.n_owner = (int)std::max(1LL, std::min(hw, n_node / (1LL << 14)));
     b.n_node = n_node;
     const int T = b.n_owner;
     b.bound.resize(T + 1);
