@@ -71,3 +71,22 @@ def compare(a, b):
         assert np.isfinite(x[0]).all() and np.abs(x[0]).max() > 0
         for p, q in zip(x, y):
             np.testing.assert_array_equal(p, q)
+
+
+def test_runs_of_every_length():
+    """Graphs of one to five steps, in any order, with and without snapshots."""
+    prob = problem()
+    for stride in (0, 4, 7):
+        prob["snapshot_stride"] = stride
+        out = []
+        for flags in (0, gfb.FLAG_NO_GRAPH):
+            s = gfb.Solver(prob, dirs=[0, 1, 2], precision=gfb.FP32, flags=flags)
+            for n in (4, 1, 9, 3, 2, 5, 11, 0, 8):
+                s.advance(n)
+            assert s.step == 43
+            s.synchronize()
+            n_launch = s.info()["kernel_launches"]
+            out.append((s.drain(), [s.state(f) for f in range(3)], n_launch))
+            s.close()
+        assert out[0][2] == out[1][2]
+        compare(out[0], out[1])
