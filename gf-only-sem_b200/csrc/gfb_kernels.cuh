@@ -95,8 +95,6 @@ template <int NG>
 struct Shape {
     static constexpr int NN = NG * NG * NG;
     static constexpr int NNP = (NN + 31) / 32 * 32;
-    static constexpr int EPB = NNP <= 32 ? 8 : (NNP <= 64 ? 4 : (NNP <= 128 ? 2 : 1));
-    static constexpr int THREADS = NNP * EPB;
 };
 
 // Assembly by the node pass.  The element kernel leaves every cell's force
@@ -190,7 +188,6 @@ template <typename Real>
 struct ElemArgs {
     int e_begin, e_end;     // range of `cells`
     const int* cells;       // the cells colour after colour
-    const uint32_t* ibool;
     const Real* geom;
     const Real* ut;
     Real* force;
@@ -1441,11 +1438,12 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_>::THREADS, ColShape<NG
 // elem_gather_kernel: the element kernel of the time loop (both precisions).
 //
 // A group of WARPS warps takes CELLS cells at a time and leaves their force
-// contributions in contrib; the node pass adds them up (NodeGather).  Against a read-modify-write of the assembled force colour
-// after colour this stores 4 (8) bytes per value in whole rows instead of
-// reading and writing 16-byte vectors node by node, needs one launch instead
-// of one per colour, and takes the cells in mesh order, so the predicted
-// displacement of the nodes that neighbours share comes from L2.
+// contributions in contrib; the node pass adds them up (NodeGather).  Against a
+// read-modify-write of the assembled force colour after colour this stores 4 (8)
+// bytes per value in whole rows instead of reading and writing 16-byte vectors
+// node by node, needs one launch instead of one per colour, and takes the cells
+// in mesh order, so the predicted displacement of the nodes that neighbours
+// share comes from L2.
 //
 // One thread per xi-line: the NG points (i = 0..NG-1, j, k) of a cell, for one
 // wavefield after the other, so the geometry is fetched once for all of them
@@ -1469,7 +1467,7 @@ __global__ void __launch_bounds__(ColShape<NG, NFLD, EPB_>::THREADS, ColShape<NG
 // Measured on 40 x 40 x 20 cells of ngll 5: FP32 with three wavefields 205 us
 // (3,780 instructions and 1,020 shared wavefronts per cell, the L1 pipe 69 %
 // busy, issue 57 %, DRAM 24 %); by colour the same took about 310 us.  FP64
-// with one wavefield and per-cell C-PML in half of the cells 378 us.
+// with one wavefield 136 us.
 // ---------------------------------------------------------------------------
 
 // Point (i, j, k) of an exchange array at P*i + NG*j + k, a cell's component
@@ -1540,10 +1538,10 @@ struct GatherArgs {
 // last step's memory is added to the cells' contributions, and the memory
 // moves on, which only uses values fixed at the start of the step.  A block
 // takes a C-PML cell at a time, one thread per (component, point); the arrays
-// are streams of whole rows.  An axis
-// that is live nowhere in a cell (its A_k are 0 there) has a memory nothing
-// reads: it is neither loaded nor updated, which is more than half of the
-// traffic in the one-axis cells that most C-PML cells are.  Inside the element
+// are streams of whole rows.  An axis that is live nowhere in a cell (its A_k
+// are 0 there) has a memory nothing reads: it is neither loaded nor updated,
+// which is more than half of the traffic in the one-axis cells that most C-PML
+// cells are.  Inside the element
 // kernel, with 12 warps per SM and every axis, the same work took 220 us on
 // 40 x 40 x 20 cells (15,600 of them C-PML, FP64, one wavefield).
 template <typename Real>

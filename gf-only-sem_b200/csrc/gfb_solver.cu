@@ -267,7 +267,7 @@ FlagWords& flag_words() {
 struct Snapshot {
     int step;
     int slot;                  // ring slot (device + pinned host), -1 once spilled
-    std::unique_ptr<unsigned char[]> host;  // spilled raw copy [NFLD][n_rec][NN][15] (float or double)
+    std::unique_ptr<unsigned char[]> host;  // spilled raw copy of the slot (snapshot_bytes)
     int fields_read = 0;
     int readers = 0;           // gfb_read_record calls copying out of the slot
     bool done = false;         // read (or released); removed once no reader holds it
@@ -278,6 +278,7 @@ struct Snapshot {
 
 struct gfb_solver {
     int device = 0;
+    int n_sm = 0;  // multiprocessors
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;   // snapshots to the host
     // beside the steps: the snapshots' merge per recording node, and the C-PML
@@ -312,7 +313,6 @@ struct gfb_solver {
     uint4* touch = nullptr;         // [node] (gfb::NodeGather)
     uint4* touch_more = nullptr;
     int gather_blocks = 0;          // persistent grid of the gather kernel
-    int gather_sm = 0;              // multiprocessors
     int plane_blocks = 0;           // of the plane kernel (0: not used)
     bool has_cpml = false, has_damping = false, has_src = false;
     int n_pml = 0, n_src = 0, n_rec = 0, slots = 0;
@@ -634,7 +634,7 @@ bool use_gather(const gfb_solver* s) {
 // that is 200 KB and more (line kernel at ngll 5 and 6, FP64) a pass then misses
 // the L1 it reads its contributions through: 498 against 480 us per step (FP64,
 // 40 x 40 x 20 cells), 187 / 177 (ngll 6, 22 x 21 x 13), 178 / 166 (one FP32
-// wavefield, 40 x 40 x 20).  Beside the plane kernel and at ngll 3 it gains:
+// wavefield at ngll 5, 40 x 40 x 20), 80 / 79 (two at ngll 4, 30 x 31 x 17).  Beside the plane kernel and at ngll 3 it gains:
 // 400 / 405 (40 x 40 x 20 x 3), 68 / 72 (20 x 20 x 10 x 3), 72 / 81 (six small
 // models), 69.5 / 72.5 (ngll 3).
 bool node_early(const gfb_solver* s) {
@@ -705,7 +705,6 @@ gfb_status launch_elem_t(gfb_solver* s, int c) {
     A.e_end = s->colour_begin[c + 1];
     if (A.e_end <= A.e_begin) return GFB_OK;
     A.cells = s->clist;
-    A.ibool = s->ibool;
     A.geom = static_cast<const Real*>(s->geom);
     A.ut = static_cast<const Real*>(s->ut);
     A.force = static_cast<Real*>(s->force);
@@ -821,11 +820,10 @@ gfb_status col_grid(gfb_solver* s) {
     auto* fn = gfb::elem_col_kernel<NG, NFLD, EPB>;
     const int smem = C::SMEM + gfb::col_model_smem(s->n_model, s->n_set);
     CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    int per_sm = 0, n_sm = 0;
+    int per_sm = 0;
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, C::THREADS, smem));
-    CU(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, s->device));
     if (per_sm < 1) return fail(GFB_ERR_UNSUPPORTED, "line element kernel does not fit on an SM");
-    s->col_blocks = per_sm * n_sm;
+    s->col_blocks = per_sm * s->n_sm;
     s->col_epb = EPB;
     return GFB_OK;
 }
@@ -866,11 +864,11 @@ gfb_status launch_gather_t(gfb_solver* s) {
     A.err = s->d_kernel_err;
     for (int q = 0; q < 36; ++q) A.D[q] = q < NG * NG ? (Real)s->dmat_host[q] : Real(0);
     for (int q = 0; q < 36; ++q) A.D2[q] = make_float2((float)A.D[q], (float)A.D[q]);
-    // a work item is a group's cells with all their wavefields (the geometry
-    // read once), or one wavefield of them where that would leave more than
-    // half of the resident groups without work
-    // wavefields in threes at ngll 5 in FP32: the plane kernel (faster from
-    // 20 x 20 x 10 cells up, 76 against 82 us per step, level below)
+    // A work item is a group's cells with all their wavefields (the geometry
+    // read once), or, where that would leave more than half of the resident
+    // groups without work, with one of them (three, plane kernel).
+    // Wavefields in threes at ngll 5 in FP32 take the plane kernel (faster from
+    // 20 x 20 x 10 cells up, 76 against 82 us per step, level below).
     if constexpr (std::is_same<Real, float>::value && NG == 5) {
         if (s->plane_blocks > 0) {
             using PS = gfb::PlaneShape;
@@ -910,7 +908,7 @@ gfb_status launch_gather_t(gfb_solver* s) {
         // with the little L1 the element kernel leaves (486 / 391 us,
         // 40 x 40 x 20)
         constexpr int threads = gfb::cell_pml_threads(S::NN);
-        const int cells = std::min(s->n_pml, s->gather_sm * (gfb::kCellPmlThreads / threads));
+        const int cells = std::min(s->n_pml, s->n_sm * (gfb::kCellPmlThreads / threads));
         P.multi = s->n_model > 1;
         const bool early = 2 * blocks <= s->gather_blocks;
         auto* fn = early ? gfb::cell_pml_kernel<Real, NG, true> : gfb::cell_pml_kernel<Real, NG, false>;
@@ -926,19 +924,17 @@ gfb_status gather_grid_t(gfb_solver* s) {
     using S = gfb::GatherShape<Real, NG>;
     auto* fn = gfb::elem_gather_kernel<Real, NG>;
     CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
-    int per_sm = 0, n_sm = 0;
+    int per_sm = 0;
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, S::THREADS, S::SMEM));
-    CU(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, s->device));
     if (per_sm < 1) return fail(GFB_ERR_UNSUPPORTED, "gather element kernel does not fit on an SM");
-    s->gather_blocks = per_sm * n_sm;
-    s->gather_sm = n_sm;
+    s->gather_blocks = per_sm * s->n_sm;
     if constexpr (std::is_same<Real, float>::value && NG == 5) {
         if (s->nfld % 3 == 0 && !(s->has_cpml && !s->node_pml)) {
             using PS = gfb::PlaneShape;
             auto* plane = s->off_points ? gfb::elem_plane_kernel<true> : gfb::elem_plane_kernel<false>;
             CU(cudaFuncSetAttribute(plane, cudaFuncAttributeMaxDynamicSharedMemorySize, PS::SMEM));
             CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, plane, PS::THREADS, PS::SMEM));
-            s->plane_blocks = per_sm * n_sm;
+            s->plane_blocks = per_sm * s->n_sm;
         }
     }
     return GFB_OK;
@@ -980,12 +976,11 @@ gfb_status set_smem_t(gfb_solver* s) {
     using S = gfb::PipeShape<Real, NG, NFLD>;
     CU(cudaFuncSetAttribute(gfb::elem_pipe_kernel<Real, NG, NFLD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             S::SMEM));
-    int per_sm = 0, n_sm = 0;
+    int per_sm = 0;
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gfb::elem_pipe_kernel<Real, NG, NFLD>, S::THREADS,
                                                      S::SMEM));
-    CU(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, s->device));
     if (per_sm < 1) return fail(GFB_ERR_UNSUPPORTED, "element kernel does not fit on an SM");
-    s->pipe_blocks = per_sm * n_sm;
+    s->pipe_blocks = per_sm * s->n_sm;
     if constexpr (std::is_same<Real, float>::value) return col_grid_t<NG, NFLD>(s);
     return GFB_OK;
 }
@@ -1130,9 +1125,9 @@ gfb_status launch_record(gfb_solver* s, void* out) {
 
 
 // Blocks of a node pass over n nodes: resident ones, looping over tiles.
-int node_grid(long long n, int per_sm) {
+int node_grid(const gfb_solver* s, long long n, int per_sm) {
     const long long per_block = gfb::kNodeTile * (gfb::kNodeThreads / 32);
-    return (int)std::max(1LL, std::min((n + per_block - 1) / per_block, 148LL * per_sm));
+    return (int)std::max(1LL, std::min((n + per_block - 1) / per_block, (long long)s->n_sm * per_sm));
 }
 
 template <typename Real, int NFLD, bool MULTI>
@@ -1148,7 +1143,7 @@ gfb_status launch_node_m(gfb_solver* s) {
         auto* fn = gfb::node_update_kernel<Real, NFLD, MULTI, false>;
         if constexpr (std::is_same<Real, float>::value)
             if (A.half_v) fn = gfb::node_update_kernel<Real, NFLD, MULTI, true>;
-        CU(launch_chained(early, fn, node_grid(s->n_node - g0, gfb::node_blocks_per_sm<Real>(false)), gfb::kNodeThreads, 0,
+        CU(launch_chained(early, fn, node_grid(s, s->n_node - g0, gfb::node_blocks_per_sm<Real>(false)), gfb::kNodeThreads, 0,
                           s->stream, A, P, g0));
         s->launches++;
     }
@@ -1162,7 +1157,7 @@ gfb_status launch_node_m(gfb_solver* s) {
             cudaStream_t q = two ? s->side_stream : s->stream;
             if (two) CU(cudaStreamWaitEvent(q, s->elem_evt, 0));
             CU(launch_chained(two ? elem_lets(s) != nullptr : early, gfb::node_pml_kernel<NFLD, MULTI>,
-                              node_grid(g0, gfb::node_blocks_per_sm<float>(true)), gfb::kNodeThreads, 0, q, A, P));
+                              node_grid(s, g0, gfb::node_blocks_per_sm<float>(true)), gfb::kNodeThreads, 0, q, A, P));
             s->launches++;
             if (two) {
                 CU(cudaEventRecord(s->pml_evt, q));
@@ -1293,8 +1288,6 @@ size_t snapshot_values(const gfb_solver* s) {
 }
 size_t snapshot_bytes(const gfb_solver* s) { return snapshot_values(s) * (s->rec_f32 ? 4 : 8); }
 
-// Convert n snapshot values starting at value `off` of a raw snapshot
-// (float or double, as recorded) to double.
 // Scatter n_out recorded points of 15 values (strain 6, u 3, v 3, a 3) into
 // the caller's arrays: output point q takes the 15 values at
 // raw + src_index(q) * 15 (float or double as recorded).  Threads split the
@@ -2324,6 +2317,7 @@ gfb_status create_impl(const gfb_mesh* m, const gfb_config* c, const gfb_source*
 
     auto s = std::make_unique<gfb_solver>();
     s->device = c->device;
+    CU(cudaDeviceGetAttribute(&s->n_sm, cudaDevAttrMultiProcessorCount, c->device));
     s->prec = c->precision;
     s->ng = m->ngll;
     s->nn = m->ngll * m->ngll * m->ngll;
