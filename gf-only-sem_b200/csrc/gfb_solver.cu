@@ -439,8 +439,8 @@ struct gfb_solver {
         for (auto e : cell_evt) cudaEventDestroy(e);
         for (auto e : copy_evt) cudaEventDestroy(e);
         for (auto p : pinned) cudaFreeHost(p);
+        bufs.clear();  // waits for the device: no kernel writes the flag any more
         if (kernel_err) flag_words().give_back(kernel_err, own_err);
-        bufs.clear();
         if (stream) cudaStreamDestroy(stream);
         if (copy_stream) cudaStreamDestroy(copy_stream);
         if (elem_evt) cudaEventDestroy(elem_evt);
@@ -1700,8 +1700,12 @@ gfb_status build_device(gfb_solver* s, const gfb_mesh* m, const gfb_source* src,
                         // factor = detJ * w_i * w_j * w_k (element_cpu.cpp:108); mu <= 0
                         // adds nothing (element_cpu.cpp:42-43)
                         const double f = m->mu[q] > 0.0 ? m->jacobian[q] * w[i0] * w[j] * w[k] : 0.0;
-                        o[9 * nn + p] = f != 0.0 ? (Real)(m->lambda_[q] * f) : Real(0);
-                        o[10 * nn + p] = f != 0.0 ? (Real)(m->mu[q] * f) : Real(0);
+                        // products of the rounded factors: what the weight's
+                        // rounding does is then the same in both.  With each product
+                        // rounded on its own, FP32 runs end 11-23 % further from FP64
+                        // (1600 steps, 16 media; strain 3.7e-6 against 3.0e-6, layered)
+                        o[9 * nn + p] = f != 0.0 ? (Real)m->lambda_[q] * (Real)f : Real(0);
+                        o[10 * nn + p] = f != 0.0 ? (Real)m->mu[q] * (Real)f : Real(0);
                         cell_off |= !(m->mu[q] > 0.0);
                     }
                     if (cell_off) off.store(true);
