@@ -1064,15 +1064,14 @@ gfb_status launch_elem(gfb_solver* s) {
     return GFB_OK;
 }
 
-gfb_status launch_assemble(gfb_solver* s);
+gfb_status launch_node(gfb_solver* s);
 
-// Autotuner of the FP32 element phase: times full sweeps of every
-// element-kernel candidate on this mesh (the gather kernel with an assembly
-// pass, the line kernel with each cells-per-group count it is built with, and
-// the thread-per-point kernel) and keeps the fastest.  A full sweep only
-// rewrites the assembled force from the current predicted displacement (the
-// first colour touching a node stores), so tuning leaves the solver's state
-// as it was.
+// Autotuner of the FP32 element phase: times the element and node phases of a
+// step with every element-kernel candidate on this mesh (the gather kernel,
+// whose assembly is part of the node phase, the line kernel by colour with each
+// cells-per-group count it is built with, and the thread-per-point kernel) and
+// keeps the fastest.  Called at the end of gfb_create, with the state at rest:
+// without a step start no source acts, so every array stays 0.
 gfb_status autotune(gfb_solver* s) {
     if (!col_kernel_eligible(s)) return GFB_OK;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -1094,7 +1093,7 @@ gfb_status autotune(gfb_solver* s) {
         if (!c.point && (st = dispatch<float, ColGridOp>(s->ng, s->nfld, s))) break;
         auto sweep = [&]() -> gfb_status {
             gfb_status r = launch_elem(s);
-            return r || !use_gather(s) ? r : launch_assemble(s);
+            return r ? r : launch_node(s);
         };
         if ((st = sweep())) break;  // warm-up
         if (cudaEventRecord(e0, s->stream) != cudaSuccess) { st = fail(GFB_ERR_CUDA, "autotune event"); break; }
@@ -1115,6 +1114,18 @@ gfb_status autotune(gfb_solver* s) {
         if (c.ms < best->ms) best = &c;
     s->point_kernel = best->point;
     s->col_variant = best->point ? 0 : best->variant;
+    // 0 without a sign, as gfb_create left it
+    const size_t nF = (size_t)s->n_node * s->F, nP = (size_t)s->n_node * s->nfld * 4;
+    CU(cudaMemsetAsync(s->u, 0, nF * 8, s->stream));
+    CU(cudaMemsetAsync(s->v, 0, nF * 8, s->stream));
+    CU(cudaMemsetAsync(s->a, 0, nF * 4, s->stream));
+    CU(cudaMemsetAsync(s->ut, 0, nP * 4, s->stream));
+    CU(cudaMemsetAsync(s->force, 0, nP * 4, s->stream));
+    if (s->w32) CU(cudaMemsetAsync(s->w32, 0, nF * 4, s->stream));
+    if (s->node_pml && s->n_pml_node > 0) {
+        CU(cudaMemsetAsync(s->npml_mem, 0, (size_t)s->n_pml_node * s->F * 3 * 4, s->stream));
+        CU(cudaMemsetAsync(s->npml_prev, 0, (size_t)s->n_pml_node * s->F * 4, s->stream));
+    }
     return dispatch<float, ColGridOp>(s->ng, s->nfld, s);
 }
 

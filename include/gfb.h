@@ -105,11 +105,11 @@ typedef struct gfb_config {
 /* Launch each step's kernels one by one instead of replaying the step as a
  * captured CUDA graph. */
 #define GFB_FLAG_NO_GRAPH 16
-/* At the end of gfb_create(_batch), time full sweeps of each FP32
- * element-kernel candidate (the default, the line kernel by colour with each
- * cells-per-group count it is built with, and the thread-per-point kernel) on
- * this mesh and keep the fastest; gfb_get_info reports the choice.  Tuning leaves the state
- * unchanged. */
+/* At the end of gfb_create(_batch), time the element and node phases of a step
+ * with each FP32 element-kernel candidate (the default, the line kernel by colour
+ * with each cells-per-group count it is built with, and the thread-per-point
+ * kernel) on this mesh and keep the fastest; gfb_get_info reports the choice.
+ * Tuning leaves the state unchanged. */
 #define GFB_FLAG_AUTOTUNE 32
 /* FP32 path: evaluate the element force from the full predicted
  * displacement at every step.  By default most steps add the force of the
